@@ -44,6 +44,10 @@ struct PhysParams
   // ghost cells in a coarser neighbour: 0 SIMPLE_COPY, 1 EXTRAPOLATE_LINEAR_MINMOD,
   // 2 / 3 CONSERVATIVE_INTERPOLATION_ORDER_2 / 4
   int prolong;
+  // FP64 form: which constants of the mixture's PI are nonzero (bit k: gpx[k]),
+  // and the slope type as an integer (0 no slopes, 1 minmod, 2), so that no
+  // kernel compares doubles for them
+  int pi64, st64;
 };
 
 struct DevMesh
@@ -216,6 +220,19 @@ atomic_max_pos_warp(double * base, int ins, double v)
   const unsigned           lo = __reduce_max_sync(grp, (unsigned)(b >> 32) == hi ? (unsigned)b : 0u);
   if ((int)(threadIdx.x & 31u) == __ffs(grp) - 1 && (hi | lo) != 0u)
     atomicMax(reinterpret_cast<unsigned long long *>(base + ins), ((unsigned long long)hi << 32) | lo);
+}
+
+// max over a full warp of doubles of which only the positive ones count (else
+// +0), on the bit patterns: high word, then low word
+__device__ __forceinline__ double
+warp_max_pos64(double v)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const bool               pos = b - 1ull < 0x7FF0000000000000ull; // positive, infinity included
+  const unsigned           h = pos ? (unsigned)(b >> 32) : 0u;
+  const unsigned           hi = __reduce_max_sync(0xffffffffu, h);
+  const unsigned           lo = __reduce_max_sync(0xffffffffu, pos && h == hi ? (unsigned)b : 0u);
+  return __hiloint2double((int)hi, (int)lo);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,353 @@
+// g5_fast64.cuh — the FP64 form's per-cell arithmetic for the stiffened-gas
+// mixture with as few FP64-pipe instructions as its results allow.
+//
+// The reference arithmetic (prim_fp64, hllc_fp64, slope_scalar<double>,
+// update_fp64 in g5_common.cuh and g5_step2d.cuh) is bound by the FP64 pipe:
+// 1.66 instructions per clock per SM on GB300, two orders of magnitude below
+// the integer and FP32 pipes.  The functions here return the same doubles
+// (compared bit for bit with the CPU oracle; only the sign of a zero may
+// differ) from fewer of them:
+//   * divisions and square roots on the integer pipes (g5_exact64.h), the
+//     quotients of one divisor sharing its reciprocal;
+//   * about two products in three on the integer pipes (mul64: 0.56 clocks per
+//     product and SM against 0.60 for the FP64 pipe, which runs beside them;
+//     the split was found by moving groups of products: all of them on the
+//     integer pipes is 8 % slower, the star state's back on the FP64 pipe 2 %);
+//   * comparisons, minima, maxima, clamps and sign tests on bit patterns;
+//   * factors of 1/2 folded into one fused multiply-add (x +- y/2 rounds once,
+//     as a separate, exact y/2 would) or carried to the next such addition;
+//   * sqrt(fl(c^2)) = c (Boldo 2015: exact in radix 2 without over- or
+//     underflow), which removes two square roots per face;
+//   * minmod slopes without the central difference: when both one-sided
+//     differences agree in sign, |q+ - q-|/2 is never below the smaller one
+//     (rounding is monotonic), so it never limits;
+//   * terms that vanish for the case at hand (pinf = 0).
+// Every shortcut assumes values that are zero or within 2^-900 .. 2^700
+// (g5_exact64.h): states read from memory are tested, results set `bad` when
+// they leave the range, and the caller then evaluates with the reference
+// functions.
+#pragma once
+
+#include "g5_common.cuh"
+#include "g5_exact64.h"
+
+namespace g5
+{
+
+__device__ __forceinline__ long long
+bits64(double x)
+{
+  return __double_as_longlong(x);
+}
+
+// a bit pattern that orders doubles as signed integers (-0 just below +0)
+__device__ __forceinline__ long long
+order64(double x)
+{
+  const long long b = bits64(x);
+  return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL);
+}
+
+// max(x, c) for c > 0, x no NaN
+__device__ __forceinline__ double
+max_pos64(double x, double c)
+{
+  return bits64(x) > bits64(c) ? x : c;
+}
+
+// x where it is positive, else +0
+__device__ __forceinline__ double
+clip0_64(double x)
+{
+  return bits64(x) > 0 ? x : 0.0;
+}
+
+// a b on the FP64 pipe, with the range test of mul64
+__device__ __forceinline__ double
+mulh64(double a, double b, bool & bad)
+{
+  const double r = a * b;
+  bad = bad || x64_raw_bad(r);
+  return r;
+}
+
+// PI = a0 gpx0 + a1 gpx1 of the stiffened-gas mixture, the terms of a zero
+// constant left out
+__device__ __forceinline__ double
+mix_PI64(const PhysParams & P, double a0, double a1, bool & bad)
+{
+  if (P.pi64 == 3)
+    return mul64(a0, P.gpx[0], bad) + mul64(a1, P.gpx[1], bad);
+  return P.pi64 == 0 ? 0.0 : (P.pi64 == 1 ? mul64(a0, P.gpx[0], bad) : mul64(a1, P.gpx[1], bad));
+}
+
+__device__ __forceinline__ double
+mix_S64(const PhysParams & P, double a0, double a1, bool & bad)
+{
+  return mul64(a0, P.xi[0], bad) + mul64(a1, P.xi[1], bad);
+}
+
+// c = sqrt((p (S + 1) + PI) / (rho S)), clipped at 0
+__device__ __forceinline__ double
+sound64(double rho, double p, double S, double PI, bool stiff, bool & bad)
+{
+  double n = mul64(p, S + 1.0, bad);
+  if (stiff)
+    n = n + PI;
+  return sqrt64(clip0_64(div64(n, mul64(rho, S, bad), bad)), bad);
+}
+
+// clamps of computePrimitives: a partial density below 1e-12, and the volume
+// fraction to [0, 1] with its ends widened by 1e-12
+__device__ __forceinline__ double
+clamp_r64(double r)
+{
+  return bits64(r) < bits64(1e-12) ? 0.0 : r;
+}
+
+__device__ __forceinline__ double
+clamp_a64(double a)
+{
+  double r = bits64(a) < bits64(1e-12) ? 0.0 : a;
+  return bits64(r) > bits64(1.0 - 1e-12) ? 1.0 : r;
+}
+
+// prim_fp64 (stiffened gases); the sound speed only when asked for.  RAW: the
+// state comes from memory
+template <int DIM, bool SOUND, bool RAW>
+__device__ __forceinline__ double
+prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
+{
+  using H = V<DIM>;
+  const bool    stiff = P.pi64 != 0;
+  const double  d = max_pos64(u[H::ID], P.smallr);
+  const Recip64 rd = recip64(d, bad);
+  const double  ux = quot64(u[H::IU], rd, bad), uy = quot64(u[H::IV], rd, bad);
+  double        k2 = mul64(ux, ux, bad) + mul64(uy, uy, bad), uz = 0.0;
+  if constexpr (DIM == 3)
+  {
+    uz = quot64(u[H::IW], rd, bad);
+    k2 = k2 + mul64(uz, uz, bad);
+  }
+  const double eint = __fma_rn(-0.5, k2, quot64(u[H::IE], rd, bad));
+  const double a0u = u[H::IA0], a1u = 1.0 - a0u;
+  const double S = mix_S64(P, a0u, a1u, bad);
+  double       n = mul64(d, eint, bad);
+  double       PI = 0.0;
+  if (stiff)
+  {
+    PI = mix_PI64(P, a0u, a1u, bad);
+    n = n - PI;
+  }
+  const double p = div64(n, S, bad);
+  const double a0 = clamp_a64(a0u);
+  if constexpr (RAW)
+  {
+    bad = bad || x64_raw_bad(d) || x64_raw_bad(u[H::IE]) || x64_raw_bad(u[H::IU]) || x64_raw_bad(u[H::IV]) || x64_raw_bad(a0u) ||
+          x64_raw_bad(u[H::IAD0]) || x64_raw_bad(u[H::IAD1]);
+    if constexpr (DIM == 3)
+      bad = bad || x64_raw_bad(u[H::IW]);
+  }
+  q[H::QR0] = clamp_r64(u[H::IAD0]);
+  q[H::QR1] = clamp_r64(u[H::IAD1]);
+  q[H::QP] = p;
+  q[H::QU] = ux;
+  q[H::QV] = uy;
+  if constexpr (DIM == 3)
+    q[H::QW] = uz;
+  q[H::QA] = a0;
+  if constexpr (SOUND)
+  {
+    double Sc = S, PIc = PI;
+    if (bits64(a0) != bits64(a0u))
+    {
+      const double a1 = 1.0 - a0;
+      Sc = mix_S64(P, a0, a1, bad);
+      if (stiff)
+        PIc = mix_PI64(P, a0, a1, bad);
+    }
+    return sound64(d, p, Sc, PIc, stiff, bad);
+  }
+  return 0.0;
+}
+
+// slope_scalar<double> for slope_type 1 (minmod) and 2.  The product of the
+// one-sided differences, whose sign decides, is not formed: when it could
+// underflow (the reference takes that as no slope) the cell is `bad`.
+__device__ __forceinline__ double
+slope_fast64(double q, double qPlus, double qMinus, int st, bool & bad)
+{
+  const double   l = q - qMinus, r = qPlus - q;
+  const uint32_t hl = x64_hi(l), hr = x64_hi(r);
+  const uint32_t el = hl & 0x7FF00000u, er = hr & 0x7FF00000u;
+  const bool     same = (int)(hl ^ hr) >= 0 && el != 0u && er != 0u;
+  bad = bad || (same && el + er < 0x3CC00000u); // |l r| may be below 2^-1074
+  const unsigned long long al = (unsigned long long)bits64(l) << 1, ar = (unsigned long long)bits64(r) << 1;
+  const bool               left = al < ar;
+  double                   m = left ? l : r;
+  if (st == 2)
+  {
+    // 2 min(|l|, |r|) against |q+ - q-| / 2
+    const double c = qPlus - qMinus;
+    m = m + m;
+    const double h = 0.5 * c;
+    m = ((unsigned long long)bits64(m) << 1) < ((unsigned long long)bits64(h) << 1) ? m : x64_make((x64_hi(h) & 0x7FFFFFFFu) | (x64_hi(m) & 0x80000000u), x64_lo(h));
+  }
+  // no slope: a zero with the sign of the central difference
+  return same ? m : x64_make(order64(qPlus) >= order64(qMinus) ? 0u : 0x80000000u, 0u);
+}
+
+// HLLC (hllc_fp64) of two reconstructed states with the mixture's S of either
+// side, scaled by dt/dx.  f: FR0 FR1 FA0 FA1 FE FU FV (FW) FUS.
+static __device__ __noinline__ double
+floor_p64(double p, double r, double smallp)
+{
+  return fmax(p, r * smallp);
+}
+
+struct Side64
+{
+  double r, u, p, e, c; // density, normal velocity, pressure, total energy, sound speed (at least smallc)
+};
+
+template <int DIM>
+__device__ __forceinline__ Side64
+hllc_side64(const double * q, double S, const PhysParams & P, bool stiff, bool & bad)
+{
+  using H = V<DIM>;
+  Side64 s;
+  s.r = max_pos64(q[H::QR0] + q[H::QR1], P.smallr);
+  double p = q[H::QP];
+  // max(p, r smallp): the product only where p is not far above it
+  if ((int)x64_hi(p) <= (int)((x64_hi(s.r) & 0x7FF00000u) + (x64_hi(P.smallp) & 0x7FF00000u) - 0x3FD00000u))
+    p = floor_p64(p, s.r, P.smallp);
+  s.u = q[H::QU];
+  double PI = 0.0;
+  if (stiff)
+    PI = mix_PI64(P, q[H::QA], 1.0 - q[H::QA], bad);
+  double n = mul64(p, S, bad);
+  if (stiff)
+    n = n + PI;
+  const double re = mul64(s.r, div64(n, s.r, bad), bad); // rho e
+  s.p = div64(stiff ? re - PI : re, S, bad);
+  double k = mul64(mul64(s.r, s.u, bad), s.u, bad) + mul64(mul64(s.r, q[H::QV], bad), q[H::QV], bad);
+  if constexpr (DIM == 3)
+    k = k + mul64(mul64(s.r, q[H::QW], bad), q[H::QW], bad);
+  s.e = __fma_rn(0.5, k, re);
+  const double c = sound64(s.r, s.p, S, PI, stiff, bad);
+  s.c = max_pos64(c, P.smallc);
+  return s;
+}
+
+template <int DIM>
+__device__ __forceinline__ void
+hllc_fast64(const double * ql, const double * qr, const Side64 & L, const Side64 & R, double dtdx, double * f, bool & bad)
+{
+  using H = V<DIM>;
+  const double cm = max_pos64(L.c, R.c);
+  const bool   lo = order64(L.u) < order64(R.u);
+  const double SL = (lo ? L.u : R.u) - cm;
+  const double SR = (lo ? R.u : L.u) + cm;
+  const double dl = L.u - SL, dr = SR - R.u;
+  const double rcl = mul64(L.r, dl, bad), rcr = mul64(R.r, dr, bad);
+  const Recip64 rs = recip64(rcr + rcl, bad);
+  const double us = quot64((mul64(rcr, R.u, bad) + mul64(rcl, L.u, bad)) + (L.p - R.p), rs, bad);
+  const double ps = quot64((mul64(rcr, L.p, bad) + mul64(rcl, R.p, bad)) + mul64(mul64(rcl, rcr, bad), L.u - R.u, bad), rs, bad);
+
+  const bool left = bits64(SL) > 0 || bits64(us) > 0;
+  double     r0 = left ? ql[H::QR0] : qr[H::QR0], r1 = left ? ql[H::QR1] : qr[H::QR1];
+  double     ro = left ? L.r : R.r, uo = left ? L.u : R.u, po = left ? L.p : R.p, eo = left ? L.e : R.e;
+  // between the outer waves: the star state of the upwind side
+  if (!(bits64(SL) > 0) && (bits64(us) > 0 || bits64(SR) > 0))
+  {
+    const double  ds = left ? -dl : dr; // S - u
+    const Recip64 rd = recip64((left ? SL : SR) - us, bad);
+    const double  fac = quot64(ds, rd, bad);
+    r0 = mul64(r0, fac, bad);
+    r1 = mul64(r1, fac, bad);
+    ro = mul64(ro, fac, bad);
+    eo = quot64((mul64(ds, eo, bad) - mul64(po, uo, bad)) + mul64(ps, us, bad), rd, bad);
+    uo = us;
+    po = ps;
+  }
+  const double fid = mulh64(r0 + r1, uo, bad);
+  const bool   up = bits64(fid) > 0;
+  f[H::FR0] = mulh64(mulh64(r0, uo, bad), dtdx, bad);
+  f[H::FR1] = mul64(mulh64(r1, uo, bad), dtdx, bad);
+  f[H::FU] = mul64(mulh64(mul64(ro, uo, bad), uo, bad) + po, dtdx, bad);
+  f[H::FE] = mul64(mulh64(eo + po, uo, bad), dtdx, bad);
+  f[H::FV] = mul64(mulh64(fid, up ? ql[H::QV] : qr[H::QV], bad), dtdx, bad);
+  if constexpr (DIM == 3)
+    f[H::FW] = mul64(mulh64(fid, up ? ql[H::QW] : qr[H::QW], bad), dtdx, bad);
+  const double phi0 = up ? ql[H::QA] : qr[H::QA];
+  f[H::FA0] = mul64(mulh64(uo, phi0, bad), dtdx, bad);
+  f[H::FA1] = mulh64(mulh64(uo, 1.0 - phi0, bad), dtdx, bad);
+  f[H::FUS] = mul64(uo, dtdx, bad);
+}
+
+// source_factors_fp64 (stiffened gases)
+template <int DIM>
+__device__ __forceinline__ void
+source_factors_fast64(const double * u, const PhysParams & P, double & st0, double & st1, bool & bad)
+{
+  using H = V<DIM>;
+  st0 = st1 = 1.0;
+  if (P.source_term != 1)
+    return;
+  const double  d = max_pos64(u[H::IAD0] + u[H::IAD1], P.smallr);
+  const Recip64 rdd = recip64(max_pos64(u[H::ID], P.smallr), bad);
+  const double  ux = quot64(u[H::IU], rdd, bad), uy = quot64(u[H::IV], rdd, bad);
+  double        k2 = mul64(ux, ux, bad) + mul64(uy, uy, bad);
+  if constexpr (DIM == 3)
+  {
+    const double uz = quot64(u[H::IW], rdd, bad);
+    k2 = k2 + mul64(uz, uz, bad);
+  }
+  const double  eint = __fma_rn(-0.5, k2, div64(u[H::IE], d, bad));
+  const double  a0 = u[H::IA0], a1 = 1.0 - a0;
+  const double  p = div64(mul64(d, eint, bad) - mix_PI64(P, a0, a1, bad), mix_S64(P, a0, a1, bad), bad);
+  const Recip64 r0 = recip64(mul64(P.gamma[0], p + P.pinf[0], bad), bad), r1 = recip64(mul64(P.gamma[1], p + P.pinf[1], bad), bad);
+  const double  kbar = div64(1.0, quot64(a0, r0, bad) + quot64(u[H::IA1], r1, bad), bad);
+  st0 = 1.0 - quot64(kbar, r0, bad);
+  st1 = 1.0 - quot64(kbar, r1, bad);
+}
+
+// the volume-fraction increment ((F_left - s u*_left) - F_right) + s u*_right, s = st a
+__device__ __forceinline__ double
+alpha_inc64(double fl, double fr, double usl, double usr, double st, double a, bool mp, bool & bad)
+{
+  if (mp)
+  {
+    usl = mul64(st, usl, bad);
+    usr = mul64(st, usr, bad);
+  }
+  return ((fl - mul64(usl, a, bad)) - fr) + mul64(usr, a, bad);
+}
+
+// end of the update: renormalised volume fractions and ID, then the new
+// state's CFL rate (ComputeDtFiveEqFunctor) when asked for
+template <int DIM>
+__device__ __forceinline__ double
+finish_fast64(double * u2, double dx, const PhysParams & P, bool want_dt, bool & bad)
+{
+  using H = V<DIM>;
+  const double sum = u2[H::IA0] + u2[H::IA1];
+  if (bits64(sum) != bits64(1.0))
+  {
+    const double inv = div64(1.0, sum, bad);
+    u2[H::IA0] = mul64(u2[H::IA0], inv, bad);
+    u2[H::IA1] = mul64(u2[H::IA1], inv, bad);
+  }
+  u2[H::ID] = u2[H::IAD0] + u2[H::IAD1];
+  if (!want_dt)
+    return 0.0;
+  double        q[H::NQ];
+  const double  c = prim_fast64<DIM, true, false>(u2, q, P, bad);
+  const Recip64 rdx = recip64(dx, bad);
+  double        r = quot64(c + fabs(q[H::QU]), rdx, bad) + quot64(c + fabs(q[H::QV]), rdx, bad);
+  if constexpr (DIM == 3)
+    r = r + quot64(c + fabs(q[H::QW]), rdx, bad);
+  return r;
+}
+
+} // namespace g5

@@ -1,5 +1,7 @@
 // g5_fp64.cu — FP64 instantiations.  Built with --fmad=false so that every
 // product and sum is rounded separately, as in the reference's arithmetic.
+#include <algorithm>
+
 #include "g5_aux.cuh"
 #include "g5_launch.h"
 #include "g5_prolong.cuh"
@@ -25,19 +27,36 @@ num_sms()
   return g_num_sms;
 }
 
-template <int B, bool MIXED>
+// whether the case takes the fast FP64 form (g5_fast64.cuh): stiffened gases,
+// its constants within the form's range (zero allowed where it may be), floors
+// whose products stay in it
+static bool
+fast64_case(const PhysParams & p)
+{
+  const auto in = [](double x, double lo, double hi) { return x >= lo && x <= hi; };
+  const auto zin = [&](double x) { return x == 0.0 || in(x < 0.0 ? -x : x, 1e-200, 1e200); };
+  bool       ok = !p.mg_any && in(p.smallr, 1e-60, 1e60) && in(p.smallc, 1e-100, 1e100);
+  for (int k = 0; k < 2; ++k)
+    ok = ok && zin(p.xi[k]) && zin(p.gpx[k]) && zin(p.gamma[k]) && zin(p.pinf[k]);
+  return ok;
+}
+
+// the equation-of-state argument of the FP64 step kernels
+constexpr int FAST64 = 0, REF64 = 2;
+
+template <int B, int STIFF>
 static cudaError_t
 launch_step2d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches)
 {
-  using T = Step2DTraits<B, MIXED>;
+  using T = Step2DTraits<B, false>;
   static bool configured = false;
   static int  occ = 1;
   if (!configured)
   {
-    cudaError_t e = cudaFuncSetAttribute(step2d_kernel<B, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
+    cudaError_t e = cudaFuncSetAttribute(step2d_kernel<B, false, false, STIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
     if (e != cudaSuccess)
       return e;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, MIXED>, T::NT, T::smem_bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, false, false, STIFF>, T::NT, T::smem_bytes);
     if (occ < 1)
       occ = 1;
     configured = true;
@@ -49,7 +68,7 @@ launch_step2d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launche
   cudaError_t e = cudaSuccess;
   if (grid >= 1)
   {
-    step2d_kernel<B, MIXED><<<grid, T::NT, T::smem_bytes, s>>>(a);
+    step2d_kernel<B, false, false, STIFF><<<grid, T::NT, T::smem_bytes, s>>>(a);
     ++*launches;
     e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -65,14 +84,14 @@ launch_step2d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launche
   return e;
 }
 
-template <int B, bool MIXED>
+template <int B, int STIFF>
 static int
 occupancy2d()
 {
-  using T = Step2DTraits<B, MIXED>;
-  cudaFuncSetAttribute(step2d_kernel<B, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
+  using T = Step2DTraits<B, false>;
+  cudaFuncSetAttribute(step2d_kernel<B, false, false, STIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, MIXED>, T::NT, T::smem_bytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, false, false, STIFF>, T::NT, T::smem_bytes);
   return occ;
 }
 
@@ -231,9 +250,9 @@ launch_step_fp64(int dim, int b, const StepArgs & a, int ctas_per_sm, cudaStream
   if (e != cudaSuccess)
     return e;
   if (dim == 2 && b == 16)
-    return launch_step2d<16, false>(a, ctas_per_sm, s, launches);
+    return fast64_case(a.p) ? launch_step2d<16, FAST64>(a, ctas_per_sm, s, launches) : launch_step2d<16, REF64>(a, ctas_per_sm, s, launches);
   if (dim == 2 && b == 8)
-    return launch_step2d<8, false>(a, ctas_per_sm, s, launches);
+    return fast64_case(a.p) ? launch_step2d<8, FAST64>(a, ctas_per_sm, s, launches) : launch_step2d<8, REF64>(a, ctas_per_sm, s, launches);
   if (dim == 3 && b == 8)
     return launch_step3d<false>(a, ctas_per_sm, s, launches);
   return cudaErrorInvalidValue;
@@ -243,9 +262,9 @@ int
 step_max_ctas_per_sm_fp64(int dim, int b)
 {
   if (dim == 2 && b == 16)
-    return occupancy2d<16, false>();
+    return std::min(occupancy2d<16, FAST64>(), occupancy2d<16, REF64>());
   if (dim == 2 && b == 8)
-    return occupancy2d<8, false>();
+    return std::min(occupancy2d<8, FAST64>(), occupancy2d<8, REF64>());
   if (dim == 3 && b == 8)
     return occupancy3d<false>();
   return 0;

@@ -134,6 +134,8 @@ make_phys(const G5Params * params)
   }
   p.mg_any = params->eos[0] != G5_EOS_STIFFENED || params->eos[1] != G5_EOS_STIFFENED;
   p.prolong = params->prolongation;
+  p.pi64 = (p.gpx[0] != 0.0 ? 1 : 0) | (p.gpx[1] != 0.0 ? 2 : 0);
+  p.st64 = p.slope_type == 1.0 ? 1 : (p.slope_type == 2.0 ? 2 : 0);
   return p;
 }
 

@@ -16,6 +16,7 @@
 #pragma once
 
 #include "g5_common.cuh"
+#include "g5_fast64.cuh"
 
 namespace g5
 {
@@ -24,11 +25,18 @@ template <int B, bool MIXED>
 struct Step2DTraits
 {
   using R = typename std::conditional<MIXED, float, double>::type;
-  static constexpr int NT = B * B;
+  // FP64: more threads than cells, so that the 320 (96) slope cells take one
+  // round and the 544 (144) faces two, at 96 registers (16x16: 420 us per
+  // shock-bubble step of 486k cells against 444 us with 256 threads at 128
+  // registers, 438 us with 384 at 80; 8x8: 147 us against 161 with 64 threads)
+  static constexpr int NT = MIXED ? B * B : (B == 16 ? 320 : 96);
+  static constexpr int CTAS = MIXED ? (B == 16 ? 4 : 8) : (B == 16 ? 2 : 7);
   static constexpr int G = B + 4;  // ghosted extent
   static constexpr int S = B + 2;  // ring extent
   static constexpr int NQ = 6;     // r0 r1 p u v a0
-  static constexpr int NREC = 15;  // dqx[5] dqy[5] hS[5] (the THINC normal is evaluated on demand)
+  // dqx[5] dqy[5] hS[5] (the THINC normal is evaluated on demand); FP64: and
+  // the mixture's S of the cell
+  static constexpr int NREC = MIXED ? 15 : 16;
   static constexpr int NFF = B * (B + 1);
   static constexpr size_t smem_bytes = sizeof(R) * (size_t)(NQ * G * G + NREC * S * S + 2 * 8 * NFF) + 64;
 };
@@ -141,11 +149,33 @@ gather_ghost_2d(const StepArgs & a, int n, int cx0, int cy0, int gx, int gy, dou
   return true;
 }
 
-template <int B, bool MIXED>
-__device__ __forceinline__ void
+// FP64 cold path: the reference's primitives of a cell whose values leave the
+// range of the fast form
+template <int DIM>
+struct State64
+{
+  double v[V<DIM>::NV];
+};
+
+template <int DIM>
+__device__ __noinline__ void
+prim_ref64(State64<DIM> u, const PhysParams * P, double * sQ, int stride)
+{
+  double q[V<DIM>::NQ];
+  prim_fp64<DIM>(u.v, q, *P);
+  for (int k = 0; k < V<DIM>::NQ; ++k)
+    sQ[k * stride] = q[k];
+}
+
+// the primitives of a cell into the ghosted arrays.  STIFF: the equation of
+// state of step2d_kernel.  Returns whether the values leave the range of the
+// fast FP64 form (the block then takes the reference arithmetic).
+template <int B, bool MIXED, int STIFF>
+__device__ __forceinline__ bool
 store_prim(typename Step2DTraits<B, MIXED>::R * sQ, int gidx, const double * u, const PhysParams & P, int eosk)
 {
   constexpr int GG = (B + 4) * (B + 4);
+  bool          bad = false;
   if constexpr (MIXED)
   {
     float q[6];
@@ -157,11 +187,24 @@ store_prim(typename Step2DTraits<B, MIXED>::R * sQ, int gidx, const double * u, 
   else
   {
     double q[6];
-    prim_fp64<2>(u, q, P);
+    if constexpr (STIFF == 2)
+      prim_fp64<2>(u, q, P);
+    else
+      prim_fast64<2, false, true>(u, q, P, bad);
+    if (bad)
+    {
+      State64<2> s;
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        s.v[v] = u[v];
+      prim_ref64<2>(s, &P, sQ + gidx, GG);
+      return true;
+    }
 #pragma unroll
     for (int k = 0; k < 6; ++k)
       sQ[k * GG + gidx] = q[k];
   }
+  return bad;
 }
 
 // Youngs normal (restated: (1,2,1)-weighted central differences), |n_x|, |n_y|
@@ -178,100 +221,63 @@ youngs_abs_2d(const R * A, int gi, R & nx, R & ny)
   ny = (nrm > R(0)) ? fabs(-gy / nrm) : R(0);
 }
 
-// reconstruct one side of a face from cell (ci, cj) (ghosted-ring coordinates)
-// dir: 0 X, 1 Y; side: +1 -> right face of the cell (qL), -1 -> left face (qR)
-template <int B, bool MIXED>
-__device__ __forceinline__ void
-face_state(const typename Step2DTraits<B, MIXED>::R * sQ,
-           const typename Step2DTraits<B, MIXED>::R * sRec,
-           int                                          ci,
-           int                                          cj,
-           int                                          dir,
-           int                                          side,
-           const PhysParams &                           P,
-           typename Step2DTraits<B, MIXED>::R *         q)
+// THINC value of the volume fraction at the cell's face
+// (scheme/ComputeFluxesAndStoreTHINCFunctor.cpp:122-283): a0 the cell's value,
+// aM and aP its neighbours' along the direction, nd the Youngs normal's
+// component, bs = +-1 the side
+__device__ __forceinline__ double
+thinc_alpha64(double a0, double aM, double aP, double nd, double bs, double thinc_beta)
 {
-  using T = Step2DTraits<B, MIXED>;
-  using R = typename T::R;
+  const double beta = thinc_beta * nd + 0.01;
+  const double Aa = (aP + aM) / 2.0;
+  const double Bb = (aP - aM) / 2.0;
+  const double C = tanh_d(0.5 * beta);
+  const double D = tanh_d(0.5 * beta * (a0 - Aa) / Bb);
+  return Aa + bs * Bb * (C + bs * D / C) / (1.0 + bs * D);
+}
+
+// FP64: reconstruct one side of a face from cell (ci, cj) (ghosted-ring
+// coordinates).  dir: 0 X, 1 Y; side: +1 -> right face of the cell (qL), -1 ->
+// left face (qR).  The reference's order; the Hancock source is stored without
+// its factor 1/2.
+template <int B>
+__device__ __forceinline__ void
+face_state_ref64(const double * sQ, const double * sRec, int ci, int cj, int dir, int side, const PhysParams & P, double * q)
+{
+  using T = Step2DTraits<B, false>;
   constexpr int G = T::G, S = T::S, GG = G * G, SS = S * S;
   const int     gi = (ci + 2) + G * (cj + 2);
   const int     si = (ci + 1) + S * (cj + 1);
-  const R       offx = dir == 0 ? R(0.5) * R(side) : R(0);
-  const R       offy = dir == 1 ? R(0.5) * R(side) : R(0);
+  const double  offx = dir == 0 ? 0.5 * side : 0.0;
+  const double  offy = dir == 1 ? 0.5 * side : 0.0;
   const bool    hancock = P.integrator == 0;
-  R             thinc_eps, thinc_beta, smallr;
-  if constexpr (MIXED)
-  {
-    thinc_eps = P.f_thinc_eps;
-    thinc_beta = P.f_thinc_beta;
-    smallr = P.f_smallr;
-  }
-  else
-  {
-    thinc_eps = P.thinc_eps;
-    thinc_beta = P.thinc_beta;
-    smallr = P.smallr;
-  }
-  R qc[5], dqx[5], dqy[5], hs[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k)
   {
-    qc[k] = sQ[k * GG + gi];
-    dqx[k] = sRec[k * SS + si];
-    dqy[k] = sRec[(5 + k) * SS + si];
-    hs[k] = sRec[(10 + k) * SS + si];
+    q[k] = sQ[k * GG + gi] + offx * sRec[k * SS + si] + offy * sRec[(5 + k) * SS + si];
+    if (hancock)
+      q[k] += 0.5 * sRec[(10 + k) * SS + si];
   }
-  const R a0 = sQ[5 * GG + gi];
-#pragma unroll
-  for (int k = 0; k < 5; ++k)
-  {
-    if constexpr (MIXED)
-      q[k] = qc[k] + offx * dqx[k] + offy * dqy[k] + (hancock ? hs[k] : R(0));
-    else
-    {
-      q[k] = qc[k] + offx * dqx[k] + offy * dqy[k];
-      if (hancock)
-        q[k] += hs[k];
-    }
-  }
+  const double a0 = sQ[5 * GG + gi];
   q[5] = a0;
   if (P.thinc)
   {
-    // THINC (scheme/ComputeFluxesAndStoreTHINCFunctor.cpp:122-283): alpha
-    // and the partial densities from the hyperbolic-tangent profile
-    const int  o = dir == 0 ? 1 : G;
-    const R *  A = sQ + 5 * GG;
-    const R    aP = A[gi + o], aM = A[gi - o];
-    const R    mono = (aP - a0) * (a0 - aM);
-    const bool req = (a0 > thinc_eps) && (a0 < R(1) - thinc_eps) && mono > R(0);
-    if (req)
+    const int      o = dir == 0 ? 1 : G;
+    const double * A = sQ + 5 * GG;
+    const double   aP = A[gi + o], aM = A[gi - o];
+    const double   mono = (aP - a0) * (a0 - aM);
+    if (a0 > P.thinc_eps && a0 < 1.0 - P.thinc_eps && mono > 0.0)
     {
-      R nxa, nya;
-      youngs_abs_2d<R, G>(A, gi, nxa, nya);
-      const R nd = dir == 0 ? nxa : nya;
-      const R beta = thinc_beta * nd + R(0.01);
-      const R Aa = (aP + aM) / R(2);
-      const R Bb = (aP - aM) / R(2);
-      R       C, D;
-      if constexpr (MIXED)
-      {
-        C = tanhf(R(0.5) * beta);
-        D = tanhf(R(0.5) * beta * (a0 - Aa) / Bb);
-      }
-      else
-      {
-        C = tanh_d(R(0.5) * beta);
-        D = tanh_d(R(0.5) * beta * (a0 - Aa) / Bb);
-      }
-      const R bs = R(side);
-      const R af = Aa + bs * Bb * (C + bs * D / C) / (R(1) + bs * D);
-      const R r0 = qc[0], r1 = qc[1];
-      R       q0 = r0 + r0 / a0 * (af - a0);
-      R       q1 = r1 + r1 / (R(1) - a0) * (a0 - af);
+      double nxa, nya;
+      youngs_abs_2d<double, G>(A, gi, nxa, nya);
+      const double af = thinc_alpha64(a0, aM, aP, dir == 0 ? nxa : nya, (double)side, P.thinc_beta);
+      const double r0 = sQ[gi], r1 = sQ[GG + gi];
+      double       q0 = r0 + r0 / a0 * (af - a0);
+      double       q1 = r1 + r1 / (1.0 - a0) * (a0 - af);
       if (hancock)
       {
-        q0 += hs[0];
-        q1 += hs[1];
+        q0 += 0.5 * sRec[10 * SS + si];
+        q1 += 0.5 * sRec[11 * SS + si];
       }
       q[0] = q0;
       q[1] = q1;
@@ -281,12 +287,248 @@ face_state(const typename Step2DTraits<B, MIXED>::R * sQ,
   }
   else
   {
-    q[0] = fmax(smallr, q[0]);
-    q[1] = fmax(smallr, q[1]);
+    q[0] = fmax(P.smallr, q[0]);
+    q[1] = fmax(P.smallr, q[1]);
   }
 }
 
-// The mixed form of face_state for a face direction known at compile time:
+// the cells either side of face ff of direction dir
+template <int B>
+__device__ __forceinline__ void
+face_cells(int dir, int ff, int & li, int & lj, int & ri, int & rj)
+{
+  if (dir == 0)
+  {
+    ri = ff % (B + 1);
+    rj = ff / (B + 1);
+    li = ri - 1;
+    lj = rj;
+  }
+  else
+  {
+    ri = ff % B;
+    rj = ff / B;
+    li = ri;
+    lj = rj - 1;
+  }
+}
+
+// FP64: the HLLC flux of face ff of direction dir, times dt/dx, in the
+// reference's arithmetic
+template <int B>
+__device__ __forceinline__ void
+face_flux_ref64(const double * sQ, const double * sRec, double * sF, int dir, int ff, double dtdx, const PhysParams & P)
+{
+  using H = V<2>;
+  constexpr int NFF = B * (B + 1);
+  int           li, lj, ri, rj;
+  face_cells<B>(dir, ff, li, lj, ri, rj);
+  double qL[6], qR[6], fl[8];
+  face_state_ref64<B>(sQ, sRec, li, lj, dir, +1, P, qL);
+  face_state_ref64<B>(sQ, sRec, ri, rj, dir, -1, P, qR);
+  if (dir == 1)
+  {
+    double t = qL[3];
+    qL[3] = qL[4];
+    qL[4] = t;
+    t = qR[3];
+    qR[3] = qR[4];
+    qR[4] = t;
+  }
+  hllc_fp64<2>(qL, qR, P, fl);
+  if (dir == 1)
+  {
+    const double t = fl[H::FU];
+    fl[H::FU] = fl[H::FV];
+    fl[H::FV] = t;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    sF[k * NFF + ff] = fl[k] * dtdx;
+}
+
+template <int B>
+__device__ __noinline__ void
+face_flux_cold64(const double * sQ, const double * sRec, double * sF, int dir, int ff, double dtdx, const PhysParams * P)
+{
+  face_flux_ref64<B>(sQ, sRec, sF, dir, ff, dtdx, *P);
+}
+
+// FP64: the reconstructed state and the mixture's S of one side (the values
+// of face_state_ref64, normal velocity first).  The direction is a run-time
+// value: X and Y faces share one copy of the flux code, which is long enough
+// to miss the instruction cache.
+template <int B>
+__device__ __forceinline__ double
+face_state_fast64(const double * sQ, const double * sRec, int ci, int cj, int dir, int side, const PhysParams & P, double * q, bool & bad)
+{
+  using T = Step2DTraits<B, false>;
+  constexpr int    G = T::G, S = T::S, GG = G * G, SS = S * S;
+  const double     off = side > 0 ? 0.5 : -0.5;
+  const int        gi = (ci + 2) + G * (cj + 2);
+  const int        si = (ci + 1) + S * (cj + 1);
+  const double *   dq = sRec + dir * 5 * SS + si;
+  const bool       hancock = P.integrator == 0;
+#pragma unroll
+  for (int k = 0; k < 5; ++k)
+  {
+    const int    from = k < 3 ? k : (k == 3 ? 3 + dir : 4 - dir);
+    const double t = __fma_rn(off, dq[from * SS], sQ[from * GG + gi]);
+    q[k] = hancock ? __fma_rn(0.5, sRec[(10 + from) * SS + si], t) : t;
+  }
+  const double a0 = sQ[5 * GG + gi];
+  double       Sm = sRec[15 * SS + si];
+  q[5] = a0;
+  if (P.thinc)
+  {
+    const int      o = dir == 0 ? 1 : G;
+    const double * A = sQ + 5 * GG;
+    const double   aP = A[gi + o], aM = A[gi - o];
+    const bool     mono = (bits64(aP) > bits64(a0) && bits64(a0) > bits64(aM)) || (bits64(aP) < bits64(a0) && bits64(a0) < bits64(aM));
+    if (mono && bits64(a0) > bits64(P.thinc_eps) && bits64(a0) < bits64(1.0 - P.thinc_eps))
+    {
+      double nxa, nya;
+      youngs_abs_2d<double, G>(A, gi, nxa, nya);
+      const double af = thinc_alpha64(a0, aM, aP, dir == 0 ? nxa : nya, side > 0 ? 1.0 : -1.0, P.thinc_beta);
+      const double r0 = sQ[gi], r1 = sQ[GG + gi];
+      double       q0 = r0 + r0 / a0 * (af - a0);
+      double       q1 = r1 + r1 / (1.0 - a0) * (a0 - af);
+      if (hancock)
+      {
+        q0 = __fma_rn(0.5, sRec[10 * SS + si], q0);
+        q1 = __fma_rn(0.5, sRec[11 * SS + si], q1);
+      }
+      q[0] = q0;
+      q[1] = q1;
+      q[5] = af;
+      Sm = mix_S64(P, af, 1.0 - af, bad);
+    }
+  }
+  else
+  {
+    q[0] = max_pos64(q[0], P.smallr);
+    q[1] = max_pos64(q[1], P.smallr);
+  }
+  return Sm;
+}
+
+template <int B>
+__device__ __forceinline__ bool
+face_flux_fast64(const double * sQ, const double * sRec, double * sF, int dir, int ff, double dtdx, const PhysParams & P)
+{
+  using H = V<2>;
+  constexpr int NFF = B * (B + 1);
+  int           li, lj, ri, rj;
+  face_cells<B>(dir, ff, li, lj, ri, rj);
+  double       qL[6], qR[6], fl[8];
+  bool         bad = false;
+  const double Sl = face_state_fast64<B>(sQ, sRec, li, lj, dir, 1, P, qL, bad);
+  const double Sr = face_state_fast64<B>(sQ, sRec, ri, rj, dir, -1, P, qR, bad);
+  const Side64 L = hllc_side64<2>(qL, Sl, P, P.pi64 != 0, bad);
+  const Side64 R = hllc_side64<2>(qR, Sr, P, P.pi64 != 0, bad);
+  hllc_fast64<2>(qL, qR, L, R, dtdx, fl, bad);
+  if (bad)
+  {
+    face_flux_cold64<B>(sQ, sRec, sF, dir, ff, dtdx, &P);
+    return true;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    sF[(k == H::FU ? H::FU + dir : k == H::FV ? H::FV - dir : k) * NFF + ff] = fl[k];
+  return false;
+}
+
+// FP64: limited slopes, Hancock source (ComputeFluxesAndStoreFunctor.cpp:
+// 174-199, without its factor 1/2) of ring cell r, in the reference's
+// arithmetic
+template <int B>
+__device__ __forceinline__ void
+hancock_ref64(const double * sQ, double * sRec, int gi, int r, double dtdx, const PhysParams & P)
+{
+  using T = Step2DTraits<B, false>;
+  constexpr int G = T::G, S = T::S, GG = G * G, SS = S * S;
+  double        q[5], dx[5], dy[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k)
+  {
+    const double * Qk = sQ + k * GG;
+    q[k] = Qk[gi];
+    dx[k] = slope_scalar<double>(q[k], Qk[gi + 1], Qk[gi - 1], P.slope_type);
+    dy[k] = slope_scalar<double>(q[k], Qk[gi + G], Qk[gi - G], P.slope_type);
+    sRec[k * SS + r] = dx[k];
+    sRec[(5 + k) * SS + r] = dy[k];
+  }
+  if (P.integrator != 0)
+    return;
+  const double a0 = sQ[5 * GG + gi];
+  const double r0 = q[0], r1 = q[1], p = q[2], u = q[3], v = q[4];
+  const double rr = r0 + r1;
+  const double c = sound_speed_mix(P, rr, p, a0, 1 - a0, r0, r1);
+  const double sr0 = (-u * (dx[0] + dx[1]) - dx[3] * rr) * dtdx + (-v * (dy[0] + dy[1]) - dy[4] * rr) * dtdx;
+  sRec[10 * SS + r] = sr0 * a0;
+  sRec[11 * SS + r] = sr0 * (1.0 - a0);
+  sRec[12 * SS + r] = (-u * dx[2] - dx[3] * rr * c * c) * dtdx + (-v * dy[2] - dy[4] * rr * c * c) * dtdx;
+  sRec[13 * SS + r] = (-u * dx[3] - dx[2] / rr) * dtdx + (-v * dy[3]) * dtdx;
+  sRec[14 * SS + r] = (-u * dx[4]) * dtdx + (-v * dy[4] - dy[2] / rr) * dtdx;
+}
+
+template <int B>
+__device__ __noinline__ void
+hancock_cold64(const double * sQ, double * sRec, int gi, int r, double dtdx, const PhysParams * P)
+{
+  hancock_ref64<B>(sQ, sRec, gi, r, dtdx, *P);
+}
+
+// the same values from the fast operations, and the mixture's S of the cell
+template <int B>
+__device__ __forceinline__ bool
+hancock_fast64(const double * sQ, double * sRec, int gi, int r, double dtdx, const PhysParams & P)
+{
+  using T = Step2DTraits<B, false>;
+  constexpr int G = T::G, S = T::S, GG = G * G, SS = S * S;
+  const bool    stiff = P.pi64 != 0;
+  const int     st = P.st64;
+  double        q[5], dx[5], dy[5];
+  bool          bad = false;
+#pragma unroll
+  for (int k = 0; k < 5; ++k)
+  {
+    const double * Qk = sQ + k * GG;
+    q[k] = Qk[gi];
+    dx[k] = 0.0;
+    dy[k] = 0.0;
+    if (st != 0)
+    {
+      dx[k] = slope_fast64(q[k], Qk[gi + 1], Qk[gi - 1], st, bad);
+      dy[k] = slope_fast64(q[k], Qk[gi + G], Qk[gi - G], st, bad);
+    }
+    sRec[k * SS + r] = dx[k];
+    sRec[(5 + k) * SS + r] = dy[k];
+  }
+  const double a0 = sQ[5 * GG + gi], a1 = 1.0 - a0;
+  const double Sm = mix_S64(P, a0, a1, bad);
+  sRec[15 * SS + r] = Sm;
+  if (P.integrator == 0)
+  {
+    const double  p = q[2], u = q[3], v = q[4];
+    const double  rr = q[0] + q[1];
+    const Recip64 rd = recip64(rr, bad);
+    const double  c = sound64(rr, p, Sm, stiff ? mix_PI64(P, a0, a1, bad) : 0.0, stiff, bad);
+    const double  dxr = mul64(dx[3], rr, bad), dyr = mul64(dy[4], rr, bad);
+    const double  sr0 = mul64(mulh64(-u, dx[0] + dx[1], bad) - dxr, dtdx, bad) + mul64(mulh64(-v, dy[0] + dy[1], bad) - dyr, dtdx, bad);
+    sRec[10 * SS + r] = mul64(sr0, a0, bad);
+    sRec[11 * SS + r] = mulh64(sr0, a1, bad);
+    sRec[12 * SS + r] = mul64(mulh64(-u, dx[2], bad) - mulh64(mul64(dxr, c, bad), c, bad), dtdx, bad) +
+                       mul64(mulh64(-v, dy[2], bad) - mulh64(mul64(dyr, c, bad), c, bad), dtdx, bad);
+    sRec[13 * SS + r] = mul64(mulh64(-u, dx[3], bad) - quot64(dx[2], rd, bad), dtdx, bad) + mul64(mulh64(-v, dy[3], bad), dtdx, bad);
+    sRec[14 * SS + r] = mul64(mulh64(-u, dx[4], bad), dtdx, bad) + mul64(mulh64(-v, dy[4], bad) - quot64(dy[2], rd, bad), dtdx, bad);
+  }
+  if (bad)
+    hancock_cold64<B>(sQ, sRec, gi, r, dtdx, &P);
+  return bad;
+}
+
+// The FP32-bulk form's state of one face side, the direction known at compile time:
 // q = (q + hs) + off * dq_dir, with q + hs stored by the slope phase, so a
 // face side reads 11 values of shared memory instead of 21.
 template <int B, int DIR, bool THINC>
@@ -454,6 +696,53 @@ update_fp64(const double * uin, double * u2, const double * sFx, const double * 
   double       q[6];
   const double c = prim_fp64<2>(u2, q, P);
   return (c + fabs(q[H::QU])) / dx + (c + fabs(q[H::QV])) / dx;
+}
+
+// FP64 cold path: the update of a cell whose values leave the fast form's
+// range, written to U2 (out, variables NC apart)
+template <int B>
+__device__ __noinline__ double
+update_cold64(State64<2> uin, double * out, const double * sFx, const double * sFy, int ci, int cj, double dx, const PhysParams * P, bool want_dt)
+{
+  double       u2[V<2>::NV];
+  const double r = update_fp64<B>(uin.v, u2, sFx, sFy, ci, cj, dx, *P, want_dt);
+  for (int v = 0; v < V<2>::NV; ++v)
+    out[v * B * B] = u2[v];
+  return r;
+}
+
+// update_fp64 from the fast operations (stiffened gases).  (The reference
+// starts each sum from 0 + F_left: the same value but for the sign of a zero.)
+template <int B>
+__device__ __forceinline__ double
+update_fast64(const double * uin, double * u2, const double * sFx, const double * sFy, int ci, int cj, double dx, const PhysParams & P, bool want_dt,
+              bool & bad)
+{
+  using H = V<2>;
+  constexpr int NFF = B * (B + 1);
+#pragma unroll
+  for (int v = 0; v < H::NV; ++v)
+    u2[v] = uin[v];
+  double     st0, st1;
+  const bool mp = P.source_term == 1;
+  source_factors_fast64<2>(uin, P, st0, st1, bad);
+  bad = bad || x64_raw_bad(uin[H::IA1]); // (the rest was tested for the primitives)
+#pragma unroll
+  for (int dir = 0; dir < 2; ++dir)
+  {
+    const double * F = dir == 0 ? sFx : sFy;
+    const int      il = dir == 0 ? ci + (B + 1) * cj : ci + B * cj;
+    const int      ir = dir == 0 ? il + 1 : il + B;
+    const double   usl = F[H::FUS * NFF + il], usr = F[H::FUS * NFF + ir];
+    u2[H::IAD0] = clamp_r64(u2[H::IAD0] + (F[H::FR0 * NFF + il] - F[H::FR0 * NFF + ir]));
+    u2[H::IAD1] = clamp_r64(u2[H::IAD1] + (F[H::FR1 * NFF + il] - F[H::FR1 * NFF + ir]));
+    u2[H::IA0] = clamp_a64(u2[H::IA0] + alpha_inc64(F[H::FA0 * NFF + il], F[H::FA0 * NFF + ir], usl, usr, st0, uin[H::IA0], mp, bad));
+    u2[H::IA1] = clamp_a64(u2[H::IA1] + alpha_inc64(F[H::FA1 * NFF + il], F[H::FA1 * NFF + ir], usl, usr, st1, uin[H::IA1], mp, bad));
+    u2[H::IE] += F[H::FE * NFF + il] - F[H::FE * NFF + ir];
+    u2[H::IU] += F[H::FU * NFF + il] - F[H::FU * NFF + ir];
+    u2[H::IV] += F[H::FV * NFF + il] - F[H::FV * NFF + ir];
+  }
+  return finish_fast64<2>(u2, dx, P, want_dt, bad);
 }
 
 // The same update in the FP32-bulk form.  FP64 is used only for the adds
@@ -639,16 +928,18 @@ finish_deferred_2d(const StepArgs & a, int j)
 
 // 4 CTAs per SM in the FP32-bulk form (64 registers), so that CTAs in the
 // FP64-heavy update overlap with CTAs in the FP32 face phase; 2 CTAs per SM
-// (128 registers) in the FP64 form
+// (96 registers) in the FP64 form
 // THINC, STIFF: the FP32-bulk form is compiled with and without the THINC
 // reconstruction and the stiffened-gas pressure path (P picks the kernel), so
-// a kernel carries only the code its case runs; the FP64 form tests both at
-// run time (STIFF = -1).  FUSED: the FP32-bulk form finishing the coarse/fine
+// a kernel carries only the code its case runs; the FP64 form tests THINC at
+// run time and has STIFF = 2 (the reference arithmetic: Mie-Grueneisen laws,
+// floors outside the fast form's range) and 0 (the fast form of
+// g5_fast64.cuh: stiffened gases).  FUSED: the FP32-bulk form finishing the coarse/fine
 // records in its tail (m.fin_tgt set; the kernel without it keeps the plain
 // block loop)
 template <int B, bool MIXED, bool THINC = false, int STIFF = -1, bool FUSED = false>
-__global__ void __launch_bounds__(B * B, MIXED ? (B == 16 ? 4 : 8) : (B == 16 ? 2 : 8))
-step2d_kernel(StepArgs a)
+__global__ void __launch_bounds__(Step2DTraits<B, MIXED>::NT, Step2DTraits<B, MIXED>::CTAS)
+step2d_kernel(const __grid_constant__ StepArgs a)
 {
   using T = Step2DTraits<B, MIXED>;
   using R = typename T::R;
@@ -709,20 +1000,37 @@ step2d_kernel(StepArgs a)
       if constexpr (MIXED)
         dtdx_r = d2f_fast(a.dt[ins]) * __frcp_rn(d2f_fast(dx));
       else
-        dtdx_r = a.dt[ins] / dx;
+        dtdx_r = a.dt[ins];
+      // FP64 fast form: a value of the block left its range (per thread until
+      // the next barrier, then for the whole CTA: the phases that follow take
+      // the reference arithmetic)
+      constexpr bool fast64 = !MIXED && STIFF != 2;
+      bool           cold = false;
+      if constexpr (fast64)
+      {
+        cold = x64_raw_bad(dtdx_r) || x64_raw_bad(dx);
+        const double q = div64(dtdx_r, dx, cold);
+        dtdx_r = cold ? dtdx_r / dx : q;
+      }
+      else if constexpr (!MIXED)
+        dtdx_r = dtdx_r / dx;
 
       // ---------------- phase 1: own cell (coalesced) + halo gather -> primitives
       // (the own cell's loads are in flight while the halo gather runs; its
       // primitives are stored last)
       const int ci = tid % B, cj = tid / B;
-      double    uin[H::NV];
+      // (the FP64 form has more threads than cells; the ones without a cell
+      // take the first halo cells)
+      const bool owner = NT == NC || tid < NC;
+      double     uin[H::NV];
+      if (owner)
       {
         const double * base = a.U + (size_t)n * H::NV * NC + tid;
 #pragma unroll
         for (int v = 0; v < H::NV; ++v)
           uin[v] = base[v * NC];
       }
-      for (int h = tid; h < NHALO; h += NT)
+      for (int h = NT == NC ? tid : (tid < NC ? tid + NT - NC : tid - NC); h < NHALO; h += NT)
       {
         int gx, gy;
         halo_coords<B>(h, gx, gy);
@@ -730,18 +1038,23 @@ step2d_kernel(StepArgs a)
         if (!gather_ghost_2d<B>(a, n, cx0, cy0, gx, gy, u))
         {
           raise_status(a.status, STATUS_MESH);
+          const double * own = a.U + (size_t)n * H::NV * NC;
 #pragma unroll
           for (int v = 0; v < H::NV; ++v)
-            u[v] = uin[v];
+            u[v] = NT == NC ? uin[v] : own[v * NC];
         }
-        store_prim<B, MIXED>(sQ, (gx + 2) + G * (gy + 2), u, P, eosk);
+        cold |= store_prim<B, MIXED, STIFF>(sQ, (gx + 2) + G * (gy + 2), u, P, eosk);
       }
-      store_prim<B, MIXED>(sQ, (ci + 2) + G * (cj + 2), uin, P, eosk);
+      if (owner)
+        cold |= store_prim<B, MIXED, STIFF>(sQ, (ci + 2) + G * (cj + 2), uin, P, eosk);
       if (tid < 10)
         sSlot[tid] = slot_v;
       if (tid == 10)
         sNext = next_v;
-      __syncthreads();
+      if constexpr (fast64)
+        cold = __syncthreads_or(cold) != 0;
+      else
+        __syncthreads();
       // the next block of this CTA: its own cells and table rows into L2 while
       // this block computes (its gather then hits L2 instead of HBM)
       if (tid < 3 && sNext < nwalk)
@@ -759,6 +1072,7 @@ step2d_kernel(StepArgs a)
       // (the block, then the row or column beyond each face, without gaps: the
       // ring's corners are never a face neighbour; r: the cell's index in the
       // ring layout)
+      const bool cold0 = cold;
       for (int h = tid; h < NC + 4 * B; h += NT)
       {
         int ri, rj;
@@ -776,68 +1090,68 @@ step2d_kernel(StepArgs a)
         }
         const int r = (ri + 1) + S * (rj + 1);
         const int gi = (ri + 2) + G * (rj + 2);
-        R         q[5], dqx[5], dqy[5];
-        R st;
-        if constexpr (MIXED)
-          st = P.f_slope_type;
+        if constexpr (!MIXED)
+        {
+          if constexpr (STIFF == 2)
+            hancock_ref64<B>(sQ, sRec, gi, r, dtdx_r, P);
+          else
+          {
+            if (cold0)
+              hancock_cold64<B>(sQ, sRec, gi, r, dtdx_r, &P);
+            else
+              cold |= hancock_fast64<B>(sQ, sRec, gi, r, dtdx_r, P);
+          }
+        }
         else
-          st = P.slope_type;
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
         {
-          const R * Qk = sQ + k * GG;
-          q[k] = Qk[gi];
-          dqx[k] = slope_scalar<R>(q[k], Qk[gi + 1], Qk[gi - 1], st);
-          dqy[k] = slope_scalar<R>(q[k], Qk[gi + G], Qk[gi - G], st);
-          sRec[k * SS + r] = dqx[k];
-          sRec[(5 + k) * SS + r] = dqy[k];
-        }
-        const R a0 = sQ[5 * GG + gi];
-        if (P.integrator == 0)
-        {
-          // Hancock half-step source (ComputeFluxesAndStoreFunctor.cpp:174-199)
-          const R r0 = q[0], r1 = q[1], p = q[2], u = q[3], v = q[4];
-          const R rr = r0 + r1;
-          R       c;
-          if constexpr (MIXED)
-            c = sound_speed_eos(P, eosk, rr, p, a0, r0, r1);
-          else
-            c = sound_speed_mix(P, rr, p, a0, 1 - a0, r0, r1);
-          const R drx0 = dqx[0], drx1 = dqx[1], dpx = dqx[2], dux = dqx[3], dvx = dqx[4];
-          const R dry0 = dqy[0], dry1 = dqy[1], dpy = dqy[2], duy = dqy[3], dvy = dqy[4];
-          const R dtdy = dtdx_r;
-          const R sr0 = (-u * (drx0 + drx1) - dux * rr) * dtdx_r + (-v * (dry0 + dry1) - dvy * rr) * dtdy;
-          const R sr0_0 = sr0 * a0;
-          const R sr0_1 = sr0 * (R(1) - a0);
-          const R su0 = (-u * dux - dpx / rr) * dtdx_r + (-v * duy) * dtdy;
-          const R sv0 = (-u * dvx) * dtdx_r + (-v * dvy - dpy / rr) * dtdy;
-          const R sp0 = (-u * dpx - dux * rr * c * c) * dtdx_r + (-v * dpy - dvy * rr * c * c) * dtdy;
-          if constexpr (MIXED)
-          {
-            // the mixed form stores the predicted centre value q + hs
-            sRec[10 * SS + r] = q[0] + R(0.5) * sr0_0;
-            sRec[11 * SS + r] = q[1] + R(0.5) * sr0_1;
-            sRec[12 * SS + r] = q[2] + R(0.5) * sp0;
-            sRec[13 * SS + r] = q[3] + R(0.5) * su0;
-            sRec[14 * SS + r] = q[4] + R(0.5) * sv0;
-          }
-          else
-          {
-            sRec[10 * SS + r] = R(0.5) * sr0_0;
-            sRec[11 * SS + r] = R(0.5) * sr0_1;
-            sRec[12 * SS + r] = R(0.5) * sp0;
-            sRec[13 * SS + r] = R(0.5) * su0;
-            sRec[14 * SS + r] = R(0.5) * sv0;
-          }
-        }
-        else if constexpr (MIXED)
-        {
+          float       q[5], dqx[5], dqy[5];
+          const float st = P.f_slope_type;
 #pragma unroll
           for (int k = 0; k < 5; ++k)
-            sRec[(10 + k) * SS + r] = q[k];
+          {
+            const float * Qk = sQ + k * GG;
+            q[k] = Qk[gi];
+            dqx[k] = slope_scalar<float>(q[k], Qk[gi + 1], Qk[gi - 1], st);
+            dqy[k] = slope_scalar<float>(q[k], Qk[gi + G], Qk[gi - G], st);
+            sRec[k * SS + r] = dqx[k];
+            sRec[(5 + k) * SS + r] = dqy[k];
+          }
+          const float a0 = sQ[5 * GG + gi];
+          if (P.integrator == 0)
+          {
+            // Hancock half-step source (ComputeFluxesAndStoreFunctor.cpp:174-199)
+            const float r0 = q[0], r1 = q[1], p = q[2], u = q[3], v = q[4];
+            const float rr = r0 + r1;
+            const float c = sound_speed_eos(P, eosk, rr, p, a0, r0, r1);
+            const float drx0 = dqx[0], drx1 = dqx[1], dpx = dqx[2], dux = dqx[3], dvx = dqx[4];
+            const float dry0 = dqy[0], dry1 = dqy[1], dpy = dqy[2], duy = dqy[3], dvy = dqy[4];
+            const float dtdy = dtdx_r;
+            const float sr0 = (-u * (drx0 + drx1) - dux * rr) * dtdx_r + (-v * (dry0 + dry1) - dvy * rr) * dtdy;
+            const float sr0_0 = sr0 * a0;
+            const float sr0_1 = sr0 * (1.0f - a0);
+            const float su0 = (-u * dux - dpx / rr) * dtdx_r + (-v * duy) * dtdy;
+            const float sv0 = (-u * dvx) * dtdx_r + (-v * dvy - dpy / rr) * dtdy;
+            const float sp0 = (-u * dpx - dux * rr * c * c) * dtdx_r + (-v * dpy - dvy * rr * c * c) * dtdy;
+            // the predicted centre value q + hs
+            sRec[10 * SS + r] = q[0] + 0.5f * sr0_0;
+            sRec[11 * SS + r] = q[1] + 0.5f * sr0_1;
+            sRec[12 * SS + r] = q[2] + 0.5f * sp0;
+            sRec[13 * SS + r] = q[3] + 0.5f * su0;
+            sRec[14 * SS + r] = q[4] + 0.5f * sv0;
+          }
+          else
+          {
+#pragma unroll
+            for (int k = 0; k < 5; ++k)
+              sRec[(10 + k) * SS + r] = q[k];
+          }
         }
       }
-      __syncthreads();
+      if constexpr (fast64)
+        cold = __syncthreads_or(cold) != 0;
+      else
+        __syncthreads();
+      const bool cold1 = cold;
 
       // ---------------- phase 3: faces (X then Y) -> HLLC -> shared fluxes
       if constexpr (MIXED)
@@ -851,53 +1165,16 @@ step2d_kernel(StepArgs a)
         }
       }
       else
-      for (int f = tid; f < 2 * NFF; f += NT)
       {
-        const int dir = f >= NFF ? 1 : 0;
-        const int ff = f - dir * NFF;
-        int       li, lj, ri, rj;
-        if (dir == 0)
+        for (int f = tid; f < 2 * NFF; f += NT)
         {
-          const int fi = ff % (B + 1), fj = ff / (B + 1);
-          li = fi - 1;
-          lj = fj;
-          ri = fi;
-          rj = fj;
+          if constexpr (STIFF == 2)
+            face_flux_ref64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
+          else if (cold1)
+            face_flux_cold64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, &P);
+          else
+            cold |= face_flux_fast64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
         }
-        else
-        {
-          const int fi = ff % B, fj = ff / B;
-          li = fi;
-          lj = fj - 1;
-          ri = fi;
-          rj = fj;
-        }
-        R qL[6], qR[6], fl[8];
-        face_state<B, MIXED>(sQ, sRec, li, lj, dir, +1, P, qL);
-        face_state<B, MIXED>(sQ, sRec, ri, rj, dir, -1, P, qR);
-        if (dir == 1)
-        {
-          R t = qL[3];
-          qL[3] = qL[4];
-          qL[4] = t;
-          t = qR[3];
-          qR[3] = qR[4];
-          qR[4] = t;
-        }
-        if constexpr (MIXED)
-          hllc_fp32<2>(qL, qR, P.f_xi[0], P.f_xi[1], P.f_gpx[0], P.f_gpx[1], P.f_smallr, P.f_smallp, P.f_smallc, fl);
-        else
-          hllc_fp64<2>(qL, qR, P, fl);
-        if (dir == 1)
-        {
-          const R t = fl[H::FU];
-          fl[H::FU] = fl[H::FV];
-          fl[H::FV] = t;
-        }
-        R * dst = dir == 0 ? sFx : sFy;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          dst[k * NFF + ff] = fl[k] * dtdx_r;
       }
       // the own cell's state for the update: the FP32-bulk form without the
       // tail reflux reads it again (an L2 hit, in flight while the CTA waits at
@@ -905,12 +1182,15 @@ step2d_kernel(StepArgs a)
       // the slope and face phases (-2 % on the droplet batch; the tail-reflux
       // kernel, with its few rounds of blocks, was 0.4 % slower with it)
       double uown[H::NV];
-      if constexpr (MIXED && !FUSED)
+      if constexpr (!FUSED)
       {
-        const double * base = a.U + (size_t)n * H::NV * NC + tid;
+        if (owner)
+        {
+          const double * base = a.U + (size_t)n * H::NV * NC + tid;
 #pragma unroll
-        for (int v = 0; v < H::NV; ++v)
-          uown[v] = __ldcg(base + v * NC);
+          for (int v = 0; v < H::NV; ++v)
+            uown[v] = __ldcg(base + v * NC);
+        }
       }
       else
       {
@@ -918,7 +1198,10 @@ step2d_kernel(StepArgs a)
         for (int v = 0; v < H::NV; ++v)
           uown[v] = uin[v];
       }
-      __syncthreads();
+      if constexpr (fast64)
+        cold = __syncthreads_or(cold) != 0;
+      else
+        __syncthreads();
 
       // ---------------- publish coarse/fine records (AMR only)
       if (a.m.reflux_slot)
@@ -970,14 +1253,31 @@ step2d_kernel(StepArgs a)
       }
       DtT    m_inv = DtT(0);
       double u2[H::NV];
-      if (!deferred)
+      if (owner && !deferred)
       {
         if constexpr (MIXED)
           m_inv = update_mixed<B>(uown, u2, sFx, sFy, ci, cj, d2f_fast(dx), P, eosk, a.invdt != nullptr);
-        else
-          m_inv = update_fp64<B>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr);
         double * out = a.U2 + (size_t)n * H::NV * NC + tid;
-        bool     finite = true;
+        if constexpr (!MIXED && STIFF == 2)
+          m_inv = update_fp64<B>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr);
+        else if constexpr (!MIXED)
+        {
+          bool bad = cold;
+          if (!bad)
+            m_inv = update_fast64<B>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr, bad);
+          if (bad)
+          {
+            State64<2> st;
+#pragma unroll
+            for (int v = 0; v < H::NV; ++v)
+              st.v[v] = uown[v];
+            m_inv = update_cold64<B>(st, out, sFx, sFy, ci, cj, dx, &P, a.invdt != nullptr);
+#pragma unroll
+            for (int v = 0; v < H::NV; ++v)
+              u2[v] = out[v * NC];
+          }
+        }
+        bool finite = true;
 #pragma unroll
         for (int v = 0; v < H::NV; ++v)
         {
@@ -999,11 +1299,14 @@ step2d_kernel(StepArgs a)
         // block (FillOutside: the last applicable face's copy rule), from the
         // new state staged in the (now free) slope area
         double * sTw = reinterpret_cast<double *>(sRec);
+        if (owner)
+        {
 #pragma unroll
-        for (int v = 0; v < H::NV; ++v)
-          sTw[v * NC + tid] = u2[v];
+          for (int v = 0; v < H::NV; ++v)
+            sTw[v * NC + tid] = u2[v];
+        }
         __syncthreads();
-        for (int t = sSlot[8]; t < sSlot[9]; ++t)
+        for (int t = sSlot[8]; owner && t < sSlot[9]; ++t)
         {
           const int e = a.m.twin_list[t];
           const int o = e >> 3, face = e & 7, dir = face >> 1, bc = P.bc[face];
@@ -1022,9 +1325,14 @@ step2d_kernel(StepArgs a)
       }
       if (a.invdt)
       {
+        if constexpr (MIXED)
+        {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-          m_inv = fmax(m_inv, __shfl_xor_sync(0xffffffffu, m_inv, o));
+          for (int o = 16; o > 0; o >>= 1)
+            m_inv = fmax(m_inv, __shfl_xor_sync(0xffffffffu, m_inv, o));
+        }
+        else
+          m_inv = warp_max_pos64(m_inv);
         if ((tid & 31) == 0)
           sRed[tid >> 5] = m_inv;
         __syncthreads();

@@ -1,0 +1,94 @@
+"""The FP64 form's fast arithmetic (csrc/g5_fast64.cuh) where its shortcuts
+could fail: zeros, pure materials, values outside its range (which take the
+reference arithmetic), non-physical states, every constant of the mixture.
+Bit for bit against the CPU oracle."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from godunov_five_eq_gb300 import configs  # noqa: E402
+from godunov_five_eq_gb300.implem import GodunovImplemGB300  # noqa: E402
+from oracle.oracle import Oracle  # noqa: E402
+from tests.helpers import amr_mesh, smooth_state, water_air_params  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+GASES = {"ideal": ((1.4, 1.648), (0.0, 0.0)), "first": ((4.4, 1.4), (6e8, 0.0)), "second": ((1.4, 4.4), (0.0, 6e8)), "both": ((4.4, 3.0), (6e8, 1e8))}
+
+
+def build(dim, b, kind, gas, **kw):
+    mesh, t = amr_mesh(dim=dim, b=b, nref=3, lmin=1, lmax=2, seed=5)
+    p = water_air_params(t, dim=dim, b=b, **kw)
+    p.gamma, p.pinf = GASES[gas]
+    U = smooth_state(mesh, t, p)
+    I = configs.ids(dim)
+    n = t.n_owned
+    V = U[:n]
+    rng = np.random.default_rng(3)
+    mom = [I["IU"], I["IV"]] + ([I["IW"]] if dim == 3 else [])
+
+    def state(a0, vel):
+        pr = np.full_like(a0, 1e5)
+        pr[: n // 2] = 1.3e5
+        U[:n] = np.moveaxis(configs.prim_to_cons(dim, p, a0, a0 * 1000.0, (1.0 - a0) * 1.2, pr, vel), 0, 1)
+
+    a0 = V[:, I["IA0"]].copy()
+    zero = [0.0 * a0 for _ in range(dim)]
+    if kind == "rest":
+        state(a0, zero)
+    elif kind == "pure":
+        state(np.where(a0 > 0.5, 1.0, 0.0), [7.0 + 0.0 * a0] + zero[1:])
+    elif kind in ("tiny", "subnormal", "huge", "nan"):
+        # a few cells far from the rest: the last owned blocks only, so that both arithmetics run
+        val = {"tiny": 1e-280, "subnormal": 3e-310, "huge": 1e215, "nan": np.nan}[kind]
+        state(a0, [1e-200 * rng.standard_normal(a0.shape) for _ in range(dim)])
+        for v in mom[:2] if kind != "nan" else mom[:1]:
+            V[-1, v, rng.integers(0, t.ncell, 5)] = val
+    elif kind == "negative":
+        cells = rng.random(a0.shape) < 0.02
+        V[:, I["IE"]] = np.where(cells, V[:, I["IE"]] * 0.2, V[:, I["IE"]])
+    return t, p, U
+
+
+CASES = [
+    (2, 16, "smooth", "ideal", {}),
+    (2, 16, "smooth", "second", dict(slope_type=2.0, source_term=1)),
+    (2, 8, "smooth", "both", dict(thinc=1, source_term=1)),
+    (2, 8, "smooth", "first", dict(integrator=1, slope_type=0.0)),
+    (2, 16, "rest", "first", {}),
+    (2, 8, "rest", "ideal", dict(slope_type=2.0)),
+    (2, 16, "pure", "first", {}),
+    (2, 8, "pure", "ideal", dict(thinc=1)),
+    (2, 16, "tiny", "ideal", {}),
+    (2, 8, "subnormal", "first", {}),
+    (2, 16, "huge", "ideal", {}),
+    (2, 16, "nan", "ideal", {}),
+    (2, 8, "negative", "ideal", {}),
+    (2, 16, "negative", "both", dict(slope_type=2.0)),
+]
+
+
+@pytest.mark.parametrize("dim,b,kind,gas,kw", CASES, ids=["-".join([str(c[0]), str(c[1]), c[2], c[3]] + sorted(c[4])) for c in CASES])
+def test_fast64_step_matches_oracle(dim, b, kind, gas, kw):
+    t, p, U = build(dim, b, kind, gas, **kw)
+    o = Oracle(t, p)
+    o.fill_outside(U)
+    dt = 1e-6
+    with np.errstate(all="ignore"):
+        ref = o.step(U, dt)[: t.n_owned]
+        full = np.zeros_like(U)
+        full[: t.n_owned] = ref
+        inv_ref = o.inv_dt(full)
+    impl = GodunovImplemGB300(p, t)
+    d_U = torch.from_numpy(U).cuda()
+    d_U2 = torch.zeros_like(d_U)
+    inv = torch.zeros(t.n_inst, dtype=torch.float64, device="cuda")
+    impl.do_time_step(d_U, d_U2, dt, mode="fp64", inv_dt_out=inv)
+    torch.cuda.synchronize()
+    got = d_U2.cpu().numpy()[: t.n_owned]
+    assert np.array_equal(got, ref, equal_nan=True), f"{(~((got == ref) | (np.isnan(got) & np.isnan(ref)))).sum()} values differ"
+    if kind == "nan":
+        assert impl.status() != 0
+    else:
+        assert np.array_equal(inv.cpu().numpy(), inv_ref)
