@@ -350,4 +350,37 @@ finish_fast64(double * u2, double dx, const PhysParams & P, bool want_dt, bool &
   return r;
 }
 
+// FP64 cold path: the reference's primitives of a cell whose values leave the
+// range of the fast form
+template <int DIM>
+struct State64
+{
+  double v[V<DIM>::NV];
+};
+
+template <int DIM>
+__device__ __noinline__ void
+prim_ref64(State64<DIM> u, const PhysParams * P, double * sQ, int stride)
+{
+  double q[V<DIM>::NQ];
+  prim_fp64<DIM>(u.v, q, *P);
+  for (int k = 0; k < V<DIM>::NQ; ++k)
+    sQ[k * stride] = q[k];
+}
+
+// THINC value of the volume fraction at the cell's face
+// (scheme/ComputeFluxesAndStoreTHINCFunctor.cpp:122-283): a0 the cell's value,
+// aM and aP its neighbours' along the direction, nd the Youngs normal's
+// component, bs = +-1 the side
+__device__ __forceinline__ double
+thinc_alpha64(double a0, double aM, double aP, double nd, double bs, double thinc_beta)
+{
+  const double beta = thinc_beta * nd + 0.01;
+  const double Aa = (aP + aM) / 2.0;
+  const double Bb = (aP - aM) / 2.0;
+  const double C = tanh_d(0.5 * beta);
+  const double D = tanh_d(0.5 * beta * (a0 - Aa) / Bb);
+  return Aa + bs * Bb * (C + bs * D / C) / (1.0 + bs * D);
+}
+
 } // namespace g5

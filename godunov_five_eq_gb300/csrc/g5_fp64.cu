@@ -7,6 +7,7 @@
 #include "g5_prolong.cuh"
 #include "g5_step2d.cuh"
 #include "g5_step3d.cuh"
+#include "g5_step3d_f64.cuh"
 
 namespace g5
 {
@@ -95,31 +96,47 @@ occupancy2d()
   return occ;
 }
 
-template <bool MIXED>
+// the 3D step: the fast form's kernel, or the reference arithmetic's
+template <int STIFF>
+struct Step3dLaunch
+{
+  static constexpr int    NT = STIFF == FAST64 ? Step3D64::NT : Step3DTraits<false>::NT;
+  static constexpr size_t smem_bytes = STIFF == FAST64 ? Step3D64::smem_bytes : Step3DTraits<false>::smem_bytes;
+  static auto
+  kernel()
+  {
+    if constexpr (STIFF == FAST64)
+      return step3d_fast64_kernel;
+    else
+      return step3d_kernel<false>;
+  }
+};
+
+template <int STIFF>
+static int
+occupancy3d()
+{
+  using K = Step3dLaunch<STIFF>;
+  cudaFuncSetAttribute(K::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem_bytes);
+  int occ = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, K::kernel(), K::NT, K::smem_bytes);
+  return occ;
+}
+
+template <int STIFF>
 static cudaError_t
 launch_step3d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches)
 {
-  using T = Step3DTraits<MIXED>;
-  static bool configured = false;
-  static int  occ = 1;
-  if (!configured)
-  {
-    cudaError_t e = cudaFuncSetAttribute(step3d_kernel<MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
-    if (e != cudaSuccess)
-      return e;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step3d_kernel<MIXED>, T::NT, T::smem_bytes);
-    if (occ < 1)
-      occ = 1;
-    configured = true;
-  }
-  const int per_sm = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
-  int       grid = num_sms() * per_sm;
+  using K = Step3dLaunch<STIFF>;
+  static const int occ = std::max(1, occupancy3d<STIFF>());
+  const int        per_sm = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
+  int              grid = num_sms() * per_sm;
   if (grid > step_count(a))
     grid = step_count(a);
   cudaError_t e = cudaSuccess;
   if (grid >= 1)
   {
-    step3d_kernel<MIXED><<<grid, T::NT, T::smem_bytes, s>>>(a);
+    K::kernel()<<<grid, K::NT, K::smem_bytes, s>>>(a);
     ++*launches;
     e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -128,22 +145,11 @@ launch_step3d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launche
   if (a.m.n_defer > 0)
   {
     const int n = a.m.n_defer * 64;
-    reflux3d_kernel<MIXED><<<(n + 31) / 32, 32, 0, s>>>(a);
+    reflux3d_kernel<false><<<(n + 31) / 32, 32, 0, s>>>(a);
     ++*launches;
     e = cudaGetLastError();
   }
   return e;
-}
-
-template <bool MIXED>
-static int
-occupancy3d()
-{
-  using T = Step3DTraits<MIXED>;
-  cudaFuncSetAttribute(step3d_kernel<MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step3d_kernel<MIXED>, T::NT, T::smem_bytes);
-  return occ;
 }
 
 bool
@@ -254,7 +260,7 @@ launch_step_fp64(int dim, int b, const StepArgs & a, int ctas_per_sm, cudaStream
   if (dim == 2 && b == 8)
     return fast64_case(a.p) ? launch_step2d<8, FAST64>(a, ctas_per_sm, s, launches) : launch_step2d<8, REF64>(a, ctas_per_sm, s, launches);
   if (dim == 3 && b == 8)
-    return launch_step3d<false>(a, ctas_per_sm, s, launches);
+    return fast64_case(a.p) ? launch_step3d<FAST64>(a, ctas_per_sm, s, launches) : launch_step3d<REF64>(a, ctas_per_sm, s, launches);
   return cudaErrorInvalidValue;
 }
 
@@ -266,7 +272,7 @@ step_max_ctas_per_sm_fp64(int dim, int b)
   if (dim == 2 && b == 8)
     return std::min(occupancy2d<8, FAST64>(), occupancy2d<8, REF64>());
   if (dim == 3 && b == 8)
-    return occupancy3d<false>();
+    return std::min(occupancy3d<FAST64>(), occupancy3d<REF64>());
   return 0;
 }
 

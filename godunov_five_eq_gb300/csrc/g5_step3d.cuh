@@ -372,7 +372,7 @@ face_state3(const typename Step3DTraits<MIXED>::R * sQ,
       }
       q[k] = t;
       if (hancock)
-        q[k] += sHS[k * SSS + si];
+        q[k] += R(0.5) * sHS[k * SSS + si]; // (the FP64 form stores the source without its factor 1/2)
     }
   }
   const R a0 = sQ[6 * GGG + gi];
@@ -407,8 +407,8 @@ face_state3(const typename Step3DTraits<MIXED>::R * sQ,
       R       q1 = r1 + r1 / (R(1) - a0) * (a0 - af);
       if (hancock)
       {
-        q0 += sHS[0 * SSS + si];
-        q1 += sHS[1 * SSS + si];
+        q0 += (MIXED ? R(1) : R(0.5)) * sHS[0 * SSS + si];
+        q1 += (MIXED ? R(1) : R(0.5)) * sHS[1 * SSS + si];
       }
       q[0] = q0;
       q[1] = q1;
@@ -477,6 +477,41 @@ face_flux3(const typename Step3DTraits<MIXED>::R * sQ, const typename Step3DTrai
 #pragma unroll
   for (int k = 0; k < 9; ++k)
     sFd[k * NFF + f] = fl[k] * dtdx_r;
+}
+
+// FP64: Hancock half-step source (ComputeFluxesAndStoreFunctor.cpp:273-306,
+// without its factor 1/2) of the ring cell r, ghosted index gi, in the
+// reference's arithmetic
+__device__ __forceinline__ void
+hancock_ref3(const double * sQ, double * sHS, int gi, int r, double dtdx, const PhysParams & P)
+{
+  using T = Step3DTraits<false>;
+  constexpr int G = T::G, GG = T::GG, GGG = T::GGG, SSS = T::SSS;
+  if (P.integrator != 0)
+    return;
+  double dx[6], dy[6], dz[6], q[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+  {
+    const double * Qk = sQ + k * GGG;
+    q[k] = Qk[gi];
+    dx[k] = slope_at<double>(Qk, gi, 1, P.slope_type);
+    dy[k] = slope_at<double>(Qk, gi, G, P.slope_type);
+    dz[k] = slope_at<double>(Qk, gi, GG, P.slope_type);
+  }
+  const double a0 = sQ[6 * GGG + gi];
+  const double r0 = q[0], r1 = q[1], p = q[2], u = q[3], v = q[4], w = q[5];
+  const double rr = r0 + r1;
+  const double c = sound_speed_mix(P, rr, p, a0, 1 - a0, r0, r1);
+  const double sr0 = (-u * (dx[0] + dx[1]) - dx[3] * rr) * dtdx + (-v * (dy[0] + dy[1]) - dy[4] * rr) * dtdx +
+                     (-w * (dz[0] + dz[1]) - dz[5] * rr) * dtdx;
+  sHS[0 * SSS + r] = sr0 * a0;
+  sHS[1 * SSS + r] = sr0 * (1.0 - a0);
+  sHS[2 * SSS + r] = (-u * dx[2] - dx[3] * rr * c * c) * dtdx + (-v * dy[2] - dy[4] * rr * c * c) * dtdx +
+                     (-w * dz[2] - dz[5] * rr * c * c) * dtdx;
+  sHS[3 * SSS + r] = (-u * dx[3] - dx[2] / rr) * dtdx + (-v * dy[3]) * dtdx + (-w * dz[3]) * dtdx;
+  sHS[4 * SSS + r] = (-u * dx[4]) * dtdx + (-v * dy[4] - dy[2] / rr) * dtdx + (-w * dz[4]) * dtdx;
+  sHS[5 * SSS + r] = (-u * dx[5]) * dtdx + (-v * dy[5]) * dtdx + (-w * dz[5] - dz[2] / rr) * dtdx;
 }
 
 // one direction of update_U (FP64, reference order); returns nothing, u2 updated
@@ -752,63 +787,48 @@ step3d_kernel(StepArgs a)
       }
       const int r = (ri + 1) + S * (rj + 1) + SS * (rk + 1);
       const int gi = (ri + 2) + G * (rj + 2) + GG * (rk + 2);
-      if (P.integrator == 0)
+      if constexpr (!MIXED)
+        hancock_ref3(sQ, sHS, gi, r, dtdx_r, P);
+      else if (P.integrator == 0)
       {
-        R st;
-        if constexpr (MIXED)
-          st = P.f_slope_type;
-        else
-          st = P.slope_type;
-        R dq[3][6], q[6];
+        const float st = P.f_slope_type;
+        float       dq[3][6], q[6];
 #pragma unroll
         for (int k = 0; k < 6; ++k)
         {
-          const R * Qk = sQ + k * GGG;
+          const float * Qk = sQ + k * GGG;
           q[k] = Qk[gi];
-          if constexpr (MIXED)
-          {
-            // x and y in one packed evaluation, z alone
-            const float2 d = slope_pair(make_float2(q[k], q[k]), make_float2(Qk[gi + 1], Qk[gi + G]), make_float2(Qk[gi - 1], Qk[gi - G]), st);
-            dq[0][k] = d.x;
-            dq[1][k] = d.y;
-          }
-          else
-          {
-            dq[0][k] = slope_at<R>(Qk, gi, 1, st);
-            dq[1][k] = slope_at<R>(Qk, gi, G, st);
-          }
-          dq[2][k] = slope_at<R>(Qk, gi, GG, st);
+          // x and y in one packed evaluation, z alone
+          const float2 d = slope_pair(make_float2(q[k], q[k]), make_float2(Qk[gi + 1], Qk[gi + G]), make_float2(Qk[gi - 1], Qk[gi - G]), st);
+          dq[0][k] = d.x;
+          dq[1][k] = d.y;
+          dq[2][k] = slope_at<float>(Qk, gi, GG, st);
         }
-        const R a0 = sQ[6 * GGG + gi];
-        const R r0 = q[0], r1 = q[1], p = q[2], u = q[3], v = q[4], w = q[5];
-        const R rr = r0 + r1;
-        R       c;
-        if constexpr (MIXED)
-          c = sound_speed_eos(P, eosk, rr, p, a0, r0, r1);
-        else
-          c = sound_speed_mix(P, rr, p, a0, 1 - a0, r0, r1);
-        const R drx0 = dq[0][0], drx1 = dq[0][1], dpx = dq[0][2], dux = dq[0][3], dvx = dq[0][4], dwx = dq[0][5];
-        const R dry0 = dq[1][0], dry1 = dq[1][1], dpy = dq[1][2], duy = dq[1][3], dvy = dq[1][4], dwy = dq[1][5];
-        const R drz0 = dq[2][0], drz1 = dq[2][1], dpz = dq[2][2], duz = dq[2][3], dvz = dq[2][4], dwz = dq[2][5];
-        const R dtdx = dtdx_r, dtdy = dtdx_r, dtdz = dtdx_r;
+        const float a0 = sQ[6 * GGG + gi];
+        const float r0 = q[0], r1 = q[1], p = q[2], u = q[3], v = q[4], w = q[5];
+        const float rr = r0 + r1;
+        const float c = sound_speed_eos(P, eosk, rr, p, a0, r0, r1);
+        const float drx0 = dq[0][0], drx1 = dq[0][1], dpx = dq[0][2], dux = dq[0][3], dvx = dq[0][4], dwx = dq[0][5];
+        const float dry0 = dq[1][0], dry1 = dq[1][1], dpy = dq[1][2], duy = dq[1][3], dvy = dq[1][4], dwy = dq[1][5];
+        const float drz0 = dq[2][0], drz1 = dq[2][1], dpz = dq[2][2], duz = dq[2][3], dvz = dq[2][4], dwz = dq[2][5];
+        const float dtdx = dtdx_r, dtdy = dtdx_r, dtdz = dtdx_r;
         // ComputeFluxesAndStoreFunctor.cpp:273-306
-        const R sr0 = (-u * (drx0 + drx1) - dux * rr) * dtdx + (-v * (dry0 + dry1) - dvy * rr) * dtdy +
-                      (-w * (drz0 + drz1) - dwz * rr) * dtdz;
-        const R sr0_0 = sr0 * a0;
-        const R sr0_1 = sr0 * (R(1) - a0);
-        const R su0 = (-u * dux - dpx / rr) * dtdx + (-v * duy) * dtdy + (-w * duz) * dtdz;
-        const R sv0 = (-u * dvx) * dtdx + (-v * dvy - dpy / rr) * dtdy + (-w * dvz) * dtdz;
-        const R sw0 = (-u * dwx) * dtdx + (-v * dwy) * dtdy + (-w * dwz - dpz / rr) * dtdz;
-        const R sp0 = (-u * dpx - dux * rr * c * c) * dtdx + (-v * dpy - dvy * rr * c * c) * dtdy +
-                      (-w * dpz - dwz * rr * c * c) * dtdz;
-        sHS[0 * SSS + r] = R(0.5) * sr0_0;
-        sHS[1 * SSS + r] = R(0.5) * sr0_1;
-        sHS[2 * SSS + r] = R(0.5) * sp0;
-        sHS[3 * SSS + r] = R(0.5) * su0;
-        sHS[4 * SSS + r] = R(0.5) * sv0;
-        sHS[5 * SSS + r] = R(0.5) * sw0;
+        const float sr0 = (-u * (drx0 + drx1) - dux * rr) * dtdx + (-v * (dry0 + dry1) - dvy * rr) * dtdy +
+                          (-w * (drz0 + drz1) - dwz * rr) * dtdz;
+        const float sr0_0 = sr0 * a0;
+        const float sr0_1 = sr0 * (1.0f - a0);
+        const float su0 = (-u * dux - dpx / rr) * dtdx + (-v * duy) * dtdy + (-w * duz) * dtdz;
+        const float sv0 = (-u * dvx) * dtdx + (-v * dvy - dpy / rr) * dtdy + (-w * dvz) * dtdz;
+        const float sw0 = (-u * dwx) * dtdx + (-v * dwy) * dtdy + (-w * dwz - dpz / rr) * dtdz;
+        const float sp0 = (-u * dpx - dux * rr * c * c) * dtdx + (-v * dpy - dvy * rr * c * c) * dtdy +
+                          (-w * dpz - dwz * rr * c * c) * dtdz;
+        sHS[0 * SSS + r] = 0.5f * sr0_0;
+        sHS[1 * SSS + r] = 0.5f * sr0_1;
+        sHS[2 * SSS + r] = 0.5f * sp0;
+        sHS[3 * SSS + r] = 0.5f * su0;
+        sHS[4 * SSS + r] = 0.5f * sv0;
+        sHS[5 * SSS + r] = 0.5f * sw0;
       }
-
     }
     __syncthreads();
 

@@ -1,0 +1,578 @@
+// g5_step3d_f64.cuh — the 3D block timestep in FP64 with the fast arithmetic
+// of g5_fast64.cuh (stiffened gases).  The phases, the shared arrays and the
+// coarse/fine records are those of step3d_kernel (g5_step3d.cuh), whose FP64
+// form is the reference arithmetic; the results are the same doubles.
+//
+// One CTA of 576 threads per 8^3 block: the 576 faces of a direction take one
+// round (512 threads took two, the second with 64 faces), at 112 registers.
+// The three directions run through one copy of the face code (a run-time
+// direction): three would not fit the instruction cache.  A value outside the
+// fast form's range sends the rest of the block to the reference arithmetic
+// (the `cold` functions).
+#pragma once
+
+#include "g5_fast64.cuh"
+#include "g5_step3d.cuh"
+
+namespace g5
+{
+
+struct Step3D64
+{
+  using T = Step3DTraits<false>;
+  static constexpr int NT = 576;
+  static constexpr int NTHINC = 640; // cells with a face of one direction
+  // sQ, sHS, the mixture's S of the ring, the face fluxes of one direction
+  static constexpr int OFF_HS = T::NQ * T::GGG, OFF_S = OFF_HS + T::NHS * T::SSS, OFF_F = OFF_S + T::SSS;
+  static constexpr size_t smem_bytes = sizeof(double) * (size_t)(OFF_F + T::NF * T::NFF) + 64;
+  static_assert(NT == T::NFF, "one round of faces per direction");
+};
+
+// the unit stride of a direction in the ghosted (12^3) and ring (10^3) arrays
+__device__ __forceinline__ int
+ghost_stride3(int dir)
+{
+  return dir == 0 ? 1 : (dir == 1 ? Step3D64::T::G : Step3D64::T::GG);
+}
+__device__ __forceinline__ int
+ring_stride3(int dir)
+{
+  return dir == 0 ? 1 : (dir == 1 ? Step3D64::T::S : Step3D64::T::SS);
+}
+
+// Hancock source of one face-neighbour cell (hancock_ref3 in the fast
+// operations) and the mixture's S; true when a value left the range
+__device__ __forceinline__ bool
+hancock_fast3(const double * sQ, double * sHS, double * sS, int gi, int r, double dtdx, const PhysParams & P)
+{
+  using T = Step3D64::T;
+  constexpr int G = T::G, GG = T::GG, GGG = T::GGG, SSS = T::SSS;
+  bool          bad = false;
+  const double  a0 = sQ[6 * GGG + gi], a1 = 1.0 - a0;
+  const double  S = mix_S64(P, a0, a1, bad);
+  sS[r] = S;
+  if (P.integrator != 0)
+    return bad;
+  const int     st = P.st64;
+  const bool    stiff = P.pi64 != 0;
+  const double  p = sQ[2 * GGG + gi];
+  const double  rr = sQ[gi] + sQ[GGG + gi];
+  const Recip64 rd = recip64(rr, bad);
+  const double  c = sound64(rr, p, S, stiff ? mix_PI64(P, a0, a1, bad) : 0.0, stiff, bad);
+  // each source is a sum over the directions, x first
+  double sr = 0.0, sp = 0.0, sv[3] = { 0.0, 0.0, 0.0 };
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+  {
+    const int o = e == 0 ? 1 : (e == 1 ? G : GG);
+    double    d[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+    {
+      const double * Qk = sQ + k * GGG + gi;
+      d[k] = st != 0 ? slope_fast64(Qk[0], Qk[o], Qk[-o], st, bad) : 0.0;
+    }
+    const double mu = -sQ[(3 + e) * GGG + gi];
+    const double dr = mul64(d[3 + e], rr, bad);
+    const double tr = mul64(mulh64(mu, d[0] + d[1], bad) - dr, dtdx, bad);
+    const double tp = mul64(mulh64(mu, d[2], bad) - mulh64(mul64(dr, c, bad), c, bad), dtdx, bad);
+    sr = e == 0 ? tr : sr + tr;
+    sp = e == 0 ? tp : sp + tp;
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+    {
+      double t = mulh64(mu, d[3 + f], bad);
+      if (f == e)
+        t = t - quot64(d[2], rd, bad);
+      t = mul64(t, dtdx, bad);
+      sv[f] = e == 0 ? t : sv[f] + t;
+    }
+  }
+  sHS[r] = mul64(sr, a0, bad);
+  sHS[SSS + r] = mul64(sr, a1, bad);
+  sHS[2 * SSS + r] = sp;
+#pragma unroll
+  for (int f = 0; f < 3; ++f)
+    sHS[(3 + f) * SSS + r] = sv[f];
+  return bad;
+}
+
+__device__ __noinline__ void
+hancock_cold3(const double * sQ, double * sHS, int gi, int r, double dtdx, const PhysParams * P)
+{
+  hancock_ref3(sQ, sHS, gi, r, dtdx, *P);
+}
+
+// the reconstructed state of one face side (face_state3<false>, the normal
+// velocity first) and the mixture's S; gi, si: the cell in the ghosted and
+// ring arrays, o the direction's stride, side +1 the cell's right face
+__device__ __forceinline__ double
+face_state_fast3(const double * sQ, const double * sHS, const double * sS, int gi, int si, int o, int dir, int side, const PhysParams & P, double * q,
+                 bool & bad)
+{
+  using T = Step3D64::T;
+  constexpr int G = T::G, GG = T::GG, GGG = T::GGG, SSS = T::SSS;
+  const double  off = side > 0 ? 0.5 : -0.5;
+  const int     st = P.st64;
+  const bool    hancock = P.integrator == 0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+  {
+    const int      from = k < 3 ? k : (k == 3 ? 3 + dir : (k == 3 + dir ? 3 : k));
+    const double * Qk = sQ + from * GGG + gi;
+    double         t = Qk[0];
+    if (st != 0)
+      t = __fma_rn(off, slope_fast64(t, Qk[o], Qk[-o], st, bad), t);
+    q[k] = hancock ? __fma_rn(0.5, sHS[from * SSS + si], t) : t;
+  }
+  const double a0 = sQ[6 * GGG + gi];
+  double       S = sS[si];
+  q[6] = a0;
+  if (P.thinc)
+  {
+    const double * A = sQ + 6 * GGG;
+    const double   aP = A[gi + o], aM = A[gi - o];
+    const bool     mono = (bits64(aP) > bits64(a0) && bits64(a0) > bits64(aM)) || (bits64(aP) < bits64(a0) && bits64(a0) < bits64(aM));
+    if (mono && bits64(a0) > bits64(P.thinc_eps) && bits64(a0) < bits64(1.0 - P.thinc_eps))
+    {
+      const double nd = youngs_abs_3d<double, G, GG>(A, gi, dir);
+      const double af = thinc_alpha64(a0, aM, aP, nd, side > 0 ? 1.0 : -1.0, P.thinc_beta);
+      const double r0 = sQ[gi], r1 = sQ[GGG + gi];
+      q[0] = r0 + r0 / a0 * (af - a0);
+      q[1] = r1 + r1 / (1.0 - a0) * (a0 - af);
+      if (hancock)
+      {
+        q[0] = __fma_rn(0.5, sHS[si], q[0]);
+        q[1] = __fma_rn(0.5, sHS[SSS + si], q[1]);
+      }
+      q[6] = af;
+      S = mix_S64(P, af, 1.0 - af, bad);
+    }
+  }
+  else
+  {
+    q[0] = max_pos64(q[0], P.smallr);
+    q[1] = max_pos64(q[1], P.smallr);
+  }
+  return S;
+}
+
+__device__ __noinline__ void
+face_flux_cold3(const double * sQ, const double * sHS, double * sF, int f, int dir, double dtdx, const PhysParams * P)
+{
+  if (dir == 0)
+    face_flux3<false, 0, -1>(sQ, sHS, f, sF, dtdx, *P);
+  else if (dir == 1)
+    face_flux3<false, 1, -1>(sQ, sHS, f, sF, dtdx, *P);
+  else
+    face_flux3<false, 2, -1>(sQ, sHS, f, sF, dtdx, *P);
+}
+
+// HLLC flux of face f of direction dir, scaled by dt/dx (face_flux3<false>)
+__device__ __forceinline__ bool
+face_flux_fast3(const double * sQ, const double * sHS, const double * sS, double * sF, int f, int dir, double dtdx, const PhysParams & P)
+{
+  using T = Step3D64::T;
+  using H = V<3>;
+  constexpr int B = T::B, G = T::G, GG = T::GG, S = T::S, SS = T::SS, NFF = T::NFF;
+  const int     ex = B + (dir == 0), ey = B + (dir == 1);
+  const int     fi = f % ex, fj = (f / ex) % ey, fk = f / (ex * ey);
+  const int     gR = (fi + 2) + G * (fj + 2) + GG * (fk + 2), sR = (fi + 1) + S * (fj + 1) + SS * (fk + 1);
+  const int     o = ghost_stride3(dir);
+  double        qL[7], qR[7], fl[9];
+  bool          bad = false;
+  const double  Sl = face_state_fast3(sQ, sHS, sS, gR - o, sR - ring_stride3(dir), o, dir, 1, P, qL, bad);
+  const double  Sr = face_state_fast3(sQ, sHS, sS, gR, sR, o, dir, -1, P, qR, bad);
+  const Side64  L = hllc_side64<3>(qL, Sl, P, P.pi64 != 0, bad);
+  const Side64  R = hllc_side64<3>(qR, Sr, P, P.pi64 != 0, bad);
+  hllc_fast64<3>(qL, qR, L, R, dtdx, fl, bad);
+  if (bad)
+  {
+    face_flux_cold3(sQ, sHS, sF, f, dir, dtdx, &P);
+    return true;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k)
+    sF[(k == H::FU ? H::FU + dir : (k >= H::FV && k == H::FU + dir ? H::FU : k)) * NFF + f] = fl[k];
+  return false;
+}
+
+// end of the update of a cell whose values left the range: the reference's
+// renormalisation and CFL rate; writes the cell (variables NC apart)
+__device__ __noinline__ double
+finish_cold3(State64<3> s, double * out, double dx, const PhysParams * P, bool want_dt)
+{
+  using H = V<3>;
+  double *     u2 = s.v;
+  const double inv = 1.0 / (u2[H::IA0] + u2[H::IA1]);
+  u2[H::ID] = u2[H::IAD0] + u2[H::IAD1];
+  u2[H::IA0] *= inv;
+  u2[H::IA1] *= inv;
+  for (int v = 0; v < H::NV; ++v)
+    out[v * 512] = u2[v];
+  if (!want_dt)
+    return 0.0;
+  double       q[7];
+  const double c = prim_fp64<3>(u2, q, *P);
+  return (c + fabs(q[H::QU])) / dx + (c + fabs(q[H::QV])) / dx + (c + fabs(q[H::QW])) / dx;
+}
+
+__device__ __noinline__ double2
+source_cold3(State64<3> s, const PhysParams * P)
+{
+  double2 st;
+  source_factors_fp64<3>(s.v, *P, st.x, st.y);
+  return st;
+}
+
+__device__ __forceinline__ State64<3>
+pack_state3(const double * u)
+{
+  State64<3> s;
+#pragma unroll
+  for (int v = 0; v < V<3>::NV; ++v)
+    s.v[v] = u[v];
+  return s;
+}
+
+static __global__ void __launch_bounds__(Step3D64::NT, 1)
+step3d_fast64_kernel(const __grid_constant__ StepArgs a)
+{
+  using T = Step3D64::T;
+  using H = V<3>;
+  constexpr int B = T::B, NT = Step3D64::NT, G = T::G, GG = T::GG, GGG = T::GGG, S = T::S, SS = T::SS, NC = 512;
+  constexpr int NFF = T::NFF;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *           sQ = reinterpret_cast<double *>(smem_raw);
+  double *           sHS = sQ + Step3D64::OFF_HS;
+  double *           sS = sQ + Step3D64::OFF_S;
+  double *           sF = sQ + Step3D64::OFF_F;
+  __shared__ double  sRed[NT / 32];
+  __shared__ int     sSlot[12]; // the block's reflux slots (faces 0-5), then its defer slots
+  __shared__ int     sNext;     // the CTA's next block
+  const int          tid = threadIdx.x;
+  const PhysParams & P = a.p;
+  const bool         owner = tid < NC;
+  const int          ci = tid % B, cj = (tid / B) % B, ck = tid / (B * B);
+
+  const int nwalk = step_count(a);
+  for (int iw = blockIdx.x; iw < nwalk;)
+  {
+    const int    n = a.work ? a.work[iw] : iw;
+    // the next block is claimed now (the ticket's latency hides behind the gather)
+    const int    next_v = tid == 12 ? claim_next(a, iw, nwalk) : 0;
+    const int    ins = a.m.inst ? a.m.inst[n] : 0;
+    const double dx = P.level_dx[a.m.level[n]];
+    const int    c0[3] = { a.m.coord[n * 3 + 0], a.m.coord[n * 3 + 1], a.m.coord[n * 3 + 2] };
+    int          slot_v = -1; // coarse/fine slots, stored to shared memory after the gather
+    if (a.m.reflux_slot && tid < 12)
+      slot_v = tid < 6 ? a.m.reflux_slot[n * 6 + tid] : a.m.defer_slot[n * 6 + tid - 6];
+    // a value left the fast form's range (per thread until the next barrier,
+    // then for the CTA)
+    double dtdx = a.dt[ins];
+    bool   cold = x64_raw_bad(dtdx) || x64_raw_bad(dx);
+    {
+      const double q = div64(dtdx, dx, cold);
+      dtdx = cold ? dtdx / dx : q;
+    }
+
+    // ---------------- phase 1: own cell + halo -> primitives (the threads
+    // without a cell take the first halo cells)
+    const double * own = a.U + (size_t)n * H::NV * NC + tid;
+    const int      nhalo = HALO3_FULL + (P.thinc != 0 ? HALO3_ALPHA : 0);
+    // the own cell is the walk's first item of the threads that have one
+    for (int it = owner ? -1 : 0, h = owner ? 0 : tid - NC; it < 0 || h < nhalo; ++it)
+    {
+      int    gidx;
+      double u[H::NV];
+      if (it < 0)
+      {
+        gidx = (ci + 2) + G * (cj + 2) + GG * (ck + 2);
+#pragma unroll
+        for (int v = 0; v < H::NV; ++v)
+          u[v] = own[v * NC];
+        h = tid + NT - NC;
+      }
+      else
+      {
+        int g[3];
+        halo_coords_3d(h, g);
+        gidx = (g[0] + 2) + G * (g[1] + 2) + GG * (g[2] + 2);
+        if (h >= HALO3_FULL)
+        {
+          if (!gather_ghost_3d<true>(a, n, c0, g, u))
+          {
+            raise_status(a.status, STATUS_MESH);
+            u[H::IA0] = a.U[((size_t)n * H::NV + H::IA0) * NC + tid % NC];
+          }
+          const bool b = x64_raw_bad(u[H::IA0]);
+          cold = cold || b;
+          sQ[6 * GGG + gidx] = b ? alpha_prim<false>(u[H::IA0]) : clamp_a64(u[H::IA0]);
+          h += NT;
+          continue;
+        }
+        if (!gather_ghost_3d(a, n, c0, g, u))
+        {
+          raise_status(a.status, STATUS_MESH);
+          const double * cell = a.U + (size_t)n * H::NV * NC + tid % NC;
+#pragma unroll
+          for (int v = 0; v < H::NV; ++v)
+            u[v] = cell[v * NC];
+        }
+        h += NT;
+      }
+      double q[7];
+      bool   bad = false;
+      prim_fast64<3, false, true>(u, q, P, bad);
+      if (bad)
+      {
+        cold = true;
+        prim_ref64<3>(pack_state3(u), &P, sQ + gidx, GGG);
+      }
+      else
+      {
+#pragma unroll
+        for (int k = 0; k < 7; ++k)
+          sQ[k * GGG + gidx] = q[k];
+      }
+    }
+    if (tid < 12)
+      sSlot[tid] = slot_v;
+    if (tid == 12)
+      sNext = next_v;
+    cold = __syncthreads_or(cold) != 0;
+    // the next block of this CTA: its own cells and table rows into L2
+    if (tid < 3 && sNext < nwalk)
+    {
+      const int nn = a.work ? a.work[sNext] : sNext;
+      if (tid == 0)
+        prefetch_l2_range(a.U + (size_t)nn * H::NV * NC, (unsigned)(H::NV * NC * sizeof(double)));
+      else if (tid == 1)
+        prefetch_l2_range(a.m.nbr + (size_t)nn * 27 * 8, 27 * 8 * sizeof(int32_t));
+      else
+        prefetch_l2_line(a.m.nbr_rel + (size_t)nn * 27);
+    }
+
+    // ---------------- phase 2: Hancock source of the 896 face-neighbour cells
+    // (the enumeration of step3d_kernel)
+    const bool cold0 = cold;
+    for (int h = tid; h < NC + 6 * B * B; h += NT)
+    {
+      int ri, rj, rk;
+      if (h < NC)
+      {
+        ri = h & 7;
+        rj = (h >> 3) & 7;
+        rk = h >> 6;
+      }
+      else
+      {
+        const int i = h - NC, f = i >> 6, pa = i & 7, pb = (i >> 3) & 7;
+        const int side = (f & 1) ? B : -1;
+        ri = f < 2 ? side : pa;
+        rj = f < 2 ? pa : (f < 4 ? side : pb);
+        rk = f < 4 ? pb : side;
+      }
+      const int r = (ri + 1) + S * (rj + 1) + SS * (rk + 1);
+      const int gi = (ri + 2) + G * (rj + 2) + GG * (rk + 2);
+      bool      bad = cold0;
+      if (!bad)
+        bad = hancock_fast3(sQ, sHS, sS, gi, r, dtdx, P);
+      if (bad)
+      {
+        cold = true;
+        hancock_cold3(sQ, sHS, gi, r, dtdx, &P);
+      }
+    }
+
+    // the owned cell: its running state (read again, an L2 hit), and the
+    // volume-fraction source factors
+    double u2[H::NV], st0 = 1.0, st1 = 1.0;
+    double a0n = 0.0, a1n = 0.0;
+    if (owner)
+    {
+#pragma unroll
+      for (int v = 0; v < H::NV; ++v)
+        u2[v] = __ldcg(own + v * NC);
+      a0n = u2[H::IA0];
+      a1n = u2[H::IA1];
+      if (P.source_term == 1)
+      {
+        bool bad = cold0;
+        if (!bad)
+          source_factors_fast64<3>(u2, P, st0, st1, bad);
+        if (bad)
+        {
+          const double2 st = source_cold3(pack_state3(u2), &P);
+          st0 = st.x;
+          st1 = st.y;
+        }
+      }
+      cold = cold || x64_raw_bad(a1n) || x64_raw_bad(st0) || x64_raw_bad(st1);
+    }
+    cold = __syncthreads_or(cold) != 0;
+
+    // deferred cells (next to a finer face) are finished by reflux3d_kernel
+    const int * dsl = a.m.defer_slot ? sSlot + 6 : nullptr;
+    bool        deferred = false;
+    if (dsl && owner)
+    {
+      const int cc[3] = { ci, cj, ck };
+#pragma unroll
+      for (int f = 0; f < 6; ++f)
+        deferred = deferred || (dsl[f] >= 0 && cc[f >> 1] == ((f & 1) ? B - 1 : 0));
+    }
+
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir)
+    {
+      // ---------------- phase 3: one face per thread
+      bool bad = cold;
+      if (!bad)
+        bad = face_flux_fast3(sQ, sHS, sS, sF, tid, dir, dtdx, P);
+      else
+        face_flux_cold3(sQ, sHS, sF, tid, dir, dtdx, &P);
+      cold = __syncthreads_or(bad) != 0;
+
+      // face index of the owned cell's left/right face in this direction
+      const int ext0 = B + (dir == 0), ext1 = B + (dir == 1);
+      const int il = ci + ext0 * (cj + ext1 * ck);
+      const int ir = il + (dir == 0 ? 1 : (dir == 1 ? ext0 : ext0 * ext1));
+
+      // ---------------- publish coarse/fine records of this direction (AMR only)
+      if (a.m.reflux_slot)
+      {
+        for (int side = 0; side < 2; ++side)
+        {
+          const int rs = sSlot[2 * dir + side];
+          // positions along the face: the two transverse coordinates (first, second)
+          if (rs >= 0 && tid < B * B)
+          {
+            const int t1 = tid % B, t2 = tid / B, edge = side ? B : 0;
+            const int fx = dir == 0 ? edge : t1, fy = dir == 1 ? edge : (dir == 0 ? t1 : t2), fz = dir == 2 ? edge : t2;
+            const int fidx = fx + ext0 * (fy + ext1 * fz);
+            double *  dst = a.reflux_buf + ((size_t)rs * B * B + tid) * 9;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+              dst[k] = sF[k * NFF + fidx];
+          }
+        }
+        // own face fluxes of deferred cells, this direction (left then right)
+        if (deferred)
+        {
+          for (int f = 0; f < 6; ++f)
+          {
+            const int d2 = f >> 1;
+            if (dsl[f] < 0 || (d2 == 0 ? ci : (d2 == 1 ? cj : ck)) != ((f & 1) ? B - 1 : 0))
+              continue;
+            const int t1 = d2 == 0 ? cj : ci, t2 = d2 == 2 ? cj : ck;
+            double *  dst = a.defer_buf + (((size_t)dsl[f] * B * B + t1 + B * t2) * 6 + 2 * dir) * 9;
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+            {
+              dst[k] = sF[k * NFF + il];
+              dst[9 + k] = sF[k * NFF + ir];
+            }
+          }
+        }
+      }
+
+      // ---------------- phase 4: this direction's update of the owned cell
+      // (the reference starts each sum from 0 + F_left: the same value but
+      // for the sign of a zero)
+      if (owner && !deferred)
+      {
+        const double usl = sF[H::FUS * NFF + il], usr = sF[H::FUS * NFF + ir];
+        if (cold)
+        {
+          double acc[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            acc[k] = 0.0 + sF[k * NFF + il];
+          acc[H::FA0] -= st0 * usl * a0n;
+          acc[H::FA1] -= st1 * usl * a1n;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            acc[k] = acc[k] - sF[k * NFF + ir];
+          acc[H::FA0] += st0 * usr * a0n;
+          acc[H::FA1] += st1 * usr * a1n;
+          apply_dir_fp64(u2, acc);
+        }
+        else
+        {
+          const bool mp = P.source_term == 1;
+          bool       b2 = false;
+          double     i0 = alpha_inc64(sF[H::FA0 * NFF + il], sF[H::FA0 * NFF + ir], usl, usr, st0, a0n, mp, b2);
+          double     i1 = alpha_inc64(sF[H::FA1 * NFF + il], sF[H::FA1 * NFF + ir], usl, usr, st1, a1n, mp, b2);
+          if (b2)
+          {
+            i0 = (sF[H::FA0 * NFF + il] - st0 * usl * a0n) - sF[H::FA0 * NFF + ir] + st0 * usr * a0n;
+            i1 = (sF[H::FA1 * NFF + il] - st1 * usl * a1n) - sF[H::FA1 * NFF + ir] + st1 * usr * a1n;
+          }
+          u2[H::IAD0] = clamp_r64(u2[H::IAD0] + (sF[H::FR0 * NFF + il] - sF[H::FR0 * NFF + ir]));
+          u2[H::IAD1] = clamp_r64(u2[H::IAD1] + (sF[H::FR1 * NFF + il] - sF[H::FR1 * NFF + ir]));
+          u2[H::IA0] = clamp_a64(u2[H::IA0] + i0);
+          u2[H::IA1] = clamp_a64(u2[H::IA1] + i1);
+          u2[H::IE] += sF[H::FE * NFF + il] - sF[H::FE * NFF + ir];
+          u2[H::IU] += sF[H::FU * NFF + il] - sF[H::FU * NFF + ir];
+          u2[H::IV] += sF[H::FV * NFF + il] - sF[H::FV * NFF + ir];
+          u2[H::IW] += sF[H::FW * NFF + il] - sF[H::FW * NFF + ir];
+        }
+      }
+      __syncthreads();
+    }
+
+    double m_inv = 0.0;
+    if (owner && !deferred)
+    {
+      double * out = a.U2 + (size_t)n * H::NV * NC + tid;
+      bool     bad = cold;
+      // the state before the renormalisation, for the cold path
+      if (!bad)
+      {
+        const double b0 = u2[H::IA0], b1 = u2[H::IA1];
+        m_inv = finish_fast64<3>(u2, dx, P, a.invdt != nullptr, bad);
+        if (bad)
+        {
+          u2[H::IA0] = b0;
+          u2[H::IA1] = b1;
+        }
+      }
+      if (bad)
+      {
+        m_inv = finish_cold3(pack_state3(u2), out, dx, &P, a.invdt != nullptr);
+#pragma unroll
+        for (int v = 0; v < H::NV; ++v)
+          u2[v] = out[v * NC];
+      }
+      bool finite = true;
+#pragma unroll
+      for (int v = 0; v < H::NV; ++v)
+      {
+        out[v * NC] = u2[v];
+        finite = finite && finite_bits(u2[v]);
+      }
+      if (!finite)
+        raise_status(a.status, STATUS_NONPHYSICAL);
+    }
+    if (a.invdt)
+    {
+      m_inv = warp_max_pos64(m_inv);
+      if ((tid & 31) == 0)
+        sRed[tid >> 5] = m_inv;
+      __syncthreads();
+      if (tid == 0)
+      {
+        double mm = 0.0;
+        for (int w = 0; w < NT / 32; ++w)
+          mm = bits64(sRed[w]) > bits64(mm) ? sRed[w] : mm;
+        atomic_max_pos(a.invdt + ins, mm);
+      }
+    }
+    const int next = sNext; // read before the barrier: the next block's claim overwrites it
+    __syncthreads();
+    iw = next;
+  }
+}
+
+} // namespace g5

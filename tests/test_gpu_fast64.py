@@ -66,6 +66,16 @@ CASES = [
     (2, 16, "nan", "ideal", {}),
     (2, 8, "negative", "ideal", {}),
     (2, 16, "negative", "both", dict(slope_type=2.0)),
+    (3, 8, "smooth", "first", {}),
+    (3, 8, "smooth", "second", dict(thinc=1, slope_type=2.0, source_term=1)),
+    (3, 8, "smooth", "both", dict(integrator=1, slope_type=0.0)),
+    (3, 8, "rest", "ideal", dict(thinc=1)),
+    (3, 8, "pure", "first", {}),
+    (3, 8, "tiny", "ideal", dict(source_term=1)),
+    (3, 8, "subnormal", "first", {}),
+    (3, 8, "huge", "ideal", dict(thinc=1)),
+    (3, 8, "nan", "ideal", {}),
+    (3, 8, "negative", "ideal", dict(slope_type=2.0)),
 ]
 
 
