@@ -46,30 +46,32 @@ fast64_case(const PhysParams & p)
 constexpr int FAST64 = 0, REF64 = 2;
 
 template <int B, int STIFF>
+static int
+occupancy2d(bool thinc)
+{
+  using T = Step2DTraits<B, false>;
+  const size_t smem = T::smem_bytes + (thinc ? T::smem_thinc : 0);
+  cudaFuncSetAttribute(step2d_kernel<B, false, false, STIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(T::smem_bytes + T::smem_thinc));
+  int occ = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, false, false, STIFF>, T::NT, smem);
+  return occ;
+}
+
+template <int B, int STIFF>
 static cudaError_t
 launch_step2d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches)
 {
   using T = Step2DTraits<B, false>;
-  static bool configured = false;
-  static int  occ = 1;
-  if (!configured)
-  {
-    cudaError_t e = cudaFuncSetAttribute(step2d_kernel<B, false, false, STIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
-    if (e != cudaSuccess)
-      return e;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, false, false, STIFF>, T::NT, T::smem_bytes);
-    if (occ < 1)
-      occ = 1;
-    configured = true;
-  }
-  const int per_sm = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
-  int       grid = num_sms() * per_sm;
+  static const int occs[2] = { std::max(1, occupancy2d<B, STIFF>(false)), std::max(1, occupancy2d<B, STIFF>(true)) };
+  const int        occ = occs[a.p.thinc != 0];
+  const int        per_sm = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
+  int              grid = num_sms() * per_sm;
   if (grid > step_count(a))
     grid = step_count(a);
   cudaError_t e = cudaSuccess;
   if (grid >= 1)
   {
-    step2d_kernel<B, false, false, STIFF><<<grid, T::NT, T::smem_bytes, s>>>(a);
+    step2d_kernel<B, false, false, STIFF><<<grid, T::NT, T::smem_bytes + (a.p.thinc != 0 ? T::smem_thinc : 0), s>>>(a);
     ++*launches;
     e = cudaGetLastError();
     if (e != cudaSuccess)
@@ -83,17 +85,6 @@ launch_step2d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launche
     e = cudaGetLastError();
   }
   return e;
-}
-
-template <int B, int STIFF>
-static int
-occupancy2d()
-{
-  using T = Step2DTraits<B, false>;
-  cudaFuncSetAttribute(step2d_kernel<B, false, false, STIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem_bytes);
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, false, false, STIFF>, T::NT, T::smem_bytes);
-  return occ;
 }
 
 // the 3D step: the fast form's kernel, or the reference arithmetic's
@@ -268,9 +259,9 @@ int
 step_max_ctas_per_sm_fp64(int dim, int b)
 {
   if (dim == 2 && b == 16)
-    return std::min(occupancy2d<16, FAST64>(), occupancy2d<16, REF64>());
+    return std::min(occupancy2d<16, FAST64>(true), occupancy2d<16, REF64>(true));
   if (dim == 2 && b == 8)
-    return std::min(occupancy2d<8, FAST64>(), occupancy2d<8, REF64>());
+    return std::min(occupancy2d<8, FAST64>(true), occupancy2d<8, REF64>(true));
   if (dim == 3 && b == 8)
     return std::min(occupancy3d<FAST64>(), occupancy3d<REF64>());
   return 0;

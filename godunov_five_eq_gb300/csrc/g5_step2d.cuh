@@ -38,7 +38,11 @@ struct Step2DTraits
   // the mixture's S of the cell
   static constexpr int NREC = MIXED ? 15 : 16;
   static constexpr int NFF = B * (B + 1);
+  // FP64: THINC face values of the 2 B (B + 2) cells and directions, right and
+  // left, and the list of those that have one
+  static constexpr int NTH = MIXED ? 0 : 2 * B * (B + 2);
   static constexpr size_t smem_bytes = sizeof(R) * (size_t)(NQ * G * G + NREC * S * S + 2 * 8 * NFF) + 64;
+  static constexpr size_t smem_thinc = (2 * sizeof(double) + sizeof(short)) * (size_t)NTH; // (more, with THINC)
 };
 
 // halo cell h (0 .. G*G - B*B - 1) -> ghosted coordinates
@@ -321,13 +325,43 @@ face_flux_cold64(const double * sQ, const double * sRec, double * sF, int dir, i
   face_flux_ref64<B>(sQ, sRec, sF, dir, ff, dtdx, *P);
 }
 
+// FP64: the THINC entry (cell, direction) in the arrays sAF: 2 directions of
+// B (B + 2) cells
+template <int B>
+__device__ __forceinline__ int
+thinc_index(int dir, int ci, int cj)
+{
+  return dir == 0 ? (ci + 1) + (B + 2) * cj : B * (B + 2) + ci + B * (cj + 1);
+}
+
+// the pair's face values, from its entry
+template <int B>
+__device__ __forceinline__ bool
+thinc_eval2(const double * sQ, double * sAF, int i, const PhysParams & P)
+{
+  using T = Step2DTraits<B, false>;
+  constexpr int  G = T::G, GG = G * G;
+  const int      dir = i < B * (B + 2) ? 0 : 1, k = i - dir * B * (B + 2);
+  const int      ci = dir == 0 ? k % (B + 2) - 1 : k % B, cj = dir == 0 ? k / (B + 2) : k / B - 1;
+  const double * A = sQ + 5 * GG + (ci + 2) + G * (cj + 2);
+  // (1, 2, 1)-weighted central differences (youngs_abs_2d)
+  const double gx = (__fma_rn(2.0, A[1], A[1 - G]) + A[1 + G]) - (__fma_rn(2.0, A[-1], A[-1 - G]) + A[-1 + G]);
+  const double gy = (__fma_rn(2.0, A[G], A[G - 1]) + A[G + 1]) - (__fma_rn(2.0, A[-G], A[-G - 1]) + A[-G + 1]);
+  bool         bad = false;
+  const double nd = youngs_ratio64(dir == 0 ? gx : gy, gx * gx + gy * gy, bad);
+  const int    o = dir == 0 ? 1 : G;
+  thinc_pair64(A[0], A[-o], A[o], nd, P, sAF[i], sAF[T::NTH + i], bad);
+  return bad;
+}
+
 // FP64: the reconstructed state and the mixture's S of one side (the values
 // of face_state_ref64, normal velocity first).  The direction is a run-time
 // value: X and Y faces share one copy of the flux code, which is long enough
 // to miss the instruction cache.
 template <int B>
 __device__ __forceinline__ double
-face_state_fast64(const double * sQ, const double * sRec, int ci, int cj, int dir, int side, const PhysParams & P, double * q, bool & bad)
+face_state_fast64(const double * sQ, const double * sRec, const double * sAF, int ci, int cj, int dir, int side, const PhysParams & P, double * q,
+                  bool & bad)
 {
   using T = Step2DTraits<B, false>;
   constexpr int    G = T::G, S = T::S, GG = G * G, SS = S * S;
@@ -348,27 +382,15 @@ face_state_fast64(const double * sQ, const double * sRec, int ci, int cj, int di
   q[5] = a0;
   if (P.thinc)
   {
-    const int      o = dir == 0 ? 1 : G;
-    const double * A = sQ + 5 * GG;
-    const double   aP = A[gi + o], aM = A[gi - o];
-    const bool     mono = (bits64(aP) > bits64(a0) && bits64(a0) > bits64(aM)) || (bits64(aP) < bits64(a0) && bits64(a0) < bits64(aM));
-    if (mono && bits64(a0) > bits64(P.thinc_eps) && bits64(a0) < bits64(1.0 - P.thinc_eps))
+    const double af = sAF[(side > 0 ? 0 : T::NTH) + thinc_index<B>(dir, ci, cj)];
+    if (bits64(af) != bits64(thinc_none64()))
     {
-      double nxa, nya;
-      youngs_abs_2d<double, G>(A, gi, nxa, nya);
-      const double af = thinc_alpha64(a0, aM, aP, dir == 0 ? nxa : nya, side > 0 ? 1.0 : -1.0, P.thinc_beta);
-      const double r0 = sQ[gi], r1 = sQ[GG + gi];
-      double       q0 = r0 + r0 / a0 * (af - a0);
-      double       q1 = r1 + r1 / (1.0 - a0) * (a0 - af);
-      if (hancock)
-      {
-        q0 = __fma_rn(0.5, sRec[10 * SS + si], q0);
-        q1 = __fma_rn(0.5, sRec[11 * SS + si], q1);
-      }
-      q[0] = q0;
-      q[1] = q1;
+      const ThincSide64 t = thinc_side64(a0, af, sQ[gi], sQ[GG + gi], hancock ? sRec[10 * SS + si] : 0.0, hancock ? sRec[11 * SS + si] : 0.0, &P);
+      q[0] = t.q0;
+      q[1] = t.q1;
       q[5] = af;
-      Sm = mix_S64(P, af, 1.0 - af, bad);
+      Sm = t.S;
+      bad = bad || t.bad;
     }
   }
   else
@@ -381,7 +403,7 @@ face_state_fast64(const double * sQ, const double * sRec, int ci, int cj, int di
 
 template <int B>
 __device__ __forceinline__ bool
-face_flux_fast64(const double * sQ, const double * sRec, double * sF, int dir, int ff, double dtdx, const PhysParams & P)
+face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, double * sF, int dir, int ff, double dtdx, const PhysParams & P)
 {
   using H = V<2>;
   constexpr int NFF = B * (B + 1);
@@ -389,8 +411,8 @@ face_flux_fast64(const double * sQ, const double * sRec, double * sF, int dir, i
   face_cells<B>(dir, ff, li, lj, ri, rj);
   double       qL[6], qR[6], fl[8];
   bool         bad = false;
-  const double Sl = face_state_fast64<B>(sQ, sRec, li, lj, dir, 1, P, qL, bad);
-  const double Sr = face_state_fast64<B>(sQ, sRec, ri, rj, dir, -1, P, qR, bad);
+  const double Sl = face_state_fast64<B>(sQ, sRec, sAF, li, lj, dir, 1, P, qL, bad);
+  const double Sr = face_state_fast64<B>(sQ, sRec, sAF, ri, rj, dir, -1, P, qR, bad);
   const Side64 L = hllc_side64<2>(qL, Sl, P, P.pi64 != 0, bad);
   const Side64 R = hllc_side64<2>(qR, Sr, P, P.pi64 != 0, bad);
   hllc_fast64<2>(qL, qR, L, R, dtdx, fl, bad);
@@ -919,6 +941,9 @@ step2d_kernel(const __grid_constant__ StepArgs a)
   R *          sRec = sQ + T::NQ * GG;
   R *          sFx = sRec + T::NREC * SS; // [8][NFF]  X faces (B+1) x B
   R *          sFy = sFx + 8 * NFF;       // [8][NFF]  Y faces B x (B+1)
+  R *          sAF = sFy + 8 * NFF;       // FP64: THINC face values, then the list
+  short *      sList = reinterpret_cast<short *>(sAF + 2 * T::NTH);
+  __shared__ int sThinc; // FP64: entries of the list
   using DtT = typename std::conditional<MIXED, float, double>::type;
   __shared__ DtT sRed[NT / 32];
   __shared__ int sSlot[10]; // the block's reflux slots (faces 0-3), its defer slots, its outside-twin range
@@ -941,6 +966,9 @@ step2d_kernel(const __grid_constant__ StepArgs a)
   // thread's device-scope fence and atomic; acquire: that thread's fence
   // after the atomic, then the barrier.
   constexpr bool fused = MIXED && FUSED;
+  constexpr bool fast64 = !MIXED && STIFF != 2;
+  if (fast64 && tid == 0)
+    sThinc = 0;
   for (int iw = blockIdx.x;;)
   {
     int next = iw;
@@ -971,8 +999,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       // FP64 fast form: a value of the block left its range (per thread until
       // the next barrier, then for the whole CTA: the phases that follow take
       // the reference arithmetic)
-      constexpr bool fast64 = !MIXED && STIFF != 2;
-      bool           cold = false;
+      bool cold = false;
       if constexpr (fast64)
       {
         cold = x64_raw_bad(dtdx_r) || x64_raw_bad(dx);
@@ -1115,7 +1142,27 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         }
       }
       if constexpr (fast64)
+      {
+        // the interface cells of the THINC reconstruction
+        for (int i = tid; P.thinc != 0 && i < T::NTH; i += NT)
+        {
+          const int      dir = i < B * (B + 2) ? 0 : 1, k = i - dir * B * (B + 2);
+          const int      gi = dir == 0 ? (k % (B + 2) + 1) + G * (k / (B + 2) + 2) : (k % B + 2) + G * (k / B + 1);
+          const double * A = sQ + 5 * GG + gi;
+          const int      o = dir == 0 ? 1 : G;
+          if (thinc_cell64(A[0], A[-o], A[o], P))
+            sList[atomicAdd(&sThinc, 1)] = (short)i;
+          else
+            sAF[i] = sAF[T::NTH + i] = thinc_none64();
+        }
         cold = __syncthreads_or(cold) != 0;
+        if (P.thinc != 0 && sThinc > 0 && !cold)
+        {
+          for (int i = tid; i < sThinc; i += NT)
+            cold |= thinc_eval2<B>(sQ, sAF, sList[i], P);
+          cold = __syncthreads_or(cold) != 0;
+        }
+      }
       else
         __syncthreads();
       const bool cold1 = cold;
@@ -1140,7 +1187,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
           else if (cold1)
             face_flux_cold64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, &P);
           else
-            cold |= face_flux_fast64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
+            cold |= face_flux_fast64<B>(sQ, sRec, sAF, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
         }
       }
       // the own cell's state for the update: the FP32-bulk form without the
@@ -1169,6 +1216,9 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         cold = __syncthreads_or(cold) != 0;
       else
         __syncthreads();
+
+      if (fast64 && tid == 0)
+        sThinc = 0; // (read before the barrier above, used again after the next)
 
       // ---------------- publish coarse/fine records (AMR only)
       if (a.m.reflux_slot)

@@ -22,9 +22,12 @@ struct Step3D64
   using T = Step3DTraits<false>;
   static constexpr int NT = 576;
   static constexpr int NTHINC = 640; // cells with a face of one direction
-  // sQ, sHS, the mixture's S of the ring, the face fluxes of one direction
+  // sQ, sHS, the mixture's S of the ring, the face fluxes of one direction,
+  // the direction's THINC face values (right, left) and the list of those
+  // that have one
   static constexpr int OFF_HS = T::NQ * T::GGG, OFF_S = OFF_HS + T::NHS * T::SSS, OFF_F = OFF_S + T::SSS;
-  static constexpr size_t smem_bytes = sizeof(double) * (size_t)(OFF_F + T::NF * T::NFF) + 64;
+  static constexpr int OFF_AF = OFF_F + T::NF * T::NFF;
+  static constexpr size_t smem_bytes = sizeof(double) * (size_t)(OFF_AF + 2 * NTHINC) + 2 * NTHINC + 64;
   static_assert(NT == T::NFF, "one round of faces per direction");
 };
 
@@ -104,14 +107,14 @@ hancock_cold3(const double * sQ, double * sHS, int gi, int r, double dtdx, const
 }
 
 // the reconstructed state of one face side (face_state3<false>, the normal
-// velocity first) and the mixture's S; gi, si: the cell in the ghosted and
-// ring arrays, o the direction's stride, side +1 the cell's right face
+// velocity first) and the mixture's S; gi, si, ti: the cell in the ghosted,
+// ring and THINC arrays, o the direction's stride, side +1 the cell's right face
 __device__ __forceinline__ double
-face_state_fast3(const double * sQ, const double * sHS, const double * sS, int gi, int si, int o, int dir, int side, const PhysParams & P, double * q,
-                 bool & bad)
+face_state_fast3(const double * sQ, const double * sHS, const double * sS, const double * sAF, int gi, int si, int ti, int o, int dir, int side,
+                 const PhysParams & P, double * q, bool & bad)
 {
   using T = Step3D64::T;
-  constexpr int G = T::G, GG = T::GG, GGG = T::GGG, SSS = T::SSS;
+  constexpr int GGG = T::GGG, SSS = T::SSS;
   const double  off = side > 0 ? 0.5 : -0.5;
   const int     st = P.st64;
   const bool    hancock = P.integrator == 0;
@@ -130,23 +133,15 @@ face_state_fast3(const double * sQ, const double * sHS, const double * sS, int g
   q[6] = a0;
   if (P.thinc)
   {
-    const double * A = sQ + 6 * GGG;
-    const double   aP = A[gi + o], aM = A[gi - o];
-    const bool     mono = (bits64(aP) > bits64(a0) && bits64(a0) > bits64(aM)) || (bits64(aP) < bits64(a0) && bits64(a0) < bits64(aM));
-    if (mono && bits64(a0) > bits64(P.thinc_eps) && bits64(a0) < bits64(1.0 - P.thinc_eps))
+    const double af = sAF[side > 0 ? ti : Step3D64::NTHINC + ti];
+    if (bits64(af) != bits64(thinc_none64()))
     {
-      const double nd = youngs_abs_3d<double, G, GG>(A, gi, dir);
-      const double af = thinc_alpha64(a0, aM, aP, nd, side > 0 ? 1.0 : -1.0, P.thinc_beta);
-      const double r0 = sQ[gi], r1 = sQ[GGG + gi];
-      q[0] = r0 + r0 / a0 * (af - a0);
-      q[1] = r1 + r1 / (1.0 - a0) * (a0 - af);
-      if (hancock)
-      {
-        q[0] = __fma_rn(0.5, sHS[si], q[0]);
-        q[1] = __fma_rn(0.5, sHS[SSS + si], q[1]);
-      }
+      const ThincSide64 t = thinc_side64(a0, af, sQ[gi], sQ[GGG + gi], hancock ? sHS[si] : 0.0, hancock ? sHS[SSS + si] : 0.0, &P);
+      q[0] = t.q0;
+      q[1] = t.q1;
       q[6] = af;
-      S = mix_S64(P, af, 1.0 - af, bad);
+      S = t.S;
+      bad = bad || t.bad;
     }
   }
   else
@@ -168,9 +163,70 @@ face_flux_cold3(const double * sQ, const double * sHS, double * sF, int f, int d
     face_flux3<false, 2, -1>(sQ, sHS, f, sF, dtdx, *P);
 }
 
+// the THINC entry of the cell (x, y, z) of direction dir: 10 cells along it,
+// 8 x 8 across
+__device__ __forceinline__ int
+thinc_index3(int dir, int x, int y, int z)
+{
+  return dir == 0 ? (x + 1) + 10 * (y + 8 * z) : (dir == 1 ? x + 8 * ((y + 1) + 10 * z) : x + 8 * (y + 8 * (z + 1)));
+}
+
+// the entry's cell in the ghosted arrays
+__device__ __forceinline__ int
+thinc_ghost3(int dir, int i)
+{
+  using T = Step3D64::T;
+  const int ex = dir == 0 ? 10 : 8, ey = dir == 1 ? 10 : 8;
+  const int x = i % ex - (dir == 0), y = (i / ex) % ey - (dir == 1), z = i / (ex * ey) - (dir == 2);
+  return (x + 2) + T::G * (y + 2) + T::GG * (z + 2);
+}
+
+// lists the cells of direction dir that take the THINC profile, marks the others
+__device__ __forceinline__ void
+thinc_list3(const double * sQ, double * sAF, short * sList, int * count, int dir, const PhysParams & P)
+{
+  const int o = ghost_stride3(dir);
+  for (int i = threadIdx.x; i < Step3D64::NTHINC; i += Step3D64::NT)
+  {
+    const double * A = sQ + 6 * Step3D64::T::GGG + thinc_ghost3(dir, i);
+    if (thinc_cell64(A[0], A[-o], A[o], P))
+      sList[atomicAdd(count, 1)] = (short)i;
+    else
+      sAF[i] = sAF[Step3D64::NTHINC + i] = thinc_none64();
+  }
+}
+
+// an entry's face values on both sides
+__device__ __forceinline__ bool
+thinc_eval3(const double * sQ, double * sAF, int dir, int i, const PhysParams & P)
+{
+  using T = Step3D64::T;
+  constexpr int  G = T::G, GG = T::GG;
+  const double * A = sQ + 6 * T::GGG + thinc_ghost3(dir, i);
+  // (1, 2, 1) x (1, 2, 1)-weighted central differences (youngs_abs_3d; the
+  // weights are powers of two, so each fused term rounds as the two-step one)
+  double g[3] = { 0.0, 0.0, 0.0 };
+#pragma unroll 1
+  for (int c = -1; c <= 1; ++c)
+#pragma unroll 1
+    for (int b = -1; b <= 1; ++b)
+    {
+      const double w = (b == 0 ? 2.0 : 1.0) * (c == 0 ? 2.0 : 1.0);
+      g[0] = __fma_rn(w, A[1 + G * b + GG * c] - A[-1 + G * b + GG * c], g[0]);
+      g[1] = __fma_rn(w, A[b + G + GG * c] - A[b - G + GG * c], g[1]);
+      g[2] = __fma_rn(w, A[b + G * c + GG] - A[b + G * c - GG], g[2]);
+    }
+  bool         bad = false;
+  const double n2 = (g[0] * g[0] + g[1] * g[1]) + g[2] * g[2];
+  const double nd = youngs_ratio64(dir == 0 ? g[0] : (dir == 1 ? g[1] : g[2]), n2, bad);
+  const int    o = ghost_stride3(dir);
+  thinc_pair64(A[0], A[-o], A[o], nd, P, sAF[i], sAF[Step3D64::NTHINC + i], bad);
+  return bad;
+}
+
 // HLLC flux of face f of direction dir, scaled by dt/dx (face_flux3<false>)
 __device__ __forceinline__ bool
-face_flux_fast3(const double * sQ, const double * sHS, const double * sS, double * sF, int f, int dir, double dtdx, const PhysParams & P)
+face_flux_fast3(const double * sQ, const double * sHS, const double * sS, const double * sAF, double * sF, int f, int dir, double dtdx, const PhysParams & P)
 {
   using T = Step3D64::T;
   using H = V<3>;
@@ -181,8 +237,8 @@ face_flux_fast3(const double * sQ, const double * sHS, const double * sS, double
   const int     o = ghost_stride3(dir);
   double        qL[7], qR[7], fl[9];
   bool          bad = false;
-  const double  Sl = face_state_fast3(sQ, sHS, sS, gR - o, sR - ring_stride3(dir), o, dir, 1, P, qL, bad);
-  const double  Sr = face_state_fast3(sQ, sHS, sS, gR, sR, o, dir, -1, P, qR, bad);
+  const double  Sl = face_state_fast3(sQ, sHS, sS, sAF, gR - o, sR - ring_stride3(dir), thinc_index3(dir, fi - (dir == 0), fj - (dir == 1), fk - (dir == 2)), o, dir, 1, P, qL, bad);
+  const double  Sr = face_state_fast3(sQ, sHS, sS, sAF, gR, sR, thinc_index3(dir, fi, fj, fk), o, dir, -1, P, qR, bad);
   const Side64  L = hllc_side64<3>(qL, Sl, P, P.pi64 != 0, bad);
   const Side64  R = hllc_side64<3>(qR, Sr, P, P.pi64 != 0, bad);
   hllc_fast64<3>(qL, qR, L, R, dtdx, fl, bad);
@@ -247,6 +303,9 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
   double *           sHS = sQ + Step3D64::OFF_HS;
   double *           sS = sQ + Step3D64::OFF_S;
   double *           sF = sQ + Step3D64::OFF_F;
+  double *           sAF = sQ + Step3D64::OFF_AF;
+  short *            sList = reinterpret_cast<short *>(sAF + 2 * Step3D64::NTHINC);
+  __shared__ int     sThinc[2]; // entries of the list of the current and the next direction
   __shared__ double  sRed[NT / 32];
   __shared__ int     sSlot[12]; // the block's reflux slots (faces 0-5), then its defer slots
   __shared__ int     sNext;     // the CTA's next block
@@ -256,6 +315,8 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
   const int          ci = tid % B, cj = (tid / B) % B, ck = tid / (B * B);
 
   const int nwalk = step_count(a);
+  if (tid < 2)
+    sThinc[tid] = 0;
   for (int iw = blockIdx.x; iw < nwalk;)
   {
     const int    n = a.work ? a.work[iw] : iw;
@@ -410,6 +471,8 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
       }
       cold = cold || x64_raw_bad(a1n) || x64_raw_bad(st0) || x64_raw_bad(st1);
     }
+    if (P.thinc != 0)
+      thinc_list3(sQ, sAF, sList, &sThinc[0], 0, P);
     cold = __syncthreads_or(cold) != 0;
 
     // deferred cells (next to a finer face) are finished by reflux3d_kernel
@@ -426,13 +489,24 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
 #pragma unroll 1
     for (int dir = 0; dir < 3; ++dir)
     {
-      // ---------------- phase 3: one face per thread
+      // ---------------- phase 3: one face per thread, after the direction's
+      // THINC values (listed before the last barrier)
+      if (P.thinc != 0 && sThinc[dir & 1] > 0 && !cold)
+      {
+        for (int i = tid; i < sThinc[dir & 1]; i += NT)
+          cold |= thinc_eval3(sQ, sAF, dir, sList[i], P);
+        cold = __syncthreads_or(cold) != 0;
+      }
       bool bad = cold;
       if (!bad)
-        bad = face_flux_fast3(sQ, sHS, sS, sF, tid, dir, dtdx, P);
+        bad = face_flux_fast3(sQ, sHS, sS, sAF, sF, tid, dir, dtdx, P);
       else
         face_flux_cold3(sQ, sHS, sF, tid, dir, dtdx, &P);
       cold = __syncthreads_or(bad) != 0;
+      if (tid == 0)
+        sThinc[dir & 1] = 0;
+      if (P.thinc != 0 && dir < 2)
+        thinc_list3(sQ, sAF, sList, &sThinc[(dir + 1) & 1], dir + 1, P);
 
       // face index of the owned cell's left/right face in this direction
       const int ext0 = B + (dir == 0), ext1 = B + (dir == 1);
