@@ -103,13 +103,14 @@ struct DeferInfo
   static constexpr int STRIDE = DIM == 2 ? 16 : 36;
 };
 
-// fields of one output file (pack_fields_kernel): code[k] < NV a variable of
+// fields of one output file (fields_kernel): code[k] < NV a variable of
 // U (the reference's VarId numbering), FIELD_DERIVED + q derived quantity q
 constexpr int FIELD_DERIVED = 64, MAX_PACK_FIELDS = 16;
 struct FieldList
 {
   int code[MAX_PACK_FIELDS];
   int n;
+  int need; // bit q: derived quantity q is asked for
 };
 
 struct StepArgs

@@ -300,7 +300,10 @@ inv_dt_t(const double * U, const DevMesh & m, const PhysParams & p, double * inv
   int grid = num_sms() * 8;
   if (grid > m.n_owned)
     grid = m.n_owned;
-  inv_dt_kernel<DIM, B><<<grid, 256, 0, s>>>(U, m, p, invdt);
+  if (fast64_case(p))
+    inv_dt_kernel<DIM, B, true><<<grid, 256, 0, s>>>(U, m, p, invdt);
+  else
+    inv_dt_kernel<DIM, B, false><<<grid, 256, 0, s>>>(U, m, p, invdt);
   return cudaGetLastError();
 }
 
@@ -325,7 +328,10 @@ rk2_t(const double * U, double * U2, const DevMesh & m, const PhysParams & p, do
   int grid = num_sms() * 8;
   if (grid > m.n_owned)
     grid = m.n_owned;
-  rk2_combine_kernel<DIM, B, false><<<grid, 256, 0, s>>>(U, U2, m, p, invdt);
+  if (fast64_case(p))
+    rk2_combine_kernel<DIM, B, false, true><<<grid, 256, 0, s>>>(U, U2, m, p, invdt);
+  else
+    rk2_combine_kernel<DIM, B, false, false><<<grid, 256, 0, s>>>(U, U2, m, p, invdt);
   return cudaGetLastError();
 }
 
@@ -360,7 +366,12 @@ flags_t(const double * U, const DevMesh & m, int ind, double er, double ec, doub
   int grid = num_sms() * 8;
   if (grid > m.n_owned)
     grid = m.n_owned;
-  refine_flags_kernel<DIM, B><<<grid, 256, 0, s>>>(U, m, ind, er, ec, el, lmin, lmax, flags);
+  constexpr int NC = DIM == 2 ? B * B : B * B * B;
+  // (negative thresholds keep the general kernel)
+  if (ind == 0 && er >= 0.0 && ec >= 0.0)
+    gradient_flags_kernel<DIM, B><<<std::min(m.n_owned, num_sms() * (2048 / NC)), NC, 0, s>>>(U, m, er, ec, lmin, lmax, flags);
+  else
+    refine_flags_kernel<DIM, B><<<grid, 256, 0, s>>>(U, m, ind, er, ec, el, lmin, lmax, flags);
   return cudaGetLastError();
 }
 
@@ -416,46 +427,45 @@ launch_defer_info(int dim, const DevMesh & m, const int32_t * codes, int n, int3
 
 template <int DIM, int B>
 static cudaError_t
-derived_t(const double * U, double * out, int quantity, long long oct_begin, long long num_octs, const PhysParams & p, cudaStream_t s)
+fields_t(const double * U, double * out, const FieldList & fl, long long stride, long long oct_begin, long long num_octs, const PhysParams & p,
+         cudaStream_t s)
 {
   constexpr int   NC = DIM == 2 ? B * B : B * B * B;
   const long long total = num_octs * NC;
   if (total <= 0)
     return cudaSuccess;
-  long long grid = (total + 255) / 256;
-  if (grid > (long long)num_sms() * 16)
-    grid = (long long)num_sms() * 16;
-  derived_kernel<DIM, B><<<(unsigned)grid, 256, 0, s>>>(U, out, quantity, oct_begin, num_octs, p);
+  const unsigned grid = (unsigned)std::min<long long>((total + 255) / 256, (long long)num_sms() * 16);
+  if (fast64_case(p))
+    fields_kernel<DIM, B, true><<<grid, 256, 0, s>>>(U, out, fl, stride, oct_begin, num_octs, p);
+  else
+    fields_kernel<DIM, B, false><<<grid, 256, 0, s>>>(U, out, fl, stride, oct_begin, num_octs, p);
   return cudaGetLastError();
+}
+
+static cudaError_t
+launch_fields(int dim, int b, const double * U, double * out, const FieldList & fl, long long stride, long long oct_begin, long long num_octs,
+              const PhysParams & p, cudaStream_t s)
+{
+  if (dim == 2 && b == 16)
+    return fields_t<2, 16>(U, out, fl, stride, oct_begin, num_octs, p, s);
+  if (dim == 2 && b == 8)
+    return fields_t<2, 8>(U, out, fl, stride, oct_begin, num_octs, p, s);
+  if (dim == 3 && b == 8)
+    return fields_t<3, 8>(U, out, fl, stride, oct_begin, num_octs, p, s);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t
 launch_derived(int dim, int b, const double * U, double * out, int quantity, long long oct_begin, long long num_octs, const PhysParams & p,
                cudaStream_t s)
 {
-  if (dim == 2 && b == 16)
-    return derived_t<2, 16>(U, out, quantity, oct_begin, num_octs, p, s);
-  if (dim == 2 && b == 8)
-    return derived_t<2, 8>(U, out, quantity, oct_begin, num_octs, p, s);
-  if (dim == 3 && b == 8)
-    return derived_t<3, 8>(U, out, quantity, oct_begin, num_octs, p, s);
-  return cudaErrorInvalidValue;
-}
-
-template <int DIM, int B>
-static cudaError_t
-pack_fields_t(const double * U, double * out, const FieldList & fl, long long oct_begin, long long num_octs, const PhysParams & p,
-              cudaStream_t s)
-{
-  constexpr int   NC = DIM == 2 ? B * B : B * B * B;
-  const long long total = num_octs * NC;
-  if (total <= 0)
-    return cudaSuccess;
-  long long grid = (total + 255) / 256;
-  if (grid > (long long)num_sms() * 16)
-    grid = (long long)num_sms() * 16;
-  pack_fields_kernel<DIM, B><<<(unsigned)grid, 256, 0, s>>>(U, out, fl, oct_begin, num_octs, p);
-  return cudaGetLastError();
+  // (the quantity's array covers all blocks, out[oct][cell])
+  const int nc = dim == 2 ? b * b : b * b * b;
+  FieldList fl = {};
+  fl.n = 1;
+  fl.code[0] = FIELD_DERIVED + quantity;
+  fl.need = (1 << quantity) & ~1;
+  return launch_fields(dim, b, U, out + oct_begin * nc, fl, 0, oct_begin, num_octs, p, s);
 }
 
 cudaError_t
@@ -464,17 +474,15 @@ launch_pack_fields(int dim, int b, const double * U, double * out, const int * c
 {
   if (n < 1 || n > MAX_PACK_FIELDS)
     return cudaErrorInvalidValue;
-  FieldList fl;
+  FieldList fl = {};
   fl.n = n;
-  for (int k = 0; k < MAX_PACK_FIELDS; ++k)
-    fl.code[k] = k < n ? codes[k] : 0;
-  if (dim == 2 && b == 16)
-    return pack_fields_t<2, 16>(U, out, fl, oct_begin, num_octs, p, s);
-  if (dim == 2 && b == 8)
-    return pack_fields_t<2, 8>(U, out, fl, oct_begin, num_octs, p, s);
-  if (dim == 3 && b == 8)
-    return pack_fields_t<3, 8>(U, out, fl, oct_begin, num_octs, p, s);
-  return cudaErrorInvalidValue;
+  for (int k = 0; k < n; ++k)
+  {
+    fl.code[k] = codes[k];
+    if (codes[k] > FIELD_DERIVED)
+      fl.need |= 1 << (codes[k] - FIELD_DERIVED);
+  }
+  return launch_fields(dim, b, U, out, fl, num_octs * (dim == 2 ? b * b : b * b * b), oct_begin, num_octs, p, s);
 }
 
 } // namespace g5

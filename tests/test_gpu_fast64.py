@@ -102,3 +102,50 @@ def test_fast64_step_matches_oracle(dim, b, kind, gas, kw):
         assert impl.status() != 0
     else:
         assert np.array_equal(inv.cpu().numpy(), inv_ref)
+
+
+@pytest.mark.parametrize("dim,b", [(2, 16), (2, 8), (3, 8)])
+@pytest.mark.parametrize("er,ec", [(0.1, 0.0125), (0.0, 0.0), (0.5, 0.5), (1.0, 1.0), (2.0, 1e-60), (0.25, 0.9)])
+def test_gradient_flags_match_oracle(dim, b, er, ec):
+    """Indicators exactly on a threshold, of tiny, huge, zero and NaN densities."""
+    mesh, t = amr_mesh(dim=dim, b=b, nref=3, lmin=1, lmax=2, seed=7)
+    p = water_air_params(t, dim=dim, b=b)
+    I = configs.ids(dim)
+    rng = np.random.default_rng(11)
+    n = t.n_owned
+    U = smooth_state(mesh, t, p)
+    for k, v in enumerate((I["IAD0"], I["IAD1"])):
+        base = rng.choice([1.0, 0.001, 1000.0, 1e-4, 1e60], size=(n, 1))
+        step = rng.choice([0.0, 1e-6, er, ec, 0.3, 3.0], size=(n, 1)) * rng.integers(0, 2, (n, t.ncell))
+        U[:n, v] = base * (1.0 - np.minimum(step, 0.999999) * (k + 1) / 2)
+    U[0, I["IAD0"], :3] = (np.nan, 0.0, -0.5)
+    U[1, I["IAD1"], 5] = np.inf
+    o = Oracle(t, p)
+    o.fill_outside(U)
+    for lmin, lmax in ((0, 3), (1, 2), (2, 2)):
+        with np.errstate(all="ignore"):
+            ref = o.refine_flags(U, 0, er, ec, 0.02, lmin, lmax)
+        got = GodunovImplemGB300(p, t).refine_flags(torch.from_numpy(U).cuda(), 0, er, ec, 0.02, lmin, lmax)
+        assert np.array_equal(got.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("dim,b,kind,gas", [(2, 16, "pure", "first"), (2, 8, "subnormal", "both"), (2, 16, "rest", "ideal"), (3, 8, "tiny", "second"), (3, 8, "negative", "ideal")])
+def test_fields_match_single_quantities_and_oracle(dim, b, kind, gas):
+    from oracle.oracle import derived
+
+    t, p, U = build(dim, b, kind, gas)
+    U[0, 0, :4] *= 1.0 + 2e-16 * np.arange(4)  # ID apart from the partial densities
+    impl = GodunovImplemGB300(p, t)
+    d_U = torch.from_numpy(U).cuda()
+    codes = [64 + q for q in range(8)] + [1, 0]
+    got = impl.pack_fields(d_U, codes).cpu().numpy()
+    for q in range(8):
+        with np.errstate(all="ignore"):
+            ref = np.asarray(derived(p, U, q)).reshape(U.shape[0], -1)[: t.n_owned]
+        assert np.array_equal(got[q], ref, equal_nan=True), q
+        one = impl.derived_quantity(d_U, q).cpu().numpy()[: t.n_owned, 0]
+        assert np.array_equal(one, ref, equal_nan=True), q
+    assert np.array_equal(got[8], U[: t.n_owned, 1]) and np.array_equal(got[9], U[: t.n_owned, 0])
+    with np.errstate(all="ignore"):
+        inv = Oracle(t, p).inv_dt(U)
+    assert np.array_equal(impl.compute_inv_dt(d_U).cpu().numpy(), inv)
