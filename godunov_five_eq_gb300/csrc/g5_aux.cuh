@@ -390,6 +390,15 @@ refine_flags_kernel(const double * U,
   }
 }
 
+// a pair's indicator against both thresholds: bit 0 above eps_r, bit 1 below
+// eps_c (a call, so that no compare of it runs on the FP64 pipe otherwise)
+static __device__ __noinline__ int
+gradient_exact(double C, double N, double eps_r, double eps_c)
+{
+  const double ind = normalized_gradient(C, N);
+  return (ind > eps_r ? 1 : 0) | (ind < eps_c ? 2 : 0);
+}
+
 // The SIMPLE_GRADIENT indicator (normalized_gradient of every face pair of
 // both partial densities) without its divisions.  A block's flag needs only
 // whether its largest indicator exceeds eps_r and whether it is below eps_c,
@@ -401,7 +410,7 @@ refine_flags_kernel(const double * U,
 // was bound by the FP64 pipe (24 divisions per cell: 732 us for 2.0M cells).
 template <int DIM, int B>
 __global__ void __launch_bounds__(DIM == 2 ? B * B : B * B * B)
-gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, double eps_c, int lmin, int lmax, int8_t * flags)
+gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, double eps_c, float rf, float cf, int lmin, int lmax, int8_t * flags)
 {
   using H = V<DIM>;
   constexpr int NC = (DIM == 2) ? B * B : B * B * B, NF = 2 * DIM, FC = NC / B;
@@ -427,9 +436,9 @@ gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, do
       sH[1][h] = neighbor_same_level<DIM, B>(U, m, n, hc, dir, (f & 1) ? 1 : -1, H::IAD1);
     }
     __syncthreads();
-    const bool want_r = lev < lmax && eps_r < 1.0, want_c = lev > lmin && eps_c <= 1.0;
-    const bool  c_pos = bits64(eps_c) > 0;
-    const float rf = (float)eps_r, cf = (float)eps_c;
+    // (rf, cf: the thresholds as floats; at 1 and more they decide without the cells)
+    const bool want_r = lev < lmax && bits64(eps_r) < bits64(1.0), want_c = lev > lmin && bits64(eps_c) <= bits64(1.0);
+    const bool c_pos = bits64(eps_c) > 0;
     bool       above = false, below = true; // some indicator > eps_r; all < eps_c
     if (want_r || want_c)
     {
@@ -449,9 +458,9 @@ gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, do
         undecided = undecided || (!small && ((want_r && fabsf(r - tr) <= 1e-5f * fabsf(tr)) || (want_c && fabsf(r - tc) <= 1e-5f * fabsf(tc))));
         if (undecided)
         {
-          const double ind = normalized_gradient(C, N);
-          gt = want_r && ind > eps_r;
-          lt = !want_c || ind < eps_c;
+          const int x = gradient_exact(C, N, eps_r, eps_c);
+          gt = want_r && (x & 1);
+          lt = !want_c || (x & 2);
         }
         above = above || gt;
         below = below && lt;
@@ -471,7 +480,6 @@ gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, do
         }
       }
     }
-    // (thresholds of 1 and more: the indicator is at most 1)
     const int any_above = __syncthreads_or(above), any_not = __syncthreads_or(!below);
     if (tid == 0)
     {

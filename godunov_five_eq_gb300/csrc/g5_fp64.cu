@@ -369,7 +369,7 @@ flags_t(const double * U, const DevMesh & m, int ind, double er, double ec, doub
   constexpr int NC = DIM == 2 ? B * B : B * B * B;
   // (negative thresholds keep the general kernel)
   if (ind == 0 && er >= 0.0 && ec >= 0.0)
-    gradient_flags_kernel<DIM, B><<<std::min(m.n_owned, num_sms() * (2048 / NC)), NC, 0, s>>>(U, m, er, ec, lmin, lmax, flags);
+    gradient_flags_kernel<DIM, B><<<std::min(m.n_owned, num_sms() * (2048 / NC)), NC, 0, s>>>(U, m, er, ec, (float)er, (float)ec, lmin, lmax, flags);
   else
     refine_flags_kernel<DIM, B><<<grid, 256, 0, s>>>(U, m, ind, er, ec, el, lmin, lmax, flags);
   return cudaGetLastError();
