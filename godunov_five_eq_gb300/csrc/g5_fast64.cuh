@@ -9,10 +9,11 @@
 // differ) from fewer of them:
 //   * divisions and square roots on the integer pipes (g5_exact64.h), the
 //     quotients of one divisor sharing its reciprocal;
-//   * about two products in three on the integer pipes (mul64: 0.56 clocks per
+//   * about half of the products on the integer pipes (mul64: 0.56 clocks per
 //     product and SM against 0.60 for the FP64 pipe, which runs beside them;
 //     the split was found by moving groups of products: all of them on the
-//     integer pipes is 8 % slower, the star state's back on the FP64 pipe 2 %);
+//     integer pipes is 8 % slower, the kinetic energies', the HLLC averages' or
+//     the dt/dx scaling back on the FP64 pipe 2 to 3 % each);
 //   * comparisons, minima, maxima, clamps and sign tests on bit patterns;
 //   * factors of 1/2 folded into one fused multiply-add (x +- y/2 rounds once,
 //     as a separate, exact y/2 would) or carried to the next such addition;
@@ -46,6 +47,30 @@ order64(double x)
 {
   const long long b = bits64(x);
   return b ^ ((b >> 63) & 0x7FFFFFFFFFFFFFFFLL);
+}
+
+// -x without the FP64 pipe (a selected -x is a subtraction from -0 there)
+__device__ __forceinline__ double
+neg64(double x)
+{
+  return x64_make(x64_hi(x) ^ 0x80000000u, x64_lo(x));
+}
+
+// x + y where `on`, else x: under a predicate, so that the FP64 pipe has no
+// work where it is off (an ordinary conditional sum is computed and selected)
+__device__ __forceinline__ double
+add_if64(bool on, double x, double y)
+{
+  double r = x;
+  asm volatile("{.reg .pred p; setp.ne.u32 p, %2, 0; @p add.rn.f64 %0, %0, %1;}" : "+d"(r) : "d"(y), "r"((unsigned)on));
+  return r;
+}
+
+// a / b in hardware, off the main path
+static __device__ __noinline__ double
+div_cold64(double a, double b)
+{
+  return a / b;
 }
 
 // max(x, c) for c > 0, x no NaN
@@ -91,9 +116,7 @@ mix_S64(const PhysParams & P, double a0, double a1, bool & bad)
 __device__ __forceinline__ double
 sound64(double rho, double p, double S, double PI, bool stiff, bool & bad)
 {
-  double n = mul64(p, S + 1.0, bad);
-  if (stiff)
-    n = n + PI;
+  const double n = add_if64(stiff, mul64(p, S + 1.0, bad), PI);
   return sqrt64(clip0_64(div64(n, mul64(rho, S, bad), bad)), bad);
 }
 
@@ -132,14 +155,8 @@ prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
   const double eint = __fma_rn(-0.5, k2, quot64(u[H::IE], rd, bad));
   const double a0u = u[H::IA0], a1u = 1.0 - a0u;
   const double S = mix_S64(P, a0u, a1u, bad);
-  double       n = mul64(d, eint, bad);
-  double       PI = 0.0;
-  if (stiff)
-  {
-    PI = mix_PI64(P, a0u, a1u, bad);
-    n = n - PI;
-  }
-  const double p = div64(n, S, bad);
+  const double PI = mix_PI64(P, a0u, a1u, bad);
+  const double p = div64(add_if64(stiff, mul64(d, eint, bad), neg64(PI)), S, bad);
   const double a0 = clamp_a64(a0u);
   if constexpr (RAW)
   {
@@ -163,8 +180,7 @@ prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
     {
       const double a1 = 1.0 - a0;
       Sc = mix_S64(P, a0, a1, bad);
-      if (stiff)
-        PIc = mix_PI64(P, a0, a1, bad);
+      PIc = mix_PI64(P, a0, a1, bad);
     }
     return sound64(d, p, Sc, PIc, stiff, bad);
   }
@@ -222,14 +238,10 @@ hllc_side64(const double * q, double S, const PhysParams & P, bool stiff, bool &
   if ((int)x64_hi(p) <= (int)((x64_hi(s.r) & 0x7FF00000u) + (x64_hi(P.smallp) & 0x7FF00000u) - 0x3FD00000u))
     p = floor_p64(p, s.r, P.smallp);
   s.u = q[H::QU];
-  double PI = 0.0;
-  if (stiff)
-    PI = mix_PI64(P, q[H::QA], 1.0 - q[H::QA], bad);
-  double n = mul64(p, S, bad);
-  if (stiff)
-    n = n + PI;
-  const double re = mul64(s.r, div64(n, s.r, bad), bad); // rho e
-  s.p = div64(stiff ? re - PI : re, S, bad);
+  const double PI = stiff ? mix_PI64(P, q[H::QA], 1.0 - q[H::QA], bad) : 0.0;
+  const double n = add_if64(stiff, mulh64(p, S, bad), PI);
+  const double re = mulh64(s.r, div64(n, s.r, bad), bad); // rho e
+  s.p = div64(add_if64(stiff, re, neg64(PI)), S, bad);
   double k = mul64(mul64(s.r, s.u, bad), s.u, bad) + mul64(mul64(s.r, q[H::QV], bad), q[H::QV], bad);
   if constexpr (DIM == 3)
     k = k + mul64(mul64(s.r, q[H::QW], bad), q[H::QW], bad);
@@ -260,13 +272,13 @@ hllc_fast64(const double * ql, const double * qr, const Side64 & L, const Side64
   // between the outer waves: the star state of the upwind side
   if (!(bits64(SL) > 0) && (bits64(us) > 0 || bits64(SR) > 0))
   {
-    const double  ds = left ? -dl : dr; // S - u
+    const double  ds = left ? neg64(dl) : dr; // S - u
     const Recip64 rd = recip64((left ? SL : SR) - us, bad);
     const double  fac = quot64(ds, rd, bad);
-    r0 = mul64(r0, fac, bad);
-    r1 = mul64(r1, fac, bad);
-    ro = mul64(ro, fac, bad);
-    eo = quot64((mul64(ds, eo, bad) - mul64(po, uo, bad)) + mul64(ps, us, bad), rd, bad);
+    r0 = mulh64(r0, fac, bad);
+    r1 = mulh64(r1, fac, bad);
+    ro = mulh64(ro, fac, bad);
+    eo = quot64((mulh64(ds, eo, bad) - mulh64(po, uo, bad)) + mulh64(ps, us, bad), rd, bad);
     uo = us;
     po = ps;
   }
@@ -440,7 +452,7 @@ thinc_pair64(double a0, double aM, double aP, double nd, const PhysParams & P, d
   const double D = tanh_fast64(div64(hb * (a0 - Aa), Bb, bad), bad);
   const double E = div64(D, C, bad);
   right = Aa + div64(Bb * (C + E), 1.0 + D, bad);
-  left = Aa + div64(-Bb * (C - E), 1.0 - D, bad);
+  left = Aa + div64(neg64(Bb) * (C - E), 1.0 - D, bad);
 }
 
 // |n_d| = |g_d| / |g| of a Youngs normal

@@ -475,42 +475,69 @@ hancock_fast64(const double * sQ, double * sRec, int gi, int r, double dtdx, con
 {
   using T = Step2DTraits<B, false>;
   constexpr int G = T::G, S = T::S, GG = G * G, SS = S * S;
-  const bool    stiff = P.pi64 != 0;
+  const bool    stiff = P.pi64 != 0, hancock = P.integrator == 0;
   const int     st = P.st64;
-  double        q[5], dx[5], dy[5];
   bool          bad = false;
-#pragma unroll
-  for (int k = 0; k < 5; ++k)
-  {
-    const double * Qk = sQ + k * GG;
-    q[k] = Qk[gi];
-    dx[k] = 0.0;
-    dy[k] = 0.0;
-    if (st != 0)
-    {
-      dx[k] = slope_fast64(q[k], Qk[gi + 1], Qk[gi - 1], st, bad);
-      dy[k] = slope_fast64(q[k], Qk[gi + G], Qk[gi - G], st, bad);
-    }
-    sRec[k * SS + r] = dx[k];
-    sRec[(5 + k) * SS + r] = dy[k];
-  }
-  const double a0 = sQ[5 * GG + gi], a1 = 1.0 - a0;
-  const double Sm = mix_S64(P, a0, a1, bad);
+  const double  a0 = sQ[5 * GG + gi], a1 = 1.0 - a0;
+  const double  Sm = mix_S64(P, a0, a1, bad);
   sRec[15 * SS + r] = Sm;
-  if (P.integrator == 0)
+  const double rr = sQ[gi] + sQ[GG + gi];
+  Recip64      rd = {};
+  double       c = 0.0;
+  if (hancock)
   {
-    const double  p = q[2], u = q[3], v = q[4];
-    const double  rr = q[0] + q[1];
-    const Recip64 rd = recip64(rr, bad);
-    const double  c = sound64(rr, p, Sm, stiff ? mix_PI64(P, a0, a1, bad) : 0.0, stiff, bad);
-    const double  dxr = mul64(dx[3], rr, bad), dyr = mul64(dy[4], rr, bad);
-    const double  sr0 = mul64(mulh64(-u, dx[0] + dx[1], bad) - dxr, dtdx, bad) + mul64(mulh64(-v, dy[0] + dy[1], bad) - dyr, dtdx, bad);
-    sRec[10 * SS + r] = mul64(sr0, a0, bad);
-    sRec[11 * SS + r] = mulh64(sr0, a1, bad);
-    sRec[12 * SS + r] = mul64(mulh64(-u, dx[2], bad) - mulh64(mul64(dxr, c, bad), c, bad), dtdx, bad) +
-                       mul64(mulh64(-v, dy[2], bad) - mulh64(mul64(dyr, c, bad), c, bad), dtdx, bad);
-    sRec[13 * SS + r] = mul64(mulh64(-u, dx[3], bad) - quot64(dx[2], rd, bad), dtdx, bad) + mul64(mulh64(-v, dy[3], bad), dtdx, bad);
-    sRec[14 * SS + r] = mul64(mulh64(-u, dx[4], bad), dtdx, bad) + mul64(mulh64(-v, dy[4], bad) - quot64(dy[2], rd, bad), dtdx, bad);
+    rd = recip64(rr, bad);
+    c = sound64(rr, sQ[2 * GG + gi], Sm, stiff ? mix_PI64(P, a0, a1, bad) : 0.0, stiff, bad);
+  }
+  // each source is a sum over the two directions, x first; the sums of the
+  // normal and transverse velocity change places between them.  (Rolled, as
+  // the update's directions are: the instruction cache gains more than the
+  // loop costs, 471 -> 461 us with THINC, 386 us without either way.)
+  double sr = 0.0, sp = 0.0, sv[2] = { 0.0, 0.0 };
+#pragma unroll 1
+  for (int e = 0; e < 2; ++e)
+  {
+    const int o = e == 0 ? 1 : G;
+    double    d[5]; // r0 r1 p, normal and transverse velocity
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+    {
+      const int      from = k < 3 ? k : (k == 3 ? 3 + e : 4 - e);
+      const double * Qk = sQ + from * GG + gi;
+      d[k] = st != 0 ? slope_fast64(Qk[0], Qk[o], Qk[-o], st, bad) : 0.0;
+      sRec[(5 * e + from) * SS + r] = d[k];
+    }
+    if (hancock)
+    {
+      const double mu = neg64(sQ[(3 + e) * GG + gi]);
+      const double dr = mul64(d[3], rr, bad);
+      const double tr = mul64(mulh64(mu, d[0] + d[1], bad) - dr, dtdx, bad);
+      const double tp = mul64(mulh64(mu, d[2], bad) - mulh64(mul64(dr, c, bad), c, bad), dtdx, bad);
+      const double tn = mul64(mulh64(mu, d[3], bad) - quot64(d[2], rd, bad), dtdx, bad);
+      const double tt = mul64(mulh64(mu, d[4], bad), dtdx, bad);
+      if (e == 0)
+      {
+        sr = tr;
+        sp = tp;
+        sv[0] = tn;
+        sv[1] = tt;
+      }
+      else
+      {
+        sr = sr + tr;
+        sp = sp + tp;
+        sv[0] = sv[0] + tt;
+        sv[1] = sv[1] + tn;
+      }
+    }
+  }
+  if (hancock)
+  {
+    sRec[10 * SS + r] = mul64(sr, a0, bad);
+    sRec[11 * SS + r] = mulh64(sr, a1, bad);
+    sRec[12 * SS + r] = sp;
+    sRec[13 * SS + r] = sv[0];
+    sRec[14 * SS + r] = sv[1];
   }
   if (bad)
     hancock_cold64<B>(sQ, sRec, gi, r, dtdx, &P);
@@ -716,7 +743,7 @@ update_fast64(const double * uin, double * u2, const double * sFx, const double 
   const bool mp = P.source_term == 1;
   source_factors_fast64<2>(uin, P, st0, st1, bad);
   bad = bad || x64_raw_bad(uin[H::IA1]); // (the rest was tested for the primitives)
-#pragma unroll
+#pragma unroll 1
   for (int dir = 0; dir < 2; ++dir)
   {
     const double * F = dir == 0 ? sFx : sFy;
@@ -1004,7 +1031,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       {
         cold = x64_raw_bad(dtdx_r) || x64_raw_bad(dx);
         const double q = div64(dtdx_r, dx, cold);
-        dtdx_r = cold ? dtdx_r / dx : q;
+        dtdx_r = cold ? div_cold64(dtdx_r, dx) : q;
       }
       else if constexpr (!MIXED)
         dtdx_r = dtdx_r / dx;
@@ -1024,6 +1051,40 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         for (int v = 0; v < H::NV; ++v)
           uin[v] = base[v * NC];
       }
+      if constexpr (fast64)
+      {
+        // (one copy of the conversion for the own cell and the halo)
+        for (int it = owner ? -1 : 0, h = owner ? tid + NT - NC : tid - NC; it < 0 || h < NHALO; ++it)
+        {
+          double u[H::NV];
+          int    gidx;
+          if (it < 0)
+          {
+            gidx = (ci + 2) + G * (cj + 2);
+#pragma unroll
+            for (int v = 0; v < H::NV; ++v)
+              u[v] = uin[v];
+          }
+          else
+          {
+            int gx, gy;
+            halo_coords<B>(h, gx, gy);
+            gidx = (gx + 2) + G * (gy + 2);
+            if (!gather_ghost_2d<B>(a, n, cx0, cy0, gx, gy, u))
+            {
+              raise_status(a.status, STATUS_MESH);
+              const double * own = a.U + (size_t)n * H::NV * NC;
+#pragma unroll
+              for (int v = 0; v < H::NV; ++v)
+                u[v] = own[v * NC];
+            }
+            h += NT;
+          }
+          cold |= store_prim<B, MIXED, STIFF>(sQ, gidx, u, P, eosk);
+        }
+      }
+      else
+      {
       for (int h = NT == NC ? tid : (tid < NC ? tid + NT - NC : tid - NC); h < NHALO; h += NT)
       {
         int gx, gy;
@@ -1041,6 +1102,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       }
       if (owner)
         cold |= store_prim<B, MIXED, STIFF>(sQ, (ci + 2) + G * (cj + 2), uin, P, eosk);
+      }
       if (tid < 10)
         sSlot[tid] = slot_v;
       if (tid == 10)

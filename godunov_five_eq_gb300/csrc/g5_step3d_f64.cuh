@@ -75,7 +75,7 @@ hancock_fast3(const double * sQ, double * sHS, double * sS, int gi, int r, doubl
       const double * Qk = sQ + k * GGG + gi;
       d[k] = st != 0 ? slope_fast64(Qk[0], Qk[o], Qk[-o], st, bad) : 0.0;
     }
-    const double mu = -sQ[(3 + e) * GGG + gi];
+    const double mu = neg64(sQ[(3 + e) * GGG + gi]);
     const double dr = mul64(d[3 + e], rr, bad);
     const double tr = mul64(mulh64(mu, d[0] + d[1], bad) - dr, dtdx, bad);
     const double tp = mul64(mulh64(mu, d[2], bad) - mulh64(mul64(dr, c, bad), c, bad), dtdx, bad);
@@ -334,7 +334,7 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
     bool   cold = x64_raw_bad(dtdx) || x64_raw_bad(dx);
     {
       const double q = div64(dtdx, dx, cold);
-      dtdx = cold ? dtdx / dx : q;
+      dtdx = cold ? div_cold64(dtdx, dx) : q;
     }
 
     // ---------------- phase 1: own cell + halo -> primitives (the threads
