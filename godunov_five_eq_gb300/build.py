@@ -1,7 +1,8 @@
 """In-tree build of libg5gpu.so (sm_103a) with nvcc.
 
-Six translation units compiled in parallel:
-  g5_fp64.cu   FP64 kernels, --fmad=false (bit-reproducible reference arithmetic)
+Eight translation units compiled in parallel:
+  g5_fp64.cu   FP64 kernels beside the steps, --fmad=false (bit-reproducible reference arithmetic)
+  g5_fp64_2d.cu, g5_fp64_3d.cu  FP64 step kernels, --fmad=false
   g5_mixed.cu  FP32-bulk 2D kernels and the FP32-bulk dispatch, --use_fast_math
   g5_mixed3d.cu FP32-bulk 3D kernels, --use_fast_math
   g5_capi.cu   the C ABI (include/g5gpu.h)
@@ -23,6 +24,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 UNITS = {
     "g5_fp64.cu": ["--fmad=false"],
+    "g5_fp64_2d.cu": ["--fmad=false"],
+    "g5_fp64_3d.cu": ["--fmad=false"],
     "g5_mixed.cu": ["--use_fast_math"],
     "g5_mixed3d.cu": ["--use_fast_math"],
     "g5_capi.cu": [],

@@ -61,7 +61,8 @@ fill_outside_kernel(double * U, DevMesh m, PhysParams P)
 }
 
 // CFL rate of one cell (ComputeDtFiveEqFunctor.cpp:87-134) in the reference's
-// arithmetic, and (FAST: the cases of g5_fast64.cuh) from the fast operations
+// arithmetic (KIND 2), and from the fast operations of g5_fast64.cuh (KIND 0
+// stiffened gases, 1 Mie-Grueneisen laws)
 template <int DIM>
 __device__ __forceinline__ double
 cfl_rate_ref64(const double * u, double dx, const PhysParams & P)
@@ -82,18 +83,18 @@ cfl_rate_cold64(State64<DIM> s, double dx, const PhysParams * P)
   return cfl_rate_ref64<DIM>(s.v, dx, *P);
 }
 
-template <int DIM, bool FAST>
+template <int DIM, int KIND>
 __device__ __forceinline__ double
 cfl_rate64(const double * u, double dx, const PhysParams & P)
 {
   using H = V<DIM>;
-  if constexpr (!FAST)
+  if constexpr (KIND == 2)
     return cfl_rate_ref64<DIM>(u, dx, P);
   else
   {
     double        q[H::NQ];
     bool          bad = x64_raw_bad(dx);
-    const double  c = prim_fast64<DIM, true, true>(u, q, P, bad);
+    const double  c = prim_fast64<DIM, true, true, KIND == 1>(u, q, P, bad);
     const Recip64 rdx = recip64(dx, bad);
     double        r = quot64(c + fabs(q[H::QU]), rdx, bad) + quot64(c + fabs(q[H::QV]), rdx, bad);
     if constexpr (DIM == 3)
@@ -138,7 +139,7 @@ max_rate64(double mx, double r)
 }
 
 // ComputeDtFiveEqFunctor: one CTA per block, block max, one atomic per CTA
-template <int DIM, int B, bool FAST>
+template <int DIM, int B, int KIND>
 __global__ void __launch_bounds__(256)
 inv_dt_kernel(const double * U, DevMesh m, const __grid_constant__ PhysParams P, double * invdt)
 {
@@ -155,7 +156,7 @@ inv_dt_kernel(const double * U, DevMesh m, const __grid_constant__ PhysParams P,
 #pragma unroll
       for (int v = 0; v < H::NV; ++v)
         u[v] = U[((size_t)n * H::NV + v) * NC + c];
-      mx = max_rate64(mx, cfl_rate64<DIM, FAST>(u, dx, P));
+      mx = max_rate64(mx, cfl_rate64<DIM, KIND>(u, dx, P));
     }
     block_max_rate64(mx, sred, invdt + (m.inst ? m.inst[n] : 0));
   }
@@ -164,7 +165,7 @@ inv_dt_kernel(const double * U, DevMesh m, const __grid_constant__ PhysParams P,
 // RK2_SSP final stage (SolverGodunovFiveEq.cpp:519-520, the external
 // LinearCombination with the SSP coefficients): U2 = 0.5 U + 0.5 U2 on the
 // owned blocks, fused with the CFL rate of the result (one CTA per block).
-template <int DIM, int B, bool MIXED, bool FAST = false>
+template <int DIM, int B, bool MIXED, int KIND = 2>
 __global__ void __launch_bounds__(256)
 rk2_combine_kernel(const double * U, double * U2, DevMesh m, const __grid_constant__ PhysParams P, double * invdt)
 {
@@ -198,7 +199,7 @@ rk2_combine_kernel(const double * U, double * U2, DevMesh m, const __grid_consta
         mx = fmaxf(mx, r * __frcp_rn(d2f_fast(dx)));
       }
       else if (invdt)
-        mx = max_rate64(mx, cfl_rate64<DIM, FAST>(u, dx, P));
+        mx = max_rate64(mx, cfl_rate64<DIM, KIND>(u, dx, P));
     }
     if constexpr (!MIXED)
     {
@@ -697,13 +698,13 @@ constexpr int NEED_PRESSURE = 1 << 1, NEED_SOUND = 1 << 2, NEED_EKIN = 1 << 3, N
 // every quantity of `need` at once (derived_value one at a time converts the
 // cell for each of them): d[q] of DERIVED_QUANTITY q.  False when a value
 // leaves the range of g5_fast64.cuh.
-template <int DIM>
+template <int DIM, bool MG>
 __device__ __forceinline__ bool
 derived_fast64(const double * u, int need, const PhysParams & P, double * d)
 {
   using H = V<DIM>;
   bool          bad = false;
-  const bool    stiff = P.pi64 != 0;
+  const bool    stiff = mixture_stiff64<MG>(P);
   const double  rho = max_pos64(u[H::ID], P.smallr);
   const Recip64 rd = recip64(rho, bad);
   const double  ux = quot64(u[H::IU], rd, bad), uy = quot64(u[H::IV], rd, bad);
@@ -722,7 +723,7 @@ derived_fast64(const double * u, int need, const PhysParams & P, double * d)
   if (need & (NEED_PRESSURE | NEED_SOUND | NEED_MACH))
   {
     const double a0u = u[H::IA0], a1u = 1.0 - a0u;
-    const double S = mix_S64(P, a0u, a1u, bad), PI = stiff ? mix_PI64(P, a0u, a1u, bad) : 0.0;
+    Mix64        m = mixture64<MG>(P, a0u, a1u, u[H::IAD0], u[H::IAD1], bad);
     // the mixture pressure takes the density of the partial densities in the
     // internal energy, the primitives' pressure ID: usually the same number
     const double dm = max_pos64(u[H::IAD0] + u[H::IAD1], P.smallr);
@@ -731,29 +732,22 @@ derived_fast64(const double * u, int need, const PhysParams & P, double * d)
     double     p = 0.0;
     if ((need & (NEED_SOUND | NEED_MACH)) || same)
     {
-      double n = mul64(rho, __fma_rn(-0.5, k2, quot64(u[H::IE], rd, bad)), bad);
-      if (stiff)
-        n = n - PI;
-      p = div64(n, S, bad);
+      const double n = mul64(rho, __fma_rn(-0.5, k2, quot64(u[H::IE], rd, bad)), bad);
+      p = div64(add_if64(stiff, n, neg64(m.PI)), m.S, bad);
     }
     d[1] = p;
     if ((need & NEED_PRESSURE) && !same)
     {
-      double n = mul64(dm, __fma_rn(-0.5, k2, div64(u[H::IE], dm, bad)), bad);
-      if (stiff)
-        n = n - PI;
-      d[1] = div64(n, S, bad);
+      const double n = mul64(dm, __fma_rn(-0.5, k2, div64(u[H::IE], dm, bad)), bad);
+      d[1] = div64(add_if64(stiff, n, neg64(m.PI)), m.S, bad);
     }
     if (need & (NEED_SOUND | NEED_MACH))
     {
       const double a0 = clamp_a64(a0u);
-      double       Sc = S, PIc = PI;
-      if (bits64(a0) != bits64(a0u))
-      {
-        Sc = mix_S64(P, a0, 1.0 - a0, bad);
-        PIc = stiff ? mix_PI64(P, a0, 1.0 - a0, bad) : 0.0;
-      }
-      d[2] = sound64(rho, p, Sc, PIc, stiff, bad);
+      const double r0 = clamp_r64(u[H::IAD0]), r1 = clamp_r64(u[H::IAD1]);
+      if (bits64(a0) != bits64(a0u) || (MG && (bits64(r0) != bits64(u[H::IAD0]) || bits64(r1) != bits64(u[H::IAD1]))))
+        m = mixture64<MG>(P, a0, 1.0 - a0, r0, r1, bad);
+      d[2] = sound64(rho, p, m, stiff, bad);
       if (need & NEED_MACH)
         d[4] = div64(sqrt64(k2, bad), d[2], bad);
     }
@@ -766,10 +760,10 @@ derived_fast64(const double * u, int need, const PhysParams & P, double * d)
 // variables or of a derived quantity) for blocks [oct_begin, oct_begin +
 // num_octs), in one pass over U: field k of cell g (counted from oct_begin) to
 // out[k * stride + g] (FieldList codes: a variable of U, or FIELD_DERIVED + a
-// derived quantity).  FAST: stiffened gases, the derived quantities computed
-// together; otherwise one by one in the reference's arithmetic.  12 fields (4
+// derived quantity).  KIND 0, 1 (stiffened gases, Mie-Grueneisen laws): the
+// derived quantities computed together; 2: one by one in the reference's arithmetic.  12 fields (4
 // derived) of 486k cells: 262 us with the reference arithmetic per field.
-template <int DIM, int B, bool FAST>
+template <int DIM, int B, int KIND>
 __global__ void __launch_bounds__(256)
 fields_kernel(const double * __restrict__ U, double * __restrict__ out, const __grid_constant__ FieldList fl, long long stride, long long oct_begin,
               long long num_octs, const __grid_constant__ PhysParams P)
@@ -785,11 +779,11 @@ fields_kernel(const double * __restrict__ U, double * __restrict__ out, const __
 #pragma unroll
     for (int v = 0; v < H::NV; ++v)
       u[v] = U[(oct * H::NV + v) * NC + cell];
-    bool fast = FAST;
-    if constexpr (FAST)
+    bool fast = KIND != 2;
+    if constexpr (KIND != 2)
     {
       if (fl.need != 0)
-        fast = derived_fast64<DIM>(u, fl.need, P, d);
+        fast = derived_fast64<DIM, KIND == 1>(u, fl.need, P, d);
     }
     d[0] = u[H::ID];
     for (int k = 0; k < fl.n; ++k)

@@ -31,6 +31,7 @@
 
 #include "g5_common.cuh"
 #include "g5_exact64.h"
+#include "g5_mg64.cuh"
 
 namespace g5
 {
@@ -112,12 +113,41 @@ mix_S64(const PhysParams & P, double a0, double a1, bool & bad)
   return mul64(a0, P.xi[0], bad) + mul64(a1, P.xi[1], bad);
 }
 
-// c = sqrt((p (S + 1) + PI) / (rho S)), clipped at 0
-__device__ __forceinline__ double
-sound64(double rho, double p, double S, double PI, bool stiff, bool & bad)
+// the mixture rules (MG: the general ones of g5_mg64.cuh)
+template <bool MG>
+__device__ __forceinline__ Mix64
+mixture64(const PhysParams & P, double a0, double a1, double ar0, double ar1, bool & bad)
 {
-  const double n = add_if64(stiff, mul64(p, S + 1.0, bad), PI);
-  return sqrt64(clip0_64(div64(n, mul64(rho, S, bad), bad)), bad);
+  Mix64 m;
+  if constexpr (MG)
+  {
+    const MixBad64 r = mg_mixture_fast64(&P, a0, a1, ar0, ar1);
+    m = r.m;
+    bad = bad || r.bad;
+  }
+  else
+  {
+    m.S = mix_S64(P, a0, a1, bad);
+    m.PI = m.C0 = mix_PI64(P, a0, a1, bad);
+    m.C1 = m.S + 1.0;
+  }
+  return m;
+}
+
+// whether the mixture has a PI and a C0
+template <bool MG>
+__device__ __forceinline__ bool
+mixture_stiff64(const PhysParams & P)
+{
+  return MG || P.pi64 != 0;
+}
+
+// c = sqrt((p C1 + C0) / (rho S)), clipped at 0
+__device__ __forceinline__ double
+sound64(double rho, double p, const Mix64 & m, bool stiff, bool & bad)
+{
+  const double n = add_if64(stiff, mul64(p, m.C1, bad), m.C0);
+  return sqrt64(clip0_64(div64(n, mul64(rho, m.S, bad), bad)), bad);
 }
 
 // clamps of computePrimitives: a partial density below 1e-12, and the volume
@@ -137,12 +167,12 @@ clamp_a64(double a)
 
 // prim_fp64 (stiffened gases); the sound speed only when asked for.  RAW: the
 // state comes from memory
-template <int DIM, bool SOUND, bool RAW>
+template <int DIM, bool SOUND, bool RAW, bool MG>
 __device__ __forceinline__ double
 prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
 {
   using H = V<DIM>;
-  const bool    stiff = P.pi64 != 0;
+  const bool    stiff = mixture_stiff64<MG>(P);
   const double  d = max_pos64(u[H::ID], P.smallr);
   const Recip64 rd = recip64(d, bad);
   const double  ux = quot64(u[H::IU], rd, bad), uy = quot64(u[H::IV], rd, bad);
@@ -154,9 +184,8 @@ prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
   }
   const double eint = __fma_rn(-0.5, k2, quot64(u[H::IE], rd, bad));
   const double a0u = u[H::IA0], a1u = 1.0 - a0u;
-  const double S = mix_S64(P, a0u, a1u, bad);
-  const double PI = mix_PI64(P, a0u, a1u, bad);
-  const double p = div64(add_if64(stiff, mul64(d, eint, bad), neg64(PI)), S, bad);
+  Mix64        m = mixture64<MG>(P, a0u, a1u, u[H::IAD0], u[H::IAD1], bad);
+  const double p = div64(add_if64(stiff, mul64(d, eint, bad), neg64(m.PI)), m.S, bad);
   const double a0 = clamp_a64(a0u);
   if constexpr (RAW)
   {
@@ -175,14 +204,10 @@ prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
   q[H::QA] = a0;
   if constexpr (SOUND)
   {
-    double Sc = S, PIc = PI;
-    if (bits64(a0) != bits64(a0u))
-    {
-      const double a1 = 1.0 - a0;
-      Sc = mix_S64(P, a0, a1, bad);
-      PIc = mix_PI64(P, a0, a1, bad);
-    }
-    return sound64(d, p, Sc, PIc, stiff, bad);
+    // (the mixture of the clamped state)
+    if (bits64(a0) != bits64(a0u) || (MG && (bits64(q[H::QR0]) != bits64(u[H::IAD0]) || bits64(q[H::QR1]) != bits64(u[H::IAD1]))))
+      m = mixture64<MG>(P, a0, 1.0 - a0, q[H::QR0], q[H::QR1], bad);
+    return sound64(d, p, m, stiff, bad);
   }
   return 0.0;
 }
@@ -213,8 +238,8 @@ slope_fast64(double q, double qPlus, double qMinus, int st, bool & bad)
   return same ? m : x64_make(order64(qPlus) >= order64(qMinus) ? 0u : 0x80000000u, 0u);
 }
 
-// HLLC (hllc_fp64) of two reconstructed states with the mixture's S of either
-// side, scaled by dt/dx.  f: FR0 FR1 FA0 FA1 FE FU FV (FW) FUS.
+// HLLC (hllc_fp64) of two reconstructed states, scaled by dt/dx; S the
+// mixture's of the side (stiffened gases; MG evaluates the mixture here).  f: FR0 FR1 FA0 FA1 FE FU FV (FW) FUS.
 static __device__ __noinline__ double
 floor_p64(double p, double r, double smallp)
 {
@@ -226,11 +251,12 @@ struct Side64
   double r, u, p, e, c; // density, normal velocity, pressure, total energy, sound speed (at least smallc)
 };
 
-template <int DIM>
+template <int DIM, bool MG>
 __device__ __forceinline__ Side64
-hllc_side64(const double * q, double S, const PhysParams & P, bool stiff, bool & bad)
+hllc_side64(const double * q, double S, const PhysParams & P, bool & bad)
 {
   using H = V<DIM>;
+  const bool stiff = mixture_stiff64<MG>(P);
   Side64 s;
   s.r = max_pos64(q[H::QR0] + q[H::QR1], P.smallr);
   double p = q[H::QP];
@@ -238,15 +264,23 @@ hllc_side64(const double * q, double S, const PhysParams & P, bool stiff, bool &
   if ((int)x64_hi(p) <= (int)((x64_hi(s.r) & 0x7FF00000u) + (x64_hi(P.smallp) & 0x7FF00000u) - 0x3FD00000u))
     p = floor_p64(p, s.r, P.smallp);
   s.u = q[H::QU];
-  const double PI = stiff ? mix_PI64(P, q[H::QA], 1.0 - q[H::QA], bad) : 0.0;
-  const double n = add_if64(stiff, mulh64(p, S, bad), PI);
+  Mix64 m;
+  if constexpr (MG)
+    m = mixture64<true>(P, q[H::QA], 1.0 - q[H::QA], q[H::QR0], q[H::QR1], bad);
+  else
+  {
+    m.S = S;
+    m.PI = m.C0 = stiff ? mix_PI64(P, q[H::QA], 1.0 - q[H::QA], bad) : 0.0;
+    m.C1 = S + 1.0;
+  }
+  const double n = add_if64(stiff, mulh64(p, m.S, bad), m.PI);
   const double re = mulh64(s.r, div64(n, s.r, bad), bad); // rho e
-  s.p = div64(add_if64(stiff, re, neg64(PI)), S, bad);
+  s.p = div64(add_if64(stiff, re, neg64(m.PI)), m.S, bad);
   double k = mul64(mul64(s.r, s.u, bad), s.u, bad) + mul64(mul64(s.r, q[H::QV], bad), q[H::QV], bad);
   if constexpr (DIM == 3)
     k = k + mul64(mul64(s.r, q[H::QW], bad), q[H::QW], bad);
   s.e = __fma_rn(0.5, k, re);
-  const double c = sound64(s.r, s.p, S, PI, stiff, bad);
+  const double c = sound64(s.r, s.p, m, stiff, bad);
   s.c = max_pos64(c, P.smallc);
   return s;
 }
@@ -297,8 +331,8 @@ hllc_fast64(const double * ql, const double * qr, const Side64 & L, const Side64
   f[H::FUS] = mul64(uo, dtdx, bad);
 }
 
-// source_factors_fp64 (stiffened gases)
-template <int DIM>
+// source_factors_fp64 (MG: left to the reference arithmetic)
+template <int DIM, bool MG>
 __device__ __forceinline__ void
 source_factors_fast64(const double * u, const PhysParams & P, double & st0, double & st1, bool & bad)
 {
@@ -306,6 +340,11 @@ source_factors_fast64(const double * u, const PhysParams & P, double & st0, doub
   st0 = st1 = 1.0;
   if (P.source_term != 1)
     return;
+  if constexpr (MG)
+  {
+    bad = true;
+    return;
+  }
   const double  d = max_pos64(u[H::IAD0] + u[H::IAD1], P.smallr);
   const Recip64 rdd = recip64(max_pos64(u[H::ID], P.smallr), bad);
   const double  ux = quot64(u[H::IU], rdd, bad), uy = quot64(u[H::IV], rdd, bad);
@@ -338,7 +377,7 @@ alpha_inc64(double fl, double fr, double usl, double usr, double st, double a, b
 
 // end of the update: renormalised volume fractions and ID, then the new
 // state's CFL rate (ComputeDtFiveEqFunctor) when asked for
-template <int DIM>
+template <int DIM, bool MG>
 __device__ __forceinline__ double
 finish_fast64(double * u2, double dx, const PhysParams & P, bool want_dt, bool & bad)
 {
@@ -354,7 +393,7 @@ finish_fast64(double * u2, double dx, const PhysParams & P, bool want_dt, bool &
   if (!want_dt)
     return 0.0;
   double        q[H::NQ];
-  const double  c = prim_fast64<DIM, true, false>(u2, q, P, bad);
+  const double  c = prim_fast64<DIM, true, false, MG>(u2, q, P, bad);
   const Recip64 rdx = recip64(dx, bad);
   double        r = quot64(c + fabs(q[H::QU]), rdx, bad) + quot64(c + fabs(q[H::QV]), rdx, bad);
   if constexpr (DIM == 3)

@@ -1,147 +1,15 @@
-// g5_fp64.cu — FP64 instantiations.  Built with --fmad=false so that every
+// g5_fp64.cu — FP64 instantiations beside the steps (g5_fp64_2d.cu,
+// g5_fp64_3d.cu) and the dispatch of every FP64 step.  Built with --fmad=false so that every
 // product and sum is rounded separately, as in the reference's arithmetic.
 #include <algorithm>
 
 #include "g5_aux.cuh"
+#include "g5_fp64_case.h"
 #include "g5_launch.h"
 #include "g5_prolong.cuh"
-#include "g5_step2d.cuh"
-#include "g5_step3d.cuh"
-#include "g5_step3d_f64.cuh"
 
 namespace g5
 {
-
-static int g_num_sms = 0;
-
-static int
-num_sms()
-{
-  if (g_num_sms == 0)
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_num_sms <= 0)
-      g_num_sms = 1;
-  }
-  return g_num_sms;
-}
-
-// whether the case takes the fast FP64 form (g5_fast64.cuh): stiffened gases,
-// its constants within the form's range (zero allowed where it may be), floors
-// whose products stay in it
-static bool
-fast64_case(const PhysParams & p)
-{
-  const auto in = [](double x, double lo, double hi) { return x >= lo && x <= hi; };
-  const auto zin = [&](double x) { return x == 0.0 || in(x < 0.0 ? -x : x, 1e-200, 1e200); };
-  bool       ok = !p.mg_any && in(p.smallr, 1e-60, 1e60) && in(p.smallc, 1e-100, 1e100);
-  for (int k = 0; k < 2; ++k)
-    ok = ok && zin(p.xi[k]) && zin(p.gpx[k]) && zin(p.gamma[k]) && zin(p.pinf[k]);
-  return ok;
-}
-
-// the equation-of-state argument of the FP64 step kernels
-constexpr int FAST64 = 0, REF64 = 2;
-
-template <int B, int STIFF>
-static int
-occupancy2d(bool thinc)
-{
-  using T = Step2DTraits<B, false>;
-  const size_t smem = T::smem_bytes + (thinc ? T::smem_thinc : 0);
-  cudaFuncSetAttribute(step2d_kernel<B, false, false, STIFF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(T::smem_bytes + T::smem_thinc));
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step2d_kernel<B, false, false, STIFF>, T::NT, smem);
-  return occ;
-}
-
-template <int B, int STIFF>
-static cudaError_t
-launch_step2d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches)
-{
-  using T = Step2DTraits<B, false>;
-  static const int occs[2] = { std::max(1, occupancy2d<B, STIFF>(false)), std::max(1, occupancy2d<B, STIFF>(true)) };
-  const int        occ = occs[a.p.thinc != 0];
-  const int        per_sm = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
-  int              grid = num_sms() * per_sm;
-  if (grid > step_count(a))
-    grid = step_count(a);
-  cudaError_t e = cudaSuccess;
-  if (grid >= 1)
-  {
-    step2d_kernel<B, false, false, STIFF><<<grid, T::NT, T::smem_bytes + (a.p.thinc != 0 ? T::smem_thinc : 0), s>>>(a);
-    ++*launches;
-    e = cudaGetLastError();
-    if (e != cudaSuccess)
-      return e;
-  }
-  if (a.m.n_defer > 0)
-  {
-    const int n = a.m.n_defer * B;
-    reflux2d_kernel<B, false><<<(n + 31) / 32, 32, 0, s>>>(a);
-    ++*launches;
-    e = cudaGetLastError();
-  }
-  return e;
-}
-
-// the 3D step: the fast form's kernel, or the reference arithmetic's
-template <int STIFF>
-struct Step3dLaunch
-{
-  static constexpr int    NT = STIFF == FAST64 ? Step3D64::NT : Step3DTraits<false>::NT;
-  static constexpr size_t smem_bytes = STIFF == FAST64 ? Step3D64::smem_bytes : Step3DTraits<false>::smem_bytes;
-  static auto
-  kernel()
-  {
-    if constexpr (STIFF == FAST64)
-      return step3d_fast64_kernel;
-    else
-      return step3d_kernel<false>;
-  }
-};
-
-template <int STIFF>
-static int
-occupancy3d()
-{
-  using K = Step3dLaunch<STIFF>;
-  cudaFuncSetAttribute(K::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem_bytes);
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, K::kernel(), K::NT, K::smem_bytes);
-  return occ;
-}
-
-template <int STIFF>
-static cudaError_t
-launch_step3d(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches)
-{
-  using K = Step3dLaunch<STIFF>;
-  static const int occ = std::max(1, occupancy3d<STIFF>());
-  const int        per_sm = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
-  int              grid = num_sms() * per_sm;
-  if (grid > step_count(a))
-    grid = step_count(a);
-  cudaError_t e = cudaSuccess;
-  if (grid >= 1)
-  {
-    K::kernel()<<<grid, K::NT, K::smem_bytes, s>>>(a);
-    ++*launches;
-    e = cudaGetLastError();
-    if (e != cudaSuccess)
-      return e;
-  }
-  if (a.m.n_defer > 0)
-  {
-    const int n = a.m.n_defer * 64;
-    reflux3d_kernel<false><<<(n + 31) / 32, 32, 0, s>>>(a);
-    ++*launches;
-    e = cudaGetLastError();
-  }
-  return e;
-}
 
 bool
 step_supported(int dim, int b)
@@ -246,25 +114,17 @@ launch_step_fp64(int dim, int b, const StepArgs & a, int ctas_per_sm, cudaStream
   const cudaError_t e = launch_prolong(dim, b, a, s, launches);
   if (e != cudaSuccess)
     return e;
-  if (dim == 2 && b == 16)
-    return fast64_case(a.p) ? launch_step2d<16, FAST64>(a, ctas_per_sm, s, launches) : launch_step2d<16, REF64>(a, ctas_per_sm, s, launches);
-  if (dim == 2 && b == 8)
-    return fast64_case(a.p) ? launch_step2d<8, FAST64>(a, ctas_per_sm, s, launches) : launch_step2d<8, REF64>(a, ctas_per_sm, s, launches);
+  if (dim == 2)
+    return launch_step2d_fp64(b, a, ctas_per_sm, s, launches);
   if (dim == 3 && b == 8)
-    return fast64_case(a.p) ? launch_step3d<FAST64>(a, ctas_per_sm, s, launches) : launch_step3d<REF64>(a, ctas_per_sm, s, launches);
+    return launch_step3d_fp64(a, ctas_per_sm, s, launches);
   return cudaErrorInvalidValue;
 }
 
 int
 step_max_ctas_per_sm_fp64(int dim, int b)
 {
-  if (dim == 2 && b == 16)
-    return std::min(occupancy2d<16, FAST64>(true), occupancy2d<16, REF64>(true));
-  if (dim == 2 && b == 8)
-    return std::min(occupancy2d<8, FAST64>(true), occupancy2d<8, REF64>(true));
-  if (dim == 3 && b == 8)
-    return std::min(occupancy3d<FAST64>(), occupancy3d<REF64>());
-  return 0;
+  return dim == 2 ? step_max_ctas_per_sm_fp64_2d(b) : (dim == 3 && b == 8 ? step_max_ctas_per_sm_fp64_3d() : 0);
 }
 
 template <int DIM, int B>
@@ -300,11 +160,10 @@ inv_dt_t(const double * U, const DevMesh & m, const PhysParams & p, double * inv
   int grid = num_sms() * 8;
   if (grid > m.n_owned)
     grid = m.n_owned;
-  if (fast64_case(p))
-    inv_dt_kernel<DIM, B, true><<<grid, 256, 0, s>>>(U, m, p, invdt);
-  else
-    inv_dt_kernel<DIM, B, false><<<grid, 256, 0, s>>>(U, m, p, invdt);
-  return cudaGetLastError();
+  return launch_case64(p, [&](auto k) {
+    inv_dt_kernel<DIM, B, k.value><<<grid, 256, 0, s>>>(U, m, p, invdt);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t
@@ -328,11 +187,10 @@ rk2_t(const double * U, double * U2, const DevMesh & m, const PhysParams & p, do
   int grid = num_sms() * 8;
   if (grid > m.n_owned)
     grid = m.n_owned;
-  if (fast64_case(p))
-    rk2_combine_kernel<DIM, B, false, true><<<grid, 256, 0, s>>>(U, U2, m, p, invdt);
-  else
-    rk2_combine_kernel<DIM, B, false, false><<<grid, 256, 0, s>>>(U, U2, m, p, invdt);
-  return cudaGetLastError();
+  return launch_case64(p, [&](auto k) {
+    rk2_combine_kernel<DIM, B, false, k.value><<<grid, 256, 0, s>>>(U, U2, m, p, invdt);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t
@@ -435,11 +293,10 @@ fields_t(const double * U, double * out, const FieldList & fl, long long stride,
   if (total <= 0)
     return cudaSuccess;
   const unsigned grid = (unsigned)std::min<long long>((total + 255) / 256, (long long)num_sms() * 16);
-  if (fast64_case(p))
-    fields_kernel<DIM, B, true><<<grid, 256, 0, s>>>(U, out, fl, stride, oct_begin, num_octs, p);
-  else
-    fields_kernel<DIM, B, false><<<grid, 256, 0, s>>>(U, out, fl, stride, oct_begin, num_octs, p);
-  return cudaGetLastError();
+  return launch_case64(p, [&](auto k) {
+    fields_kernel<DIM, B, k.value><<<grid, 256, 0, s>>>(U, out, fl, stride, oct_begin, num_octs, p);
+    return cudaGetLastError();
+  });
 }
 
 static cudaError_t

@@ -48,6 +48,13 @@ cudaError_t launch_derived(int dim, int b, const double * U, double * out, int q
 cudaError_t launch_pack_fields(int dim, int b, const double * U, double * out, const int * codes, int n, long long oct_begin,
                                long long num_octs, const PhysParams & p, cudaStream_t s);
 
+// the FP64 steps (g5_fp64_2d.cu, g5_fp64_3d.cu) and the occupancy maxima of
+// their kernels
+cudaError_t launch_step2d_fp64(int b, const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches);
+cudaError_t launch_step3d_fp64(const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches);
+int         step_max_ctas_per_sm_fp64_2d(int b);
+int         step_max_ctas_per_sm_fp64_3d();
+
 // the FP32-bulk 3D step of case v = 3 THINC + equation-of-state kind
 // (g5_mixed3d.cu) and the occupancy maximum of its kernels
 cudaError_t launch_step3d_mixed_case(int v, const StepArgs & a, int ctas_per_sm, cudaStream_t s, int * launches);

@@ -176,7 +176,7 @@ store_prim(typename Step2DTraits<B, MIXED>::R * sQ, int gidx, const double * u, 
     if constexpr (STIFF == 2)
       prim_fp64<2>(u, q, P);
     else
-      prim_fast64<2, false, true>(u, q, P, bad);
+      prim_fast64<2, false, true, STIFF == 1>(u, q, P, bad);
     if (bad)
     {
       State64<2> s;
@@ -401,7 +401,7 @@ face_state_fast64(const double * sQ, const double * sRec, const double * sAF, in
   return Sm;
 }
 
-template <int B>
+template <int B, bool MG>
 __device__ __forceinline__ bool
 face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, double * sF, int dir, int ff, double dtdx, const PhysParams & P)
 {
@@ -413,8 +413,8 @@ face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, dou
   bool         bad = false;
   const double Sl = face_state_fast64<B>(sQ, sRec, sAF, li, lj, dir, 1, P, qL, bad);
   const double Sr = face_state_fast64<B>(sQ, sRec, sAF, ri, rj, dir, -1, P, qR, bad);
-  const Side64 L = hllc_side64<2>(qL, Sl, P, P.pi64 != 0, bad);
-  const Side64 R = hllc_side64<2>(qR, Sr, P, P.pi64 != 0, bad);
+  const Side64 L = hllc_side64<2, MG>(qL, Sl, P, bad);
+  const Side64 R = hllc_side64<2, MG>(qR, Sr, P, bad);
   hllc_fast64<2>(qL, qR, L, R, dtdx, fl, bad);
   if (bad)
   {
@@ -469,25 +469,25 @@ hancock_cold64(const double * sQ, double * sRec, int gi, int r, double dtdx, con
 }
 
 // the same values from the fast operations, and the mixture's S of the cell
-template <int B>
+template <int B, bool MG>
 __device__ __forceinline__ bool
 hancock_fast64(const double * sQ, double * sRec, int gi, int r, double dtdx, const PhysParams & P)
 {
   using T = Step2DTraits<B, false>;
   constexpr int G = T::G, S = T::S, GG = G * G, SS = S * S;
-  const bool    stiff = P.pi64 != 0, hancock = P.integrator == 0;
+  const bool    stiff = mixture_stiff64<MG>(P), hancock = P.integrator == 0;
   const int     st = P.st64;
   bool          bad = false;
   const double  a0 = sQ[5 * GG + gi], a1 = 1.0 - a0;
-  const double  Sm = mix_S64(P, a0, a1, bad);
-  sRec[15 * SS + r] = Sm;
+  const Mix64   m = mixture64<MG>(P, a0, a1, sQ[gi], sQ[GG + gi], bad);
+  sRec[15 * SS + r] = m.S;
   const double rr = sQ[gi] + sQ[GG + gi];
   Recip64      rd = {};
   double       c = 0.0;
   if (hancock)
   {
     rd = recip64(rr, bad);
-    c = sound64(rr, sQ[2 * GG + gi], Sm, stiff ? mix_PI64(P, a0, a1, bad) : 0.0, stiff, bad);
+    c = sound64(rr, sQ[2 * GG + gi], m, stiff, bad);
   }
   // each source is a sum over the two directions, x first; the sums of the
   // normal and transverse velocity change places between them.  (Rolled, as
@@ -727,9 +727,9 @@ update_cold64(State64<2> uin, double * out, const double * sFx, const double * s
   return r;
 }
 
-// update_fp64 from the fast operations (stiffened gases).  (The reference
+// update_fp64 from the fast operations.  (The reference
 // starts each sum from 0 + F_left: the same value but for the sign of a zero.)
-template <int B>
+template <int B, bool MG>
 __device__ __forceinline__ double
 update_fast64(const double * uin, double * u2, const double * sFx, const double * sFy, int ci, int cj, double dx, const PhysParams & P, bool want_dt,
               bool & bad)
@@ -741,7 +741,7 @@ update_fast64(const double * uin, double * u2, const double * sFx, const double 
     u2[v] = uin[v];
   double     st0, st1;
   const bool mp = P.source_term == 1;
-  source_factors_fast64<2>(uin, P, st0, st1, bad);
+  source_factors_fast64<2, MG>(uin, P, st0, st1, bad);
   bad = bad || x64_raw_bad(uin[H::IA1]); // (the rest was tested for the primitives)
 #pragma unroll 1
   for (int dir = 0; dir < 2; ++dir)
@@ -758,7 +758,7 @@ update_fast64(const double * uin, double * u2, const double * sFx, const double 
     u2[H::IU] += F[H::FU * NFF + il] - F[H::FU * NFF + ir];
     u2[H::IV] += F[H::FV * NFF + il] - F[H::FV * NFF + ir];
   }
-  return finish_fast64<2>(u2, dx, P, want_dt, bad);
+  return finish_fast64<2, MG>(u2, dx, P, want_dt, bad);
 }
 
 // The same update in the FP32-bulk form.  FP64 is used only for the adds
@@ -948,9 +948,9 @@ finish_deferred_2d(const StepArgs & a, int j)
 // THINC, STIFF: the FP32-bulk form is compiled with and without the THINC
 // reconstruction and the stiffened-gas pressure path (P picks the kernel), so
 // a kernel carries only the code its case runs; the FP64 form tests THINC at
-// run time and has STIFF = 2 (the reference arithmetic: Mie-Grueneisen laws,
-// floors outside the fast form's range) and 0 (the fast form of
-// g5_fast64.cuh: stiffened gases).  FUSED: the FP32-bulk form finishing the coarse/fine
+// run time and has STIFF = 0 and 1 (the fast form of g5_fast64.cuh: stiffened
+// gases, Mie-Grueneisen laws) and 2 (the reference arithmetic: constants
+// outside the fast form's range).  FUSED: the FP32-bulk form finishing the coarse/fine
 // records in its tail (m.fin_tgt set; the kernel without it keeps the plain
 // block loop)
 template <int B, bool MIXED, bool THINC = false, int STIFF = -1, bool FUSED = false>
@@ -1155,7 +1155,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
             if (cold0)
               hancock_cold64<B>(sQ, sRec, gi, r, dtdx_r, &P);
             else
-              cold |= hancock_fast64<B>(sQ, sRec, gi, r, dtdx_r, P);
+              cold |= hancock_fast64<B, STIFF == 1>(sQ, sRec, gi, r, dtdx_r, P);
           }
         }
         else
@@ -1249,7 +1249,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
           else if (cold1)
             face_flux_cold64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, &P);
           else
-            cold |= face_flux_fast64<B>(sQ, sRec, sAF, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
+            cold |= face_flux_fast64<B, STIFF == 1>(sQ, sRec, sAF, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
         }
       }
       // the own cell's state for the update: the FP32-bulk form without the
@@ -1343,7 +1343,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         {
           bool bad = cold;
           if (!bad)
-            m_inv = update_fast64<B>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr, bad);
+            m_inv = update_fast64<B, STIFF == 1>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr, bad);
           if (bad)
           {
             State64<2> st;

@@ -1,5 +1,5 @@
 // g5_step3d_f64.cuh — the 3D block timestep in FP64 with the fast arithmetic
-// of g5_fast64.cuh (stiffened gases).  The phases, the shared arrays and the
+// of g5_fast64.cuh (MG: the Mie-Grueneisen mixture rules).  The phases, the shared arrays and the
 // coarse/fine records are those of step3d_kernel (g5_step3d.cuh), whose FP64
 // form is the reference arithmetic; the results are the same doubles.
 //
@@ -45,6 +45,7 @@ ring_stride3(int dir)
 
 // Hancock source of one face-neighbour cell (hancock_ref3 in the fast
 // operations) and the mixture's S; true when a value left the range
+template <bool MG>
 __device__ __forceinline__ bool
 hancock_fast3(const double * sQ, double * sHS, double * sS, int gi, int r, double dtdx, const PhysParams & P)
 {
@@ -52,16 +53,16 @@ hancock_fast3(const double * sQ, double * sHS, double * sS, int gi, int r, doubl
   constexpr int G = T::G, GG = T::GG, GGG = T::GGG, SSS = T::SSS;
   bool          bad = false;
   const double  a0 = sQ[6 * GGG + gi], a1 = 1.0 - a0;
-  const double  S = mix_S64(P, a0, a1, bad);
-  sS[r] = S;
+  const Mix64   m = mixture64<MG>(P, a0, a1, sQ[gi], sQ[GGG + gi], bad);
+  sS[r] = m.S;
   if (P.integrator != 0)
     return bad;
   const int     st = P.st64;
-  const bool    stiff = P.pi64 != 0;
+  const bool    stiff = mixture_stiff64<MG>(P);
   const double  p = sQ[2 * GGG + gi];
   const double  rr = sQ[gi] + sQ[GGG + gi];
   const Recip64 rd = recip64(rr, bad);
-  const double  c = sound64(rr, p, S, stiff ? mix_PI64(P, a0, a1, bad) : 0.0, stiff, bad);
+  const double  c = sound64(rr, p, m, stiff, bad);
   // each source is a sum over the directions, x first
   double sr = 0.0, sp = 0.0, sv[3] = { 0.0, 0.0, 0.0 };
 #pragma unroll
@@ -225,6 +226,7 @@ thinc_eval3(const double * sQ, double * sAF, int dir, int i, const PhysParams & 
 }
 
 // HLLC flux of face f of direction dir, scaled by dt/dx (face_flux3<false>)
+template <bool MG>
 __device__ __forceinline__ bool
 face_flux_fast3(const double * sQ, const double * sHS, const double * sS, const double * sAF, double * sF, int f, int dir, double dtdx, const PhysParams & P)
 {
@@ -239,8 +241,8 @@ face_flux_fast3(const double * sQ, const double * sHS, const double * sS, const 
   bool          bad = false;
   const double  Sl = face_state_fast3(sQ, sHS, sS, sAF, gR - o, sR - ring_stride3(dir), thinc_index3(dir, fi - (dir == 0), fj - (dir == 1), fk - (dir == 2)), o, dir, 1, P, qL, bad);
   const double  Sr = face_state_fast3(sQ, sHS, sS, sAF, gR, sR, thinc_index3(dir, fi, fj, fk), o, dir, -1, P, qR, bad);
-  const Side64  L = hllc_side64<3>(qL, Sl, P, P.pi64 != 0, bad);
-  const Side64  R = hllc_side64<3>(qR, Sr, P, P.pi64 != 0, bad);
+  const Side64  L = hllc_side64<3, MG>(qL, Sl, P, bad);
+  const Side64  R = hllc_side64<3, MG>(qR, Sr, P, bad);
   hllc_fast64<3>(qL, qR, L, R, dtdx, fl, bad);
   if (bad)
   {
@@ -291,7 +293,8 @@ pack_state3(const double * u)
   return s;
 }
 
-static __global__ void __launch_bounds__(Step3D64::NT, 1)
+template <bool MG>
+__global__ void __launch_bounds__(Step3D64::NT, 1)
 step3d_fast64_kernel(const __grid_constant__ StepArgs a)
 {
   using T = Step3D64::T;
@@ -384,7 +387,7 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
       }
       double q[7];
       bool   bad = false;
-      prim_fast64<3, false, true>(u, q, P, bad);
+      prim_fast64<3, false, true, MG>(u, q, P, bad);
       if (bad)
       {
         cold = true;
@@ -438,7 +441,7 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
       const int gi = (ri + 2) + G * (rj + 2) + GG * (rk + 2);
       bool      bad = cold0;
       if (!bad)
-        bad = hancock_fast3(sQ, sHS, sS, gi, r, dtdx, P);
+        bad = hancock_fast3<MG>(sQ, sHS, sS, gi, r, dtdx, P);
       if (bad)
       {
         cold = true;
@@ -461,7 +464,7 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
       {
         bool bad = cold0;
         if (!bad)
-          source_factors_fast64<3>(u2, P, st0, st1, bad);
+          source_factors_fast64<3, MG>(u2, P, st0, st1, bad);
         if (bad)
         {
           const double2 st = source_cold3(pack_state3(u2), &P);
@@ -499,7 +502,7 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
       }
       bool bad = cold;
       if (!bad)
-        bad = face_flux_fast3(sQ, sHS, sS, sAF, sF, tid, dir, dtdx, P);
+        bad = face_flux_fast3<MG>(sQ, sHS, sS, sAF, sF, tid, dir, dtdx, P);
       else
         face_flux_cold3(sQ, sHS, sF, tid, dir, dtdx, &P);
       cold = __syncthreads_or(bad) != 0;
@@ -605,7 +608,7 @@ step3d_fast64_kernel(const __grid_constant__ StepArgs a)
       if (!bad)
       {
         const double b0 = u2[H::IA0], b1 = u2[H::IA1];
-        m_inv = finish_fast64<3>(u2, dx, P, a.invdt != nullptr, bad);
+        m_inv = finish_fast64<3, MG>(u2, dx, P, a.invdt != nullptr, bad);
         if (bad)
         {
           u2[H::IA0] = b0;
