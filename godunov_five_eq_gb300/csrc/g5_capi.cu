@@ -46,6 +46,10 @@ struct G5Context
   int32_t *            d_batch_work = nullptr;
   uint8_t *            d_inst_active = nullptr;
   unsigned int * d_status = nullptr;
+  // g5_remap's tables on the device: stream-ordered allocations of a pool of
+  // the context's own that keeps its memory (the device's default pool gives
+  // it back at every synchronisation), released by g5_destroy
+  cudaMemPool_t  remap_pool = nullptr;
   int64_t        bytes = 0;
   struct PoolEntry
   {
@@ -301,65 +305,161 @@ do_step(G5Context * c, const double * U, double * U2, const double * d_dt, int m
   return e == cudaSuccess ? G5_OK : G5_ERR_CUDA;
 }
 
-// Plan of g5_step_host for the table being uploaded (host arrays of g5_set_mesh).
-int
-plan_host_pipe(G5Context * c, const G5Mesh * m, const std::vector<int32_t> & defer_slot, const std::vector<int32_t> & defer_list)
+// What g5_set_mesh learns from the host table in one pass over its neighbour
+// rows (3.4 MB for 3,906 3D blocks: separate passes for the checks, the
+// records, the host pipeline and the walk order took 0.63 ms, this one 0.2 ms)
+struct TableScan
 {
-  G5Context::HostPipe & hp = c->pipe;
-  const int             n_owned = m->n_owned, ns = c->ns, nch = c->nch, nfaces = 2 * c->dim;
-  const int             center = c->dim == 2 ? 4 : 13;
+  int                  rc = G5_OK;
+  int                  n_reflux = 0;
+  std::vector<int32_t> reflux_slot, defer_slot, defer_list; // coarse/fine face records
+  std::vector<int>     ready; // g5_step_host: the last copy chunk among a block's own and its neighbours'
+  std::vector<uint8_t> score; // neighbour slots at another level
+};
+
+template <int DIM>
+TableScan
+scan_table(const G5Mesh * m, const std::vector<int> & lo)
+{
+  constexpr int NS = DIM == 2 ? 9 : 27, NCH = 1 << DIM, NF = 2 * DIM, CENTER = NS / 2;
+  TableScan     t;
+  const int     n_owned = m->n_owned, n_total = m->n_owned + m->n_outside;
+  // children of a finer slot that touch the block (bit per child); the slot of each face
+  unsigned need[NS];
+  int      face_slot[NF];
+  for (int s = 0; s < NS; ++s)
+  {
+    const int d[3] = { s % 3 - 1, (s / 3) % 3 - 1, s / 9 - 1 };
+    need[s] = 0;
+    for (int ch = 0; ch < NCH; ++ch)
+    {
+      bool touches = true;
+      for (int e = 0; e < DIM; ++e)
+        if ((d[e] == -1 && !((ch >> e) & 1)) || (d[e] == 1 && ((ch >> e) & 1)))
+          touches = false;
+      need[s] |= touches ? 1u << ch : 0u;
+    }
+  }
+  for (int f = 0; f < NF; ++f)
+  {
+    const int stride = (f >> 1) == 0 ? 1 : ((f >> 1) == 1 ? 3 : 9);
+    face_slot[f] = CENTER + ((f & 1) ? stride : -stride);
+  }
+  std::vector<int> chunk((size_t)n_total, 0); // outside blocks travel with chunk 0
+  for (size_t k = 0; k + 1 < lo.size(); ++k)
+    for (int n = lo[k]; n < lo[k + 1]; ++n)
+      chunk[n] = (int)k;
+  t.ready.resize(n_owned);
+  t.score.resize(n_owned);
+  t.reflux_slot.assign((size_t)n_owned * NF, -1);
+  t.defer_slot.assign((size_t)n_owned * NF, -1);
+  for (int n = 0; n < n_owned; ++n)
+  {
+    const int8_t *  rel = m->nbr_rel + (size_t)n * NS;
+    const int32_t * row = m->nbr + (size_t)n * NS * NCH;
+    int             r = chunk[n], score = 0;
+    for (int s = 0; s < NS; ++s)
+    {
+      // (the center slot counts in the score only, as it always has)
+      score += rel[s] != 0;
+      if (s == CENTER)
+        continue;
+      const int32_t * nb = row + s * NCH;
+      if (rel[s] == 0 || rel[s] == -1)
+      {
+        // (only a finer slot lists more than one block)
+        if ((uint32_t)nb[0] >= (uint32_t)n_total)
+        {
+          t.rc = G5_ERR_MESH;
+          return t;
+        }
+        r = r > chunk[nb[0]] ? r : chunk[nb[0]];
+        continue;
+      }
+      if (rel[s] != 1)
+      {
+        t.rc = G5_ERR_MESH;
+        return t;
+      }
+      for (int ch = 0; ch < NCH; ++ch)
+      {
+        if (nb[ch] >= n_total || (((need[s] >> ch) & 1u) && nb[ch] < 0))
+        {
+          t.rc = G5_ERR_MESH;
+          return t;
+        }
+        if (nb[ch] >= 0)
+          r = r > chunk[nb[ch]] ? r : chunk[nb[ch]];
+      }
+    }
+    t.ready[n] = r;
+    t.score[n] = (uint8_t)score;
+    for (int f = 0; f < NF; ++f)
+    {
+      const int       s = face_slot[f];
+      const int32_t * nb = row + s * NCH;
+      if (rel[s] < 0 && nb[0] < n_owned)
+        t.reflux_slot[(size_t)n * NF + f] = t.n_reflux++;
+      if (rel[s] > 0)
+      {
+        bool owned = true;
+        for (int ch = 0; ch < NCH; ++ch)
+          if (nb[ch] >= n_owned)
+            owned = false;
+        if (owned)
+        {
+          t.defer_slot[(size_t)n * NF + f] = (int32_t)t.defer_list.size();
+          t.defer_list.push_back(n * 8 + f);
+        }
+      }
+    }
+  }
+  return t;
+}
+
+// Copy chunks of g5_step_host: bounds of the owned blocks of each
+std::vector<int>
+host_chunks(const G5Context * c, const G5Mesh * m)
+{
   // 8 chunks of at least 64 blocks, or in 2D more (up to 16) when the chunks
   // would exceed about 3.5 MB (the copy of chunk 0 is the pipeline's start-up
   // latency, each chunk's step launch has a fixed cost; 3D chunks of that size
   // hold too few blocks whose 26 neighbours have all arrived)
-  const double          mbytes = (double)(n_owned + m->n_outside) * c->nv * (c->dim == 2 ? c->b * c->b : c->b * c->b * c->b) * 8.0 / (1 << 20);
-  int                   K = n_owned / 64;
+  const int    n_owned = m->n_owned;
+  const double mbytes = (double)(n_owned + m->n_outside) * c->nv * (c->dim == 2 ? c->b * c->b : c->b * c->b * c->b) * 8.0 / (1 << 20);
+  int          K = n_owned / 64;
   K = K > 8 ? 8 : K;
-  const int             Kb = (int)(mbytes / 3.5 + 0.5);
+  const int Kb = (int)(mbytes / 3.5 + 0.5);
   K = c->dim == 2 && Kb > K && Kb <= n_owned / 64 ? Kb : K;
   K = K < 1 ? 1 : (K > 16 ? 16 : K);
-  hp.K = K;
-  hp.lo.assign(K + 1, 0);
+  std::vector<int> lo(K + 1);
   for (int k = 0; k <= K; ++k)
-    hp.lo[k] = (int)((int64_t)n_owned * k / K);
-  std::vector<int> chunk(n_owned);
-  for (int k = 0; k < K; ++k)
-    for (int n = hp.lo[k]; n < hp.lo[k + 1]; ++n)
-      chunk[n] = k;
-  // outside blocks travel with chunk 0
-  auto arrival = [&](int b) { return b >= n_owned ? 0 : chunk[b]; };
-  std::vector<int> ready(n_owned);
-  for (int n = 0; n < n_owned; ++n)
-  {
-    int r = chunk[n];
-    for (int s = 0; s < ns; ++s)
-    {
-      if (s == center)
-        continue;
-      const int32_t * nb = m->nbr + ((size_t)n * ns + s) * nch;
-      // only a finer slot lists more than one block
-      const int       nread = m->nbr_rel[(size_t)n * ns + s] > 0 ? nch : 1;
-      for (int ch = 0; ch < nread; ++ch)
-        if (nb[ch] >= 0)
-          r = r > arrival(nb[ch]) ? r : arrival(nb[ch]);
-    }
-    ready[n] = r;
-  }
+    lo[k] = (int)((int64_t)n_owned * k / K);
+  return lo;
+}
+
+// Plan of g5_step_host for the table being uploaded (host arrays of g5_set_mesh).
+int
+plan_host_pipe(G5Context * c, const G5Mesh * m, const std::vector<int> & lo, const TableScan & t)
+{
+  G5Context::HostPipe &  hp = c->pipe;
+  const int              n_owned = m->n_owned, ns = c->ns, nch = c->nch, K = (int)lo.size() - 1;
+  const std::vector<int> & ready = t.ready;
+  hp.K = K;
+  hp.lo = lo;
   // a block with coarse/fine records is final once its finer face neighbours are stepped
   std::vector<int> final_(ready);
-  for (int n = 0; n < n_owned; ++n)
-    for (int f = 0; f < nfaces; ++f)
-    {
-      if (defer_slot.empty() || defer_slot[(size_t)n * nfaces + f] < 0)
-        continue;
-      int d[3] = { 0, 0, 0 };
-      d[f >> 1] = (f & 1) ? 1 : -1;
-      const int       s = (d[0] + 1) + 3 * (d[1] + 1) + (c->dim == 3 ? 9 * (d[2] + 1) : 0);
-      const int32_t * nb = m->nbr + ((size_t)n * ns + s) * nch;
-      for (int ch = 0; ch < nch; ++ch)
-        if (nb[ch] >= 0 && nb[ch] < n_owned)
-          final_[n] = final_[n] > ready[nb[ch]] ? final_[n] : ready[nb[ch]];
-    }
+  for (int32_t code : t.defer_list)
+  {
+    const int n = code >> 3, f = code & 7;
+    int       d[3] = { 0, 0, 0 };
+    d[f >> 1] = (f & 1) ? 1 : -1;
+    const int       s = (d[0] + 1) + 3 * (d[1] + 1) + (c->dim == 3 ? 9 * (d[2] + 1) : 0);
+    const int32_t * nb = m->nbr + ((size_t)n * ns + s) * nch;
+    for (int ch = 0; ch < nch; ++ch)
+      if (nb[ch] >= 0 && nb[ch] < n_owned)
+        final_[n] = final_[n] > ready[nb[ch]] ? final_[n] : ready[nb[ch]];
+  }
   std::vector<int32_t>   work;
   std::vector<int32_t> & recs = hp.recs;
   recs.clear();
@@ -372,7 +472,7 @@ plan_host_pipe(G5Context * c, const G5Mesh * m, const std::vector<int32_t> & def
       if (ready[n] == k)
         work.push_back(n);
     hp.rec_off[k] = (int)recs.size();
-    for (int32_t code : defer_list)
+    for (int32_t code : t.defer_list)
       if (final_[code >> 3] == k)
         recs.push_back(code);
   }
@@ -381,8 +481,9 @@ plan_host_pipe(G5Context * c, const G5Mesh * m, const std::vector<int32_t> & def
   hp.out_off.assign(K + 1, 0);
   hp.out_list.clear();
   std::vector<int> out_ready(K, 0);
-  for (int n = 0; n < n_owned; ++n)
-    out_ready[chunk[n]] = out_ready[chunk[n]] > final_[n] ? out_ready[chunk[n]] : final_[n];
+  for (int k = 0; k < K; ++k)
+    for (int n = lo[k]; n < lo[k + 1]; ++n)
+      out_ready[k] = out_ready[k] > final_[n] ? out_ready[k] : final_[n];
   for (int k = 0; k < K; ++k)
   {
     hp.out_off[k] = (int)hp.out_list.size();
@@ -479,6 +580,8 @@ g5_destroy(G5Context * ctx)
     cudaStreamDestroy(hp.s_in);
   if (hp.s_out)
     cudaStreamDestroy(hp.s_out);
+  if (ctx->remap_pool)
+    cudaMemPoolDestroy(ctx->remap_pool); // (outstanding frees complete first)
   delete ctx;
   return G5_OK;
 }
@@ -496,37 +599,18 @@ g5_set_mesh(G5Context * c, const G5Mesh * m)
   const int n_owned = m->n_owned, n_total = m->n_owned + m->n_outside;
   const int n_inst = m->n_inst > 0 ? m->n_inst : 1;
   const int ns = c->ns, nch = c->nch, dim = c->dim;
-  // ---- validate the table (the reference asserts these in StencilHelper / hashmap lookups)
-  if (g5::validate_table(dim, m) != G5_OK)
+  // ---- validate the table (the reference asserts these in StencilHelper /
+  // hashmap lookups; the neighbour rows in the scan)
+  if (g5::validate_blocks(m) != G5_OK)
     return G5_ERR_MESH;
-
-  // ---- coarse/fine face records
-  const int            nfaces = 2 * dim;
-  std::vector<int32_t> reflux_slot((size_t)n_owned * nfaces, -1), defer_slot((size_t)n_owned * nfaces, -1), defer_list;
-  int                  n_reflux = 0, n_defer = 0;
-  for (int n = 0; n < n_owned; ++n)
-    for (int f = 0; f < nfaces; ++f)
-    {
-      int d[3] = { 0, 0, 0 };
-      d[f >> 1] = (f & 1) ? 1 : -1;
-      const int s = (d[0] + 1) + 3 * (d[1] + 1) + (dim == 3 ? 9 * (d[2] + 1) : 0);
-      const int rel = m->nbr_rel[(size_t)n * ns + s];
-      const int * nb = m->nbr + ((size_t)n * ns + s) * nch;
-      if (rel < 0 && nb[0] < n_owned)
-        reflux_slot[(size_t)n * nfaces + f] = n_reflux++;
-      if (rel > 0)
-      {
-        bool owned = true;
-        for (int ch = 0; ch < nch; ++ch)
-          if (nb[ch] >= n_owned)
-            owned = false;
-        if (owned)
-        {
-          defer_slot[(size_t)n * nfaces + f] = n_defer++;
-          defer_list.push_back(n * 8 + f);
-        }
-      }
-    }
+  const int              nfaces = 2 * dim;
+  const std::vector<int> chunks = host_chunks(c, m);
+  const TableScan        scan = dim == 2 ? scan_table<2>(m, chunks) : scan_table<3>(m, chunks);
+  if (scan.rc != G5_OK)
+    return scan.rc;
+  // coarse/fine face records
+  const std::vector<int32_t> &reflux_slot = scan.reflux_slot, &defer_slot = scan.defer_slot;
+  const int                   n_reflux = scan.n_reflux, n_defer = (int)scan.defer_list.size();
 
   free_mesh(c);
   // work of the previous mesh may still run on another stream: the buffers
@@ -590,7 +674,7 @@ g5_set_mesh(G5Context * c, const G5Mesh * m)
   c->n_inst = n_inst;
   c->n_defer = n_defer;
   c->n_reflux = n_reflux;
-  if (plan_host_pipe(c, m, defer_slot, defer_list))
+  if (plan_host_pipe(c, m, chunks, scan))
   {
     free_mesh(c);
     return G5_ERR_CUDA;
@@ -651,14 +735,13 @@ g5_set_mesh(G5Context * c, const G5Mesh * m)
     // another level first (their gathers restrict or prolong, they publish or
     // defer coarse/fine records: they cost more), so that the last round of
     // the persistent grid holds cheap same-level blocks
-    std::vector<int32_t> order(n_owned), score(n_owned, 0);
+    std::vector<int32_t> order(n_owned), first(ns + 2, 0);
     for (int n = 0; n < n_owned; ++n)
-    {
-      order[n] = n;
-      for (int sl = 0; sl < ns; ++sl)
-        score[n] += m->nbr_rel[(size_t)n * ns + sl] != 0;
-    }
-    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return score[x] > score[y]; });
+      ++first[ns - scan.score[n] + 1];
+    for (int k = 0; k <= ns; ++k)
+      first[k + 1] += first[k];
+    for (int n = 0; n < n_owned; ++n)
+      order[first[ns - scan.score[n]]++] = n;
     if (n_owned > 0 && dev_upload(c, &c->d_walk, order.data(), order.size()))
     {
       free_mesh(c);
@@ -1155,6 +1238,38 @@ g5_refine_flags(G5Context * ctx,
            : G5_ERR_CUDA;
 }
 
+namespace
+{
+// stream-ordered device memory of one g5_remap call (freed with cudaFreeAsync);
+// under stream capture from the device's own pool, as allocation nodes
+cudaError_t
+remap_alloc(G5Context * c, void ** p, size_t bytes, cudaStream_t st)
+{
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+  {
+    cudaGetLastError();
+    return cudaMallocAsync(p, bytes, st);
+  }
+  if (!c->remap_pool)
+  {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c->device;
+    const cudaError_t e = cudaMemPoolCreate(&c->remap_pool, &props);
+    if (e != cudaSuccess)
+    {
+      c->remap_pool = nullptr;
+      return e;
+    }
+    uint64_t keep = UINT64_MAX;
+    cudaMemPoolSetAttribute(c->remap_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  return cudaMallocFromPoolAsync(p, bytes, c->remap_pool, st);
+}
+} // namespace
+
 extern "C" int
 g5_remap(G5Context * ctx, const G5Remap * r, const double * d_Uold, double * d_Unew, void * stream)
 {
@@ -1212,9 +1327,9 @@ g5_remap(G5Context * ctx, const G5Remap * r, const double * d_Uold, double * d_U
   int8_t *     d_kind = nullptr;
   int32_t *    d_src = nullptr;
   const size_t nk = (size_t)r->n_new, ns = (size_t)r->n_new * nch * sizeof(int32_t);
-  if (cudaMallocAsync((void **)&d_kind, nk, st) != cudaSuccess)
+  if (remap_alloc(ctx, (void **)&d_kind, nk, st) != cudaSuccess)
     return G5_ERR_CUDA;
-  if (cudaMallocAsync((void **)&d_src, ns, st) != cudaSuccess)
+  if (remap_alloc(ctx, (void **)&d_src, ns, st) != cudaSuccess)
   {
     cudaFreeAsync(d_kind, st);
     return G5_ERR_CUDA;
@@ -1231,7 +1346,7 @@ g5_remap(G5Context * ctx, const G5Remap * r, const double * d_Uold, double * d_U
   {
     int32_t *    d_rows = nullptr;
     const size_t nb = refine_rows.size() * sizeof(int32_t);
-    if (cudaMallocAsync((void **)&d_rows, nb, st) != cudaSuccess)
+    if (remap_alloc(ctx, (void **)&d_rows, nb, st) != cudaSuccess)
       return G5_ERR_CUDA;
     if (cudaMemcpyAsync(d_rows, refine_rows.data(), nb, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         g5::launch_remap_prolong(ctx->dim, ctx->b, ctx->prm.prolongation, d_Uold, d_Unew, dev_mesh(ctx), d_rows,

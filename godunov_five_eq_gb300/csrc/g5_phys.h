@@ -26,19 +26,13 @@ eos_params_valid(const G5Params * prm)
   return true;
 }
 
-// Block-table check shared by g5_set_mesh and g5_step_static (the reference
-// asserts the same facts in StencilHelper and its hashmap lookups): levels in
-// range, instance ids below n_inst, relation codes in {-1, 0, 1}, a valid
-// block for every coarser or same-level slot and for every child of a finer
-// slot that touches the block (the other children may be -1), outside blocks
-// mirroring owned ones.  Array presence is the caller's check.  Returns G5_OK
-// or G5_ERR_MESH.
+// Checks of a block table outside its neighbour rows: levels and instance ids
+// in range, outside blocks mirroring owned ones.  Returns G5_OK or G5_ERR_MESH.
 inline int
-validate_table(int dim, const G5Mesh * m)
+validate_blocks(const G5Mesh * m)
 {
   const int n_owned = m->n_owned, n_total = m->n_owned + m->n_outside;
   const int n_inst = m->n_inst > 0 ? m->n_inst : 1;
-  const int ns = dim == 2 ? 9 : 27, nch = dim == 2 ? 4 : 8, center = dim == 2 ? 4 : 13;
   for (int n = 0; n < n_total; ++n)
     if (m->level[n] < 0 || m->level[n] > 31)
       return G5_ERR_MESH;
@@ -46,6 +40,26 @@ validate_table(int dim, const G5Mesh * m)
     for (int n = 0; n < n_total; ++n)
       if (m->inst[n] < 0 || m->inst[n] >= n_inst)
         return G5_ERR_MESH;
+  for (int o = 0; o < m->n_outside; ++o)
+    if (m->out_src[o] < 0 || m->out_src[o] >= n_owned)
+      return G5_ERR_MESH;
+  return G5_OK;
+}
+
+// Block-table check of g5_step_static; g5_set_mesh makes the same one while it
+// reads the rows (scan_table in g5_capi.cu).  (The reference asserts the same
+// facts in StencilHelper and its hashmap lookups): validate_blocks, relation
+// codes in {-1, 0, 1}, a valid block for every coarser or same-level slot and
+// for every child of a finer slot that touches the block (the other children
+// may be -1).  Array presence is the caller's check.  Returns G5_OK or
+// G5_ERR_MESH.
+inline int
+validate_table(int dim, const G5Mesh * m)
+{
+  const int n_owned = m->n_owned, n_total = m->n_owned + m->n_outside;
+  const int ns = dim == 2 ? 9 : 27, nch = dim == 2 ? 4 : 8, center = dim == 2 ? 4 : 13;
+  if (validate_blocks(m) != G5_OK)
+    return G5_ERR_MESH;
   for (int n = 0; n < n_owned; ++n)
     for (int s = 0; s < ns; ++s)
     {
@@ -75,9 +89,6 @@ validate_table(int dim, const G5Mesh * m)
           return G5_ERR_MESH;
       }
     }
-  for (int o = 0; o < m->n_outside; ++o)
-    if (m->out_src[o] < 0 || m->out_src[o] >= n_owned)
-      return G5_ERR_MESH;
   return G5_OK;
 }
 
