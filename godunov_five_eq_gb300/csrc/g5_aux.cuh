@@ -391,39 +391,136 @@ refine_flags_kernel(const double * U,
   }
 }
 
-// a pair's indicator against both thresholds: bit 0 above eps_r, bit 1 below
-// eps_c (a call, so that no compare of it runs on the FP64 pipe otherwise)
-static __device__ __noinline__ int
-gradient_exact(double C, double N, double eps_r, double eps_c)
-{
-  const double ind = normalized_gradient(C, N);
-  return (ind > eps_r ? 1 : 0) | (ind < eps_c ? 2 : 0);
-}
-
 // The SIMPLE_GRADIENT indicator (normalized_gradient of every face pair of
 // both partial densities) without its divisions.  A block's flag needs only
-// whether its largest indicator exceeds eps_r and whether it is below eps_c,
-// so each pair is compared with both thresholds: its difference in FP64, the
-// comparisons with the products threshold x largest magnitude in FP32, and
-// the reference's rounded quotient only within 1e-5 of a threshold (or for
-// values a float does not hold).  Every interior pair is taken once, from a
-// shared-memory copy of the block.  One thread per cell.  The division form
-// was bound by the FP64 pipe (24 divisions per cell: 732 us for 2.0M cells).
+// its largest indicator, compared with eps_r and eps_c: it is found in FP32
+// (the differences in FP64, everything else on floats), and only a block
+// whose largest indicator lies within 1e-5 of a threshold, or that holds
+// values floats do not decide (infinities, NaN, magnitudes of 1e30 and more or
+// at the reference's 0.001), evaluates the reference's rounded quotients.
+// Every interior pair is taken once, from a shared-memory copy of the block.
+// One thread per cell.  2.0M cells: the division form was bound by the FP64
+// pipe (24 divisions per cell, 732 us), a form comparing every pair with both
+// thresholds by the ALU pipe (980 instructions per cell, 94 us).
+template <int DIM, int B>
+struct GradientTile
+{
+  static constexpr int NC = DIM == 2 ? B * B : B * B * B, NF = 2 * DIM, FC = NC / B;
+  double v[2][NC], h[2][NF * FC]; // the block, its face neighbours
+  float  vf[2][NC], hf[2][NF * FC];
+};
+
+// neighbor_same_level of both partial densities for a cell on the block's face
+template <int DIM, int B>
+__device__ __forceinline__ void
+halo_densities(const double * __restrict__ U, const DevMesh & m, int n, const int * cell, int dir, int side, double & h0, double & h1)
+{
+  using H = V<DIM>;
+  constexpr int NC = (DIM == 2) ? B * B : B * B * B;
+  constexpr int NS = (DIM == 2) ? 9 : 27, NCH = (DIM == 2) ? 4 : 8;
+  const int     s = NS / 2 + side * (dir == 0 ? 1 : (dir == 1 ? 3 : 9));
+  const int     rel = m.nbr_rel[n * NS + s];
+  const int *   nb = m.nbr + (n * NS + s) * NCH;
+  int           v[3] = { cell[0], cell[1], cell[2] };
+  v[dir] = side < 0 ? B - 1 : 0; // the same-level neighbour's cell
+  int c[3] = { v[0], v[1], v[2] }, src = nb[0];
+  if (rel < 0)
+  {
+#pragma unroll
+    for (int e = 0; e < DIM; ++e)
+      c[e] = ((m.coord[n * 3 + e] + (e == dir ? side : 0)) & 1) * (B / 2) + (v[e] >> 1);
+  }
+  else if (rel > 0)
+  {
+    int kid = 0;
+#pragma unroll
+    for (int e = 0; e < DIM; ++e)
+    {
+      const int k = v[e] >= B / 2 ? 1 : 0;
+      kid |= k << e;
+      c[e] = 2 * v[e] - k * B;
+    }
+    src = nb[kid];
+  }
+  const bool here = src < 0 || src >= m.n_owned; // outside the domain: the cell itself
+  const int  k = here ? cell[0] + B * (cell[1] + B * cell[2]) : c[0] + B * (c[1] + B * c[2]);
+  const double * p = U + (size_t)(here ? n : src) * H::NV * NC + k;
+  if (here || rel <= 0)
+  {
+    h0 = p[H::IAD0 * NC];
+    h1 = p[H::IAD1 * NC];
+    return;
+  }
+  h0 = 0.0;
+  h1 = 0.0;
+#pragma unroll
+  for (int o = 0; o < NCH; ++o)
+  {
+    const int off = (o & 1) + B * (((o >> 1) & 1) + B * (o >> 2));
+    h0 += p[H::IAD0 * NC + off];
+    h1 += p[H::IAD1 * NC + off];
+  }
+  h0 = h0 / NCH;
+  h1 = h1 / NCH;
+}
+
+// f(variable, own value's index, neighbour's index or -1 - halo index) over the
+// face pairs of one cell
+template <int DIM, int B, typename F>
+__device__ __forceinline__ void
+gradient_pairs(int tid, F f)
+{
+  constexpr int FC = GradientTile<DIM, B>::FC;
+  const int     cell[3] = { tid % B, (tid / B) % B, DIM == 3 ? tid / (B * B) : 0 };
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int d = 0; d < DIM; ++d)
+    {
+      const int o = d == 0 ? 1 : (d == 1 ? B : B * B);
+      const int p = d == 0 ? cell[1] + (DIM == 3 ? B * cell[2] : 0) : (d == 1 ? cell[0] + (DIM == 3 ? B * cell[2] : 0) : cell[0] + B * cell[1]);
+      f(t, cell[d] < B - 1 ? tid + o : -1 - ((2 * d + 1) * FC + p));
+      if (cell[d] == 0)
+        f(t, -1 - (2 * d * FC + p));
+    }
+}
+
+// the cell's pairs in the reference's arithmetic: bit 0 some indicator above
+// eps_r, bit 1 some not below eps_c
+template <int DIM, int B>
+__device__ __noinline__ int
+gradient_exact(const GradientTile<DIM, B> * g, int tid, double eps_r, double eps_c)
+{
+  int bits = 0;
+  gradient_pairs<DIM, B>(tid, [&](int t, int n) {
+    const double ind = normalized_gradient(g->v[t][tid], n >= 0 ? g->v[t][n] : g->h[t][-1 - n]);
+    bits |= (ind > eps_r ? 1 : 0) | (ind < eps_c ? 0 : 2);
+  });
+  return bits;
+}
+
 template <int DIM, int B>
 __global__ void __launch_bounds__(DIM == 2 ? B * B : B * B * B)
 gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, double eps_c, float rf, float cf, int lmin, int lmax, int8_t * flags)
 {
   using H = V<DIM>;
-  constexpr int NC = (DIM == 2) ? B * B : B * B * B, NF = 2 * DIM, FC = NC / B;
-  __shared__ double sC[2][NC], sH[2][NF * FC]; // the block, its face neighbours
-  const int         tid = threadIdx.x;
-  const int         cell[3] = { tid % B, (tid / B) % B, DIM == 3 ? tid / (B * B) : 0 };
-  for (int n = blockIdx.x; n < m.n_owned; n += gridDim.x)
+  using T = GradientTile<DIM, B>;
+  constexpr int NC = T::NC, NF = T::NF, FC = T::FC;
+  __shared__ T        g;
+  __shared__ unsigned sMax[2]; // largest indicator (float bits; all ones: undecided) of this and the next block
+  const int           tid = threadIdx.x;
+  if (tid < 2)
+    sMax[tid] = 0u;
+  int par = 0;
+  for (int n = blockIdx.x; n < m.n_owned; n += gridDim.x, par ^= 1)
   {
     const int      lev = m.level[n];
     const double * base = U + (size_t)n * H::NV * NC;
-    sC[0][tid] = base[H::IAD0 * NC + tid];
-    sC[1][tid] = base[H::IAD1 * NC + tid];
+    const double   v0 = base[H::IAD0 * NC + tid], v1 = base[H::IAD1 * NC + tid];
+    g.v[0][tid] = v0;
+    g.v[1][tid] = v1;
+    g.vf[0][tid] = fabsf(d2f_nan(v0));
+    g.vf[1][tid] = fabsf(d2f_nan(v1));
     for (int h = tid; h < NF * FC; h += NC)
     {
       const int f = h / FC, p = h % FC, dir = f >> 1;
@@ -433,60 +530,47 @@ gradient_flags_kernel(const double * __restrict__ U, DevMesh m, double eps_r, do
       hc[e1] = p % B;
       if (DIM == 3)
         hc[e2] = p / B;
-      sH[0][h] = neighbor_same_level<DIM, B>(U, m, n, hc, dir, (f & 1) ? 1 : -1, H::IAD0);
-      sH[1][h] = neighbor_same_level<DIM, B>(U, m, n, hc, dir, (f & 1) ? 1 : -1, H::IAD1);
+      double h0, h1;
+      halo_densities<DIM, B>(U, m, n, hc, dir, (f & 1) ? 1 : -1, h0, h1);
+      g.h[0][h] = h0;
+      g.h[1][h] = h1;
+      g.hf[0][h] = fabsf(d2f_nan(h0));
+      g.hf[1][h] = fabsf(d2f_nan(h1));
     }
     __syncthreads();
-    // (rf, cf: the thresholds as floats; at 1 and more they decide without the cells)
-    const bool want_r = lev < lmax && bits64(eps_r) < bits64(1.0), want_c = lev > lmin && bits64(eps_c) <= bits64(1.0);
-    const bool c_pos = bits64(eps_c) > 0;
-    bool       above = false, below = true; // some indicator > eps_r; all < eps_c
-    if (want_r || want_c)
+    float qmax = 0.0f;
+    bool  plain = true;
+    gradient_pairs<DIM, B>(tid, [&](int t, int k) {
+      const double N = k >= 0 ? g.v[t][k] : g.h[t][-1 - k];
+      const float  vmax = fmaxf(g.vf[t][tid], k >= 0 ? g.vf[t][k] : g.hf[t][-1 - k]);
+      const float  q = __fdividef(fabsf(d2f_fast(g.v[t][tid] - N)), vmax);
+      // (a NaN drops out of fmaxf: the sum below keeps it)
+      plain = plain && (g.vf[t][tid] + vmax) < 1e30f && fabsf(vmax - 0.001f) > 1e-8f && (k >= 0 ? g.vf[t][k] : g.hf[t][-1 - k]) < 1e30f;
+      qmax = fmaxf(qmax, vmax < 0.001f ? 0.0f : q);
+    });
+    const unsigned w = __reduce_max_sync(0xffffffffu, plain ? __float_as_uint(qmax) : 0xffffffffu);
+    if ((tid & 31) == 0)
+      atomicMax(&sMax[par], w);
+    __syncthreads();
+    const unsigned top = sMax[par];
+    const float    q = __uint_as_float(top);
+    // thresholds of 1 and more decide without the cells (the indicator is at
+    // most 1); the others when q is not within 1e-5 of them
+    const bool want_r = bits64(eps_r) < bits64(1.0), want_c = bits64(eps_c) <= bits64(1.0);
+    bool       above = want_r && q > rf, below = !want_c || q < cf || (q == 0.0f && bits64(eps_c) > 0);
+    const bool near = top == 0xffffffffu || (want_r && fabsf(q - rf) <= 1e-5f * rf && q != 0.0f) || (want_c && fabsf(q - cf) <= 1e-5f * cf && q != 0.0f);
+    if (near)
     {
-      auto pair = [&](double C, double N) {
-        const double             diff = C - N;
-        const unsigned long long ac = (unsigned long long)bits64(C) << 1, an = (unsigned long long)bits64(N) << 1;
-        const double             vmax = __longlong_as_double((long long)((ac > an ? ac : an) >> 1));
-        const float              df = fabsf(d2f_fast(diff)), vf = d2f_fast(vmax);
-        // (an exponent a float does not hold, infinities and NaN: undecided)
-        const bool  wide = (x64_hi(vmax) & 0x7FF00000u) >= (1100u << 20);
-        bool        undecided = wide || fabsf(vf - 0.001f) <= 1e-8f;
-        const bool  small = vf < 0.001f; // the reference's 0
-        const float r = small ? 0.0f : df;
-        const float tr = rf * vf, tc = cf * vf;
-        bool        gt = want_r && !small && r > tr;
-        bool        lt = want_c ? (small ? c_pos : r < tc) : true;
-        undecided = undecided || (!small && ((want_r && fabsf(r - tr) <= 1e-5f * fabsf(tr)) || (want_c && fabsf(r - tc) <= 1e-5f * fabsf(tc))));
-        if (undecided)
-        {
-          const int x = gradient_exact(C, N, eps_r, eps_c);
-          gt = want_r && (x & 1);
-          lt = !want_c || (x & 2);
-        }
-        above = above || gt;
-        below = below && lt;
-      };
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-      {
-        const double C = sC[t][tid];
-#pragma unroll
-        for (int d = 0; d < DIM; ++d)
-        {
-          const int o = d == 0 ? 1 : (d == 1 ? B : B * B);
-          const int p = d == 0 ? cell[1] + (DIM == 3 ? B * cell[2] : 0) : (d == 1 ? cell[0] + (DIM == 3 ? B * cell[2] : 0) : cell[0] + B * cell[1]);
-          pair(C, cell[d] < B - 1 ? sC[t][tid + o] : sH[t][(2 * d + 1) * FC + p]);
-          if (cell[d] == 0)
-            pair(C, sH[t][2 * d * FC + p]);
-        }
-      }
+      const int x = gradient_exact<DIM, B>(&g, tid, eps_r, eps_c);
+      above = __syncthreads_or(x & 1) != 0;
+      below = __syncthreads_or(x & 2) == 0;
     }
-    const int any_above = __syncthreads_or(above), any_not = __syncthreads_or(!below);
     if (tid == 0)
     {
-      const bool coarsen = lev > lmin && !any_not; // (eps_c > 1: every indicator is below)
-      flags[n] = (int8_t)(lev < lmax && any_above ? 2 : (coarsen ? 0 : 1));
+      flags[n] = (int8_t)(lev < lmax && above ? 2 : (lev > lmin && below ? 0 : 1));
+      sMax[par ^ 1] = 0u; // (last read before the barrier above)
     }
+    __syncthreads();
   }
 }
 
