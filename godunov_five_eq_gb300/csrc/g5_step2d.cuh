@@ -29,7 +29,10 @@ struct Step2DTraits
   // round and the 544 (144) faces two, at 96 registers (16x16: 420 us per
   // shock-bubble step of 486k cells against 444 us with 256 threads at 128
   // registers, 438 us with 384 at 80; 8x8: 147 us against 161 with 64 threads)
-  static constexpr int NT = MIXED ? B * B : (B == 16 ? 320 : 96);
+  // FP32-bulk: a thread per cell of a 16x16 block (288, 320 or 544 threads are
+  // 8 % and more slower), two per cell of an 8x8 block (32-block shock tube 10.1
+  // -> 9.1 us, 122k-cell AMR shock-bubble 34.6 -> 31.0 us per step)
+  static constexpr int NT = MIXED ? (B == 16 ? 256 : 128) : (B == 16 ? 320 : 96);
   static constexpr int CTAS = MIXED ? (B == 16 ? 4 : 8) : (B == 16 ? 2 : 7);
   static constexpr int G = B + 4;  // ghosted extent
   static constexpr int S = B + 2;  // ring extent
@@ -847,9 +850,10 @@ apply_mixed_2d(const double * uin, double * u2, const float (&h)[2][5], const fl
   }
   // renormalisation
   const double sa = u2[H::IA0] + u2[H::IA1];
-  const double d = sa - 1.0;
-  if (d != 0.0)
+  // (a compare of bits: an FP64 compare per cell is 1 to 2 % of the step)
+  if (__double_as_longlong(sa) != __double_as_longlong(1.0))
   {
+    const double d = sa - 1.0;
     if ((__double_as_longlong(d) & 0x7FFFFFFFFFFFFFFFLL) < __double_as_longlong(1e-8))
     {
       u2[H::IA0] = fma(-u2[H::IA0], d, u2[H::IA0]);

@@ -618,9 +618,10 @@ apply_mixed_3d(double * u2, const float (&hh)[3][2], const float (&ll)[3][2], co
     u2[ive[e]] += ff_to_d(s, t);
   }
   const double sa = u2[H::IA0] + u2[H::IA1];
-  const double d = sa - 1.0;
-  if (d != 0.0)
+  // (a compare of bits: an FP64 compare per cell is 1 to 2 % of the step)
+  if (__double_as_longlong(sa) != __double_as_longlong(1.0))
   {
+    const double d = sa - 1.0;
     if ((__double_as_longlong(d) & 0x7FFFFFFFFFFFFFFFLL) < __double_as_longlong(1e-8))
     {
       u2[H::IA0] = fma(-u2[H::IA0], d, u2[H::IA0]);
