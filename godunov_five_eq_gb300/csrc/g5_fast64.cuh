@@ -212,13 +212,12 @@ prim_fast64(const double * u, double * q, const PhysParams & P, bool & bad)
   return 0.0;
 }
 
-// slope_scalar<double> for slope_type 1 (minmod) and 2.  The product of the
-// one-sided differences, whose sign decides, is not formed: when it could
+// slope_scalar<double> for slope_type 1 (minmod) and 2, from the one-sided
+// differences l and r.  Their product, whose sign decides, is not formed: when it could
 // underflow (the reference takes that as no slope) the cell is `bad`.
 __device__ __forceinline__ double
-slope_fast64(double q, double qPlus, double qMinus, int st, bool & bad)
+limit_fast64(double l, double r, double qPlus, double qMinus, int st, bool & bad)
 {
-  const double   l = q - qMinus, r = qPlus - q;
   const uint32_t hl = x64_hi(l), hr = x64_hi(r);
   const uint32_t el = hl & 0x7FF00000u, er = hr & 0x7FF00000u;
   const bool     same = (int)(hl ^ hr) >= 0 && el != 0u && er != 0u;
@@ -236,6 +235,12 @@ slope_fast64(double q, double qPlus, double qMinus, int st, bool & bad)
   }
   // no slope: a zero with the sign of the central difference
   return same ? m : x64_make(order64(qPlus) >= order64(qMinus) ? 0u : 0x80000000u, 0u);
+}
+
+__device__ __forceinline__ double
+slope_fast64(double q, double qPlus, double qMinus, int st, bool & bad)
+{
+  return limit_fast64(q - qMinus, qPlus - q, qPlus, qMinus, st, bad);
 }
 
 // HLLC (hllc_fp64) of two reconstructed states, scaled by dt/dx; S the
@@ -417,21 +422,6 @@ prim_ref64(State64<DIM> u, const PhysParams * P, double * sQ, int stride)
   prim_fp64<DIM>(u.v, q, *P);
   for (int k = 0; k < V<DIM>::NQ; ++k)
     sQ[k * stride] = q[k];
-}
-
-// THINC value of the volume fraction at the cell's face
-// (scheme/ComputeFluxesAndStoreTHINCFunctor.cpp:122-283): a0 the cell's value,
-// aM and aP its neighbours' along the direction, nd the Youngs normal's
-// component, bs = +-1 the side
-__device__ __forceinline__ double
-thinc_alpha64(double a0, double aM, double aP, double nd, double bs, double thinc_beta)
-{
-  const double beta = thinc_beta * nd + 0.01;
-  const double Aa = (aP + aM) / 2.0;
-  const double Bb = (aP - aM) / 2.0;
-  const double C = tanh_d(0.5 * beta);
-  const double D = tanh_d(0.5 * beta * (a0 - Aa) / Bb);
-  return Aa + bs * Bb * (C + bs * D / C) / (1.0 + bs * D);
 }
 
 // ---------------------------------------------------------------------------

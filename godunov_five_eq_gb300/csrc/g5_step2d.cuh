@@ -16,7 +16,6 @@
 #pragma once
 
 #include "g5_common.cuh"
-#include "g5_fast64.cuh"
 
 namespace g5
 {
@@ -25,27 +24,17 @@ template <int B, bool MIXED>
 struct Step2DTraits
 {
   using R = typename std::conditional<MIXED, float, double>::type;
-  // FP64: more threads than cells, so that the 320 (96) slope cells take one
-  // round and the 544 (144) faces two, at 96 registers (16x16: 420 us per
-  // shock-bubble step of 486k cells against 444 us with 256 threads at 128
-  // registers, 438 us with 384 at 80; 8x8: 147 us against 161 with 64 threads)
   // FP32-bulk: a thread per cell of a 16x16 block (288, 320 or 544 threads are
   // 8 % and more slower), two per cell of an 8x8 block (32-block shock tube 10.1
   // -> 9.1 us, 122k-cell AMR shock-bubble 34.6 -> 31.0 us per step)
-  static constexpr int NT = MIXED ? (B == 16 ? 256 : 128) : (B == 16 ? 320 : 96);
-  static constexpr int CTAS = MIXED ? (B == 16 ? 4 : 8) : (B == 16 ? 2 : 7);
+  static constexpr int NT = MIXED && B == 8 ? 128 : B * B;
+  static constexpr int CTAS = MIXED ? (B == 16 ? 4 : 8) : (B == 16 ? 2 : 8);
   static constexpr int G = B + 4;  // ghosted extent
   static constexpr int S = B + 2;  // ring extent
   static constexpr int NQ = 6;     // r0 r1 p u v a0
-  // dqx[5] dqy[5] hS[5] (the THINC normal is evaluated on demand); FP64: and
-  // the mixture's S of the cell
-  static constexpr int NREC = MIXED ? 15 : 16;
+  static constexpr int NREC = 15;  // dqx[5] dqy[5] hS[5] (the THINC normal is evaluated on demand)
   static constexpr int NFF = B * (B + 1);
-  // FP64: THINC face values of the 2 B (B + 2) cells and directions, right and
-  // left, and the list of those that have one
-  static constexpr int NTH = MIXED ? 0 : 2 * B * (B + 2);
   static constexpr size_t smem_bytes = sizeof(R) * (size_t)(NQ * G * G + NREC * S * S + 2 * 8 * NFF) + 64;
-  static constexpr size_t smem_thinc = (2 * sizeof(double) + sizeof(short)) * (size_t)NTH; // (more, with THINC)
 };
 
 // halo cell h (0 .. G*G - B*B - 1) -> ghosted coordinates
@@ -156,15 +145,12 @@ gather_ghost_2d(const StepArgs & a, int n, int cx0, int cy0, int gx, int gy, dou
   return true;
 }
 
-// the primitives of a cell into the ghosted arrays.  STIFF: the equation of
-// state of step2d_kernel.  Returns whether the values leave the range of the
-// fast FP64 form (the block then takes the reference arithmetic).
-template <int B, bool MIXED, int STIFF>
-__device__ __forceinline__ bool
+// the primitives of a cell into the ghosted arrays
+template <int B, bool MIXED>
+__device__ __forceinline__ void
 store_prim(typename Step2DTraits<B, MIXED>::R * sQ, int gidx, const double * u, const PhysParams & P, int eosk)
 {
   constexpr int GG = (B + 4) * (B + 4);
-  bool          bad = false;
   if constexpr (MIXED)
   {
     float q[6];
@@ -176,24 +162,11 @@ store_prim(typename Step2DTraits<B, MIXED>::R * sQ, int gidx, const double * u, 
   else
   {
     double q[6];
-    if constexpr (STIFF == 2)
-      prim_fp64<2>(u, q, P);
-    else
-      prim_fast64<2, false, true, STIFF == 1>(u, q, P, bad);
-    if (bad)
-    {
-      State64<2> s;
-#pragma unroll
-      for (int v = 0; v < 8; ++v)
-        s.v[v] = u[v];
-      prim_ref64<2>(s, &P, sQ + gidx, GG);
-      return true;
-    }
+    prim_fp64<2>(u, q, P);
 #pragma unroll
     for (int k = 0; k < 6; ++k)
       sQ[k * GG + gidx] = q[k];
   }
-  return bad;
 }
 
 // Youngs normal (restated: (1,2,1)-weighted central differences), |n_x|, |n_y|
@@ -208,6 +181,21 @@ youngs_abs_2d(const R * A, int gi, R & nx, R & ny)
   nrm = sqrt(nrm);
   nx = (nrm > R(0)) ? fabs(-gx / nrm) : R(0);
   ny = (nrm > R(0)) ? fabs(-gy / nrm) : R(0);
+}
+
+// THINC value of the volume fraction at the cell's face
+// (scheme/ComputeFluxesAndStoreTHINCFunctor.cpp:122-283): a0 the cell's value,
+// aM and aP its neighbours' along the direction, nd the Youngs normal's
+// component, bs = +-1 the side
+__device__ __forceinline__ double
+thinc_alpha64(double a0, double aM, double aP, double nd, double bs, double thinc_beta)
+{
+  const double beta = thinc_beta * nd + 0.01;
+  const double Aa = (aP + aM) / 2.0;
+  const double Bb = (aP - aM) / 2.0;
+  const double C = tanh_d(0.5 * beta);
+  const double D = tanh_d(0.5 * beta * (a0 - Aa) / Bb);
+  return Aa + bs * Bb * (C + bs * D / C) / (1.0 + bs * D);
 }
 
 // FP64: reconstruct one side of a face from cell (ci, cj) (ghosted-ring
@@ -321,115 +309,6 @@ face_flux_ref64(const double * sQ, const double * sRec, double * sF, int dir, in
     sF[k * NFF + ff] = fl[k] * dtdx;
 }
 
-template <int B>
-__device__ __noinline__ void
-face_flux_cold64(const double * sQ, const double * sRec, double * sF, int dir, int ff, double dtdx, const PhysParams * P)
-{
-  face_flux_ref64<B>(sQ, sRec, sF, dir, ff, dtdx, *P);
-}
-
-// FP64: the THINC entry (cell, direction) in the arrays sAF: 2 directions of
-// B (B + 2) cells
-template <int B>
-__device__ __forceinline__ int
-thinc_index(int dir, int ci, int cj)
-{
-  return dir == 0 ? (ci + 1) + (B + 2) * cj : B * (B + 2) + ci + B * (cj + 1);
-}
-
-// the pair's face values, from its entry
-template <int B>
-__device__ __forceinline__ bool
-thinc_eval2(const double * sQ, double * sAF, int i, const PhysParams & P)
-{
-  using T = Step2DTraits<B, false>;
-  constexpr int  G = T::G, GG = G * G;
-  const int      dir = i < B * (B + 2) ? 0 : 1, k = i - dir * B * (B + 2);
-  const int      ci = dir == 0 ? k % (B + 2) - 1 : k % B, cj = dir == 0 ? k / (B + 2) : k / B - 1;
-  const double * A = sQ + 5 * GG + (ci + 2) + G * (cj + 2);
-  // (1, 2, 1)-weighted central differences (youngs_abs_2d)
-  const double gx = (__fma_rn(2.0, A[1], A[1 - G]) + A[1 + G]) - (__fma_rn(2.0, A[-1], A[-1 - G]) + A[-1 + G]);
-  const double gy = (__fma_rn(2.0, A[G], A[G - 1]) + A[G + 1]) - (__fma_rn(2.0, A[-G], A[-G - 1]) + A[-G + 1]);
-  bool         bad = false;
-  const double nd = youngs_ratio64(dir == 0 ? gx : gy, gx * gx + gy * gy, bad);
-  const int    o = dir == 0 ? 1 : G;
-  thinc_pair64(A[0], A[-o], A[o], nd, P, sAF[i], sAF[T::NTH + i], bad);
-  return bad;
-}
-
-// FP64: the reconstructed state and the mixture's S of one side (the values
-// of face_state_ref64, normal velocity first).  The direction is a run-time
-// value: X and Y faces share one copy of the flux code, which is long enough
-// to miss the instruction cache.
-template <int B>
-__device__ __forceinline__ double
-face_state_fast64(const double * sQ, const double * sRec, const double * sAF, int ci, int cj, int dir, int side, const PhysParams & P, double * q,
-                  bool & bad)
-{
-  using T = Step2DTraits<B, false>;
-  constexpr int    G = T::G, S = T::S, GG = G * G, SS = S * S;
-  const double     off = side > 0 ? 0.5 : -0.5;
-  const int        gi = (ci + 2) + G * (cj + 2);
-  const int        si = (ci + 1) + S * (cj + 1);
-  const double *   dq = sRec + dir * 5 * SS + si;
-  const bool       hancock = P.integrator == 0;
-#pragma unroll
-  for (int k = 0; k < 5; ++k)
-  {
-    const int    from = k < 3 ? k : (k == 3 ? 3 + dir : 4 - dir);
-    const double t = __fma_rn(off, dq[from * SS], sQ[from * GG + gi]);
-    q[k] = hancock ? __fma_rn(0.5, sRec[(10 + from) * SS + si], t) : t;
-  }
-  const double a0 = sQ[5 * GG + gi];
-  double       Sm = sRec[15 * SS + si];
-  q[5] = a0;
-  if (P.thinc)
-  {
-    const double af = sAF[(side > 0 ? 0 : T::NTH) + thinc_index<B>(dir, ci, cj)];
-    if (bits64(af) != bits64(thinc_none64()))
-    {
-      const ThincSide64 t = thinc_side64(a0, af, sQ[gi], sQ[GG + gi], hancock ? sRec[10 * SS + si] : 0.0, hancock ? sRec[11 * SS + si] : 0.0, &P);
-      q[0] = t.q0;
-      q[1] = t.q1;
-      q[5] = af;
-      Sm = t.S;
-      bad = bad || t.bad;
-    }
-  }
-  else
-  {
-    q[0] = max_pos64(q[0], P.smallr);
-    q[1] = max_pos64(q[1], P.smallr);
-  }
-  return Sm;
-}
-
-template <int B, bool MG>
-__device__ __forceinline__ bool
-face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, double * sF, int dir, int ff, double dtdx, const PhysParams & P)
-{
-  using H = V<2>;
-  constexpr int NFF = B * (B + 1);
-  int           li, lj, ri, rj;
-  face_cells<B>(dir, ff, li, lj, ri, rj);
-  double       qL[6], qR[6], fl[8];
-  bool         bad = false;
-  const double Sl = face_state_fast64<B>(sQ, sRec, sAF, li, lj, dir, 1, P, qL, bad);
-  const double Sr = face_state_fast64<B>(sQ, sRec, sAF, ri, rj, dir, -1, P, qR, bad);
-  const Side64 L = hllc_side64<2, MG>(qL, Sl, P, bad);
-  const Side64 R = hllc_side64<2, MG>(qR, Sr, P, bad);
-  hllc_fast64<2>(qL, qR, L, R, dtdx, fl, bad);
-  if (bad)
-  {
-    face_flux_cold64<B>(sQ, sRec, sF, dir, ff, dtdx, &P);
-    return true;
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    sF[(k == H::FU ? H::FU + dir : k == H::FV ? H::FV - dir : k) * NFF + ff] = fl[k];
-  return false;
-}
-
 // FP64: limited slopes, Hancock source (ComputeFluxesAndStoreFunctor.cpp:
 // 174-199, without its factor 1/2) of ring cell r, in the reference's
 // arithmetic
@@ -462,89 +341,6 @@ hancock_ref64(const double * sQ, double * sRec, int gi, int r, double dtdx, cons
   sRec[12 * SS + r] = (-u * dx[2] - dx[3] * rr * c * c) * dtdx + (-v * dy[2] - dy[4] * rr * c * c) * dtdx;
   sRec[13 * SS + r] = (-u * dx[3] - dx[2] / rr) * dtdx + (-v * dy[3]) * dtdx;
   sRec[14 * SS + r] = (-u * dx[4]) * dtdx + (-v * dy[4] - dy[2] / rr) * dtdx;
-}
-
-template <int B>
-__device__ __noinline__ void
-hancock_cold64(const double * sQ, double * sRec, int gi, int r, double dtdx, const PhysParams * P)
-{
-  hancock_ref64<B>(sQ, sRec, gi, r, dtdx, *P);
-}
-
-// the same values from the fast operations, and the mixture's S of the cell
-template <int B, bool MG>
-__device__ __forceinline__ bool
-hancock_fast64(const double * sQ, double * sRec, int gi, int r, double dtdx, const PhysParams & P)
-{
-  using T = Step2DTraits<B, false>;
-  constexpr int G = T::G, S = T::S, GG = G * G, SS = S * S;
-  const bool    stiff = mixture_stiff64<MG>(P), hancock = P.integrator == 0;
-  const int     st = P.st64;
-  bool          bad = false;
-  const double  a0 = sQ[5 * GG + gi], a1 = 1.0 - a0;
-  const Mix64   m = mixture64<MG>(P, a0, a1, sQ[gi], sQ[GG + gi], bad);
-  sRec[15 * SS + r] = m.S;
-  const double rr = sQ[gi] + sQ[GG + gi];
-  Recip64      rd = {};
-  double       c = 0.0;
-  if (hancock)
-  {
-    rd = recip64(rr, bad);
-    c = sound64(rr, sQ[2 * GG + gi], m, stiff, bad);
-  }
-  // each source is a sum over the two directions, x first; the sums of the
-  // normal and transverse velocity change places between them.  (Rolled, as
-  // the update's directions are: the instruction cache gains more than the
-  // loop costs, 471 -> 461 us with THINC, 386 us without either way.)
-  double sr = 0.0, sp = 0.0, sv[2] = { 0.0, 0.0 };
-#pragma unroll 1
-  for (int e = 0; e < 2; ++e)
-  {
-    const int o = e == 0 ? 1 : G;
-    double    d[5]; // r0 r1 p, normal and transverse velocity
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-    {
-      const int      from = k < 3 ? k : (k == 3 ? 3 + e : 4 - e);
-      const double * Qk = sQ + from * GG + gi;
-      d[k] = st != 0 ? slope_fast64(Qk[0], Qk[o], Qk[-o], st, bad) : 0.0;
-      sRec[(5 * e + from) * SS + r] = d[k];
-    }
-    if (hancock)
-    {
-      const double mu = neg64(sQ[(3 + e) * GG + gi]);
-      const double dr = mul64(d[3], rr, bad);
-      const double tr = mul64(mulh64(mu, d[0] + d[1], bad) - dr, dtdx, bad);
-      const double tp = mul64(mulh64(mu, d[2], bad) - mulh64(mul64(dr, c, bad), c, bad), dtdx, bad);
-      const double tn = mul64(mulh64(mu, d[3], bad) - quot64(d[2], rd, bad), dtdx, bad);
-      const double tt = mul64(mulh64(mu, d[4], bad), dtdx, bad);
-      if (e == 0)
-      {
-        sr = tr;
-        sp = tp;
-        sv[0] = tn;
-        sv[1] = tt;
-      }
-      else
-      {
-        sr = sr + tr;
-        sp = sp + tp;
-        sv[0] = sv[0] + tt;
-        sv[1] = sv[1] + tn;
-      }
-    }
-  }
-  if (hancock)
-  {
-    sRec[10 * SS + r] = mul64(sr, a0, bad);
-    sRec[11 * SS + r] = mulh64(sr, a1, bad);
-    sRec[12 * SS + r] = sp;
-    sRec[13 * SS + r] = sv[0];
-    sRec[14 * SS + r] = sv[1];
-  }
-  if (bad)
-    hancock_cold64<B>(sQ, sRec, gi, r, dtdx, &P);
-  return bad;
 }
 
 // The FP32-bulk form's state of one face side, the direction known at compile time:
@@ -715,53 +511,6 @@ update_fp64(const double * uin, double * u2, const double * sFx, const double * 
   double       q[6];
   const double c = prim_fp64<2>(u2, q, P);
   return (c + fabs(q[H::QU])) / dx + (c + fabs(q[H::QV])) / dx;
-}
-
-// FP64 cold path: the update of a cell whose values leave the fast form's
-// range, written to U2 (out, variables NC apart)
-template <int B>
-__device__ __noinline__ double
-update_cold64(State64<2> uin, double * out, const double * sFx, const double * sFy, int ci, int cj, double dx, const PhysParams * P, bool want_dt)
-{
-  double       u2[V<2>::NV];
-  const double r = update_fp64<B>(uin.v, u2, sFx, sFy, ci, cj, dx, *P, want_dt);
-  for (int v = 0; v < V<2>::NV; ++v)
-    out[v * B * B] = u2[v];
-  return r;
-}
-
-// update_fp64 from the fast operations.  (The reference
-// starts each sum from 0 + F_left: the same value but for the sign of a zero.)
-template <int B, bool MG>
-__device__ __forceinline__ double
-update_fast64(const double * uin, double * u2, const double * sFx, const double * sFy, int ci, int cj, double dx, const PhysParams & P, bool want_dt,
-              bool & bad)
-{
-  using H = V<2>;
-  constexpr int NFF = B * (B + 1);
-#pragma unroll
-  for (int v = 0; v < H::NV; ++v)
-    u2[v] = uin[v];
-  double     st0, st1;
-  const bool mp = P.source_term == 1;
-  source_factors_fast64<2, MG>(uin, P, st0, st1, bad);
-  bad = bad || x64_raw_bad(uin[H::IA1]); // (the rest was tested for the primitives)
-#pragma unroll 1
-  for (int dir = 0; dir < 2; ++dir)
-  {
-    const double * F = dir == 0 ? sFx : sFy;
-    const int      il = dir == 0 ? ci + (B + 1) * cj : ci + B * cj;
-    const int      ir = dir == 0 ? il + 1 : il + B;
-    const double   usl = F[H::FUS * NFF + il], usr = F[H::FUS * NFF + ir];
-    u2[H::IAD0] = clamp_r64(u2[H::IAD0] + (F[H::FR0 * NFF + il] - F[H::FR0 * NFF + ir]));
-    u2[H::IAD1] = clamp_r64(u2[H::IAD1] + (F[H::FR1 * NFF + il] - F[H::FR1 * NFF + ir]));
-    u2[H::IA0] = clamp_a64(u2[H::IA0] + alpha_inc64(F[H::FA0 * NFF + il], F[H::FA0 * NFF + ir], usl, usr, st0, uin[H::IA0], mp, bad));
-    u2[H::IA1] = clamp_a64(u2[H::IA1] + alpha_inc64(F[H::FA1 * NFF + il], F[H::FA1 * NFF + ir], usl, usr, st1, uin[H::IA1], mp, bad));
-    u2[H::IE] += F[H::FE * NFF + il] - F[H::FE * NFF + ir];
-    u2[H::IU] += F[H::FU * NFF + il] - F[H::FU * NFF + ir];
-    u2[H::IV] += F[H::FV * NFF + il] - F[H::FV * NFF + ir];
-  }
-  return finish_fast64<2, MG>(u2, dx, P, want_dt, bad);
 }
 
 // The same update in the FP32-bulk form.  FP64 is used only for the adds
@@ -947,14 +696,12 @@ finish_deferred_2d(const StepArgs & a, int j)
 }
 
 // 4 CTAs per SM in the FP32-bulk form (64 registers), so that CTAs in the
-// FP64-heavy update overlap with CTAs in the FP32 face phase; 2 CTAs per SM
-// (96 registers) in the FP64 form
+// FP64-heavy update overlap with CTAs in the FP32 face phase.
 // THINC, STIFF: the FP32-bulk form is compiled with and without the THINC
 // reconstruction and the stiffened-gas pressure path (P picks the kernel), so
-// a kernel carries only the code its case runs; the FP64 form tests THINC at
-// run time and has STIFF = 0 and 1 (the fast form of g5_fast64.cuh: stiffened
-// gases, Mie-Grueneisen laws) and 2 (the reference arithmetic: constants
-// outside the fast form's range).  FUSED: the FP32-bulk form finishing the coarse/fine
+// a kernel carries only the code its case runs; the FP64 form is the reference
+// arithmetic and tests both at run time (STIFF = -1; g5_step2d_f64.cuh holds
+// the kernel that all but its odd cases take).  FUSED: the FP32-bulk form finishing the coarse/fine
 // records in its tail (m.fin_tgt set; the kernel without it keeps the plain
 // block loop)
 template <int B, bool MIXED, bool THINC = false, int STIFF = -1, bool FUSED = false>
@@ -972,9 +719,6 @@ step2d_kernel(const __grid_constant__ StepArgs a)
   R *          sRec = sQ + T::NQ * GG;
   R *          sFx = sRec + T::NREC * SS; // [8][NFF]  X faces (B+1) x B
   R *          sFy = sFx + 8 * NFF;       // [8][NFF]  Y faces B x (B+1)
-  R *          sAF = sFy + 8 * NFF;       // FP64: THINC face values, then the list
-  short *      sList = reinterpret_cast<short *>(sAF + 2 * T::NTH);
-  __shared__ int sThinc; // FP64: entries of the list
   using DtT = typename std::conditional<MIXED, float, double>::type;
   __shared__ DtT sRed[NT / 32];
   __shared__ int sSlot[10]; // the block's reflux slots (faces 0-3), its defer slots, its outside-twin range
@@ -997,9 +741,6 @@ step2d_kernel(const __grid_constant__ StepArgs a)
   // thread's device-scope fence and atomic; acquire: that thread's fence
   // after the atomic, then the barrier.
   constexpr bool fused = MIXED && FUSED;
-  constexpr bool fast64 = !MIXED && STIFF != 2;
-  if (fast64 && tid == 0)
-    sThinc = 0;
   for (int iw = blockIdx.x;;)
   {
     int next = iw;
@@ -1026,19 +767,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       if constexpr (MIXED)
         dtdx_r = d2f_fast(a.dt[ins]) * __frcp_rn(d2f_fast(dx));
       else
-        dtdx_r = a.dt[ins];
-      // FP64 fast form: a value of the block left its range (per thread until
-      // the next barrier, then for the whole CTA: the phases that follow take
-      // the reference arithmetic)
-      bool cold = false;
-      if constexpr (fast64)
-      {
-        cold = x64_raw_bad(dtdx_r) || x64_raw_bad(dx);
-        const double q = div64(dtdx_r, dx, cold);
-        dtdx_r = cold ? div_cold64(dtdx_r, dx) : q;
-      }
-      else if constexpr (!MIXED)
-        dtdx_r = dtdx_r / dx;
+        dtdx_r = a.dt[ins] / dx;
 
       // ---------------- phase 1: own cell (coalesced) + halo gather -> primitives
       // (the own cell's loads are in flight while the halo gather runs; its
@@ -1055,40 +784,6 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         for (int v = 0; v < H::NV; ++v)
           uin[v] = base[v * NC];
       }
-      if constexpr (fast64)
-      {
-        // (one copy of the conversion for the own cell and the halo)
-        for (int it = owner ? -1 : 0, h = owner ? tid + NT - NC : tid - NC; it < 0 || h < NHALO; ++it)
-        {
-          double u[H::NV];
-          int    gidx;
-          if (it < 0)
-          {
-            gidx = (ci + 2) + G * (cj + 2);
-#pragma unroll
-            for (int v = 0; v < H::NV; ++v)
-              u[v] = uin[v];
-          }
-          else
-          {
-            int gx, gy;
-            halo_coords<B>(h, gx, gy);
-            gidx = (gx + 2) + G * (gy + 2);
-            if (!gather_ghost_2d<B>(a, n, cx0, cy0, gx, gy, u))
-            {
-              raise_status(a.status, STATUS_MESH);
-              const double * own = a.U + (size_t)n * H::NV * NC;
-#pragma unroll
-              for (int v = 0; v < H::NV; ++v)
-                u[v] = own[v * NC];
-            }
-            h += NT;
-          }
-          cold |= store_prim<B, MIXED, STIFF>(sQ, gidx, u, P, eosk);
-        }
-      }
-      else
-      {
       for (int h = NT == NC ? tid : (tid < NC ? tid + NT - NC : tid - NC); h < NHALO; h += NT)
       {
         int gx, gy;
@@ -1102,19 +797,15 @@ step2d_kernel(const __grid_constant__ StepArgs a)
           for (int v = 0; v < H::NV; ++v)
             u[v] = NT == NC ? uin[v] : own[v * NC];
         }
-        cold |= store_prim<B, MIXED, STIFF>(sQ, (gx + 2) + G * (gy + 2), u, P, eosk);
+        store_prim<B, MIXED>(sQ, (gx + 2) + G * (gy + 2), u, P, eosk);
       }
       if (owner)
-        cold |= store_prim<B, MIXED, STIFF>(sQ, (ci + 2) + G * (cj + 2), uin, P, eosk);
-      }
+        store_prim<B, MIXED>(sQ, (ci + 2) + G * (cj + 2), uin, P, eosk);
       if (tid < 10)
         sSlot[tid] = slot_v;
       if (tid == 10)
         sNext = next_v;
-      if constexpr (fast64)
-        cold = __syncthreads_or(cold) != 0;
-      else
-        __syncthreads();
+      __syncthreads();
       // the next block of this CTA: its own cells and table rows into L2 while
       // this block computes (its gather then hits L2 instead of HBM)
       if (tid < 3 && sNext < nwalk)
@@ -1132,7 +823,6 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       // (the block, then the row or column beyond each face, without gaps: the
       // ring's corners are never a face neighbour; r: the cell's index in the
       // ring layout)
-      const bool cold0 = cold;
       for (int h = tid; h < NC + 4 * B; h += NT)
       {
         int ri, rj;
@@ -1152,15 +842,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         const int gi = (ri + 2) + G * (rj + 2);
         if constexpr (!MIXED)
         {
-          if constexpr (STIFF == 2)
-            hancock_ref64<B>(sQ, sRec, gi, r, dtdx_r, P);
-          else
-          {
-            if (cold0)
-              hancock_cold64<B>(sQ, sRec, gi, r, dtdx_r, &P);
-            else
-              cold |= hancock_fast64<B, STIFF == 1>(sQ, sRec, gi, r, dtdx_r, P);
-          }
+          hancock_ref64<B>(sQ, sRec, gi, r, dtdx_r, P);
         }
         else
         {
@@ -1207,31 +889,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
           }
         }
       }
-      if constexpr (fast64)
-      {
-        // the interface cells of the THINC reconstruction
-        for (int i = tid; P.thinc != 0 && i < T::NTH; i += NT)
-        {
-          const int      dir = i < B * (B + 2) ? 0 : 1, k = i - dir * B * (B + 2);
-          const int      gi = dir == 0 ? (k % (B + 2) + 1) + G * (k / (B + 2) + 2) : (k % B + 2) + G * (k / B + 1);
-          const double * A = sQ + 5 * GG + gi;
-          const int      o = dir == 0 ? 1 : G;
-          if (thinc_cell64(A[0], A[-o], A[o], P))
-            sList[atomicAdd(&sThinc, 1)] = (short)i;
-          else
-            sAF[i] = sAF[T::NTH + i] = thinc_none64();
-        }
-        cold = __syncthreads_or(cold) != 0;
-        if (P.thinc != 0 && sThinc > 0 && !cold)
-        {
-          for (int i = tid; i < sThinc; i += NT)
-            cold |= thinc_eval2<B>(sQ, sAF, sList[i], P);
-          cold = __syncthreads_or(cold) != 0;
-        }
-      }
-      else
-        __syncthreads();
-      const bool cold1 = cold;
+      __syncthreads();
 
       // ---------------- phase 3: faces (X then Y) -> HLLC -> shared fluxes
       if constexpr (MIXED)
@@ -1248,12 +906,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       {
         for (int f = tid; f < 2 * NFF; f += NT)
         {
-          if constexpr (STIFF == 2)
-            face_flux_ref64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
-          else if (cold1)
-            face_flux_cold64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, &P);
-          else
-            cold |= face_flux_fast64<B, STIFF == 1>(sQ, sRec, sAF, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
+          face_flux_ref64<B>(sQ, sRec, f < NFF ? sFx : sFy, f < NFF ? 0 : 1, f < NFF ? f : f - NFF, dtdx_r, P);
         }
       }
       // the own cell's state for the update: the FP32-bulk form without the
@@ -1278,13 +931,7 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         for (int v = 0; v < H::NV; ++v)
           uown[v] = uin[v];
       }
-      if constexpr (fast64)
-        cold = __syncthreads_or(cold) != 0;
-      else
-        __syncthreads();
-
-      if (fast64 && tid == 0)
-        sThinc = 0; // (read before the barrier above, used again after the next)
+      __syncthreads();
 
       // ---------------- publish coarse/fine records (AMR only)
       if (a.m.reflux_slot)
@@ -1341,25 +988,8 @@ step2d_kernel(const __grid_constant__ StepArgs a)
         if constexpr (MIXED)
           m_inv = update_mixed<B>(uown, u2, sFx, sFy, ci, cj, d2f_fast(dx), P, eosk, a.invdt != nullptr);
         double * out = a.U2 + (size_t)n * H::NV * NC + tid;
-        if constexpr (!MIXED && STIFF == 2)
+        if constexpr (!MIXED)
           m_inv = update_fp64<B>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr);
-        else if constexpr (!MIXED)
-        {
-          bool bad = cold;
-          if (!bad)
-            m_inv = update_fast64<B, STIFF == 1>(uown, u2, sFx, sFy, ci, cj, dx, P, a.invdt != nullptr, bad);
-          if (bad)
-          {
-            State64<2> st;
-#pragma unroll
-            for (int v = 0; v < H::NV; ++v)
-              st.v[v] = uown[v];
-            m_inv = update_cold64<B>(st, out, sFx, sFy, ci, cj, dx, &P, a.invdt != nullptr);
-#pragma unroll
-            for (int v = 0; v < H::NV; ++v)
-              u2[v] = out[v * NC];
-          }
-        }
         bool finite = true;
 #pragma unroll
         for (int v = 0; v < H::NV; ++v)

@@ -107,36 +107,25 @@ hancock_cold3(const double * sQ, double * sHS, int gi, int r, double dtdx, const
   hancock_ref3(sQ, sHS, gi, r, dtdx, *P);
 }
 
-// the reconstructed state of one face side (face_state3<false>, the normal
-// velocity first) and the mixture's S; gi, si, ti: the cell in the ghosted,
-// ring and THINC arrays, o the direction's stride, side +1 the cell's right face
+// the state of one face side beyond its linear reconstruction q: THINC values
+// (ti: the cell's entry) or the floor of the partial densities.  Returns the
+// mixture's S; gi, si: the cell in the ghosted and ring arrays, af the side's
+// THINC values
 __device__ __forceinline__ double
-face_state_fast3(const double * sQ, const double * sHS, const double * sS, const double * sAF, int gi, int si, int ti, int o, int dir, int side,
-                 const PhysParams & P, double * q, bool & bad)
+face_side_fast3(const double * sQ, const double * sHS, const double * sS, const double * af_side, int gi, int si, int ti, const PhysParams & P, double * q,
+                bool & bad)
 {
   using T = Step3D64::T;
   constexpr int GGG = T::GGG, SSS = T::SSS;
-  const double  off = side > 0 ? 0.5 : -0.5;
-  const int     st = P.st64;
-  const bool    hancock = P.integrator == 0;
-#pragma unroll
-  for (int k = 0; k < 6; ++k)
-  {
-    const int      from = k < 3 ? k : (k == 3 ? 3 + dir : (k == 3 + dir ? 3 : k));
-    const double * Qk = sQ + from * GGG + gi;
-    double         t = Qk[0];
-    if (st != 0)
-      t = __fma_rn(off, slope_fast64(t, Qk[o], Qk[-o], st, bad), t);
-    q[k] = hancock ? __fma_rn(0.5, sHS[from * SSS + si], t) : t;
-  }
-  const double a0 = sQ[6 * GGG + gi];
-  double       S = sS[si];
+  const double  a0 = sQ[6 * GGG + gi];
+  double        S = sS[si];
   q[6] = a0;
   if (P.thinc)
   {
-    const double af = sAF[side > 0 ? ti : Step3D64::NTHINC + ti];
+    const double af = af_side[ti];
     if (bits64(af) != bits64(thinc_none64()))
     {
+      const bool        hancock = P.integrator == 0;
       const ThincSide64 t = thinc_side64(a0, af, sQ[gi], sQ[GGG + gi], hancock ? sHS[si] : 0.0, hancock ? sHS[SSS + si] : 0.0, &P);
       q[0] = t.q0;
       q[1] = t.q1;
@@ -232,15 +221,40 @@ face_flux_fast3(const double * sQ, const double * sHS, const double * sS, const 
 {
   using T = Step3D64::T;
   using H = V<3>;
-  constexpr int B = T::B, G = T::G, GG = T::GG, S = T::S, SS = T::SS, NFF = T::NFF;
+  constexpr int B = T::B, G = T::G, GG = T::GG, GGG = T::GGG, S = T::S, SS = T::SS, SSS = T::SSS, NFF = T::NFF;
   const int     ex = B + (dir == 0), ey = B + (dir == 1);
   const int     fi = f % ex, fj = (f / ex) % ey, fk = f / (ex * ey);
   const int     gR = (fi + 2) + G * (fj + 2) + GG * (fk + 2), sR = (fi + 1) + S * (fj + 1) + SS * (fk + 1);
   const int     o = ghost_stride3(dir);
   double        qL[7], qR[7], fl[9];
   bool          bad = false;
-  const double  Sl = face_state_fast3(sQ, sHS, sS, sAF, gR - o, sR - ring_stride3(dir), thinc_index3(dir, fi - (dir == 0), fj - (dir == 1), fk - (dir == 2)), o, dir, 1, P, qL, bad);
-  const double  Sr = face_state_fast3(sQ, sHS, sS, sAF, gR, sR, thinc_index3(dir, fi, fj, fk), o, dir, -1, P, qR, bad);
+  // both sides' linear states (face_state3<false>, the normal velocity first):
+  // of a component's four values across the face, the middle difference serves
+  // both slopes
+  const int     sL = sR - ring_stride3(dir), st = P.st64;
+  const bool    hancock = P.integrator == 0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+  {
+    const int      from = k < 3 ? k : (k == 3 ? 3 + dir : (k == 3 + dir ? 3 : k));
+    const double * Q = sQ + from * GGG + gR;
+    const double   b = Q[-o], c = Q[0];
+    qL[k] = b;
+    qR[k] = c;
+    if (st != 0)
+    {
+      const double a_ = Q[-2 * o], d = Q[o], m = c - b;
+      qL[k] = __fma_rn(0.5, limit_fast64(b - a_, m, c, a_, st, bad), b);
+      qR[k] = __fma_rn(-0.5, limit_fast64(m, d - c, d, b, st, bad), c);
+    }
+    if (hancock)
+    {
+      qL[k] = __fma_rn(0.5, sHS[from * SSS + sL], qL[k]);
+      qR[k] = __fma_rn(0.5, sHS[from * SSS + sR], qR[k]);
+    }
+  }
+  const double  Sl = face_side_fast3(sQ, sHS, sS, sAF, gR - o, sL, thinc_index3(dir, fi - (dir == 0), fj - (dir == 1), fk - (dir == 2)), P, qL, bad);
+  const double  Sr = face_side_fast3(sQ, sHS, sS, sAF + Step3D64::NTHINC, gR, sR, thinc_index3(dir, fi, fj, fk), P, qR, bad);
   const Side64  L = hllc_side64<3, MG>(qL, Sl, P, bad);
   const Side64  R = hllc_side64<3, MG>(qR, Sr, P, bad);
   hllc_fast64<3>(qL, qR, L, R, dtdx, fl, bad);

@@ -188,3 +188,24 @@ def test_mie_grueneisen_step_and_fields_match_oracle(law, other, dim, kw, thinc)
     f = impl.pack_fields(d_U, [64 + q for q in range(8)]).cpu().numpy()
     for q in range(8):
         assert np.array_equal(f[q], np.asarray(derived(p, U, q)).reshape(U.shape[0], -1)[:n], equal_nan=True), q
+
+
+@pytest.mark.parametrize("nref,thinc", [(1, 0), (2, 1), (40, 0), (40, 1)])
+def test_half_block_round_in_the_solver_loop(nref, thinc):
+    """16x16 blocks few enough for a last round in halves (and more): walls,
+    coarse/fine records and the boundary fill inside the step, five steps."""
+    mesh, t = amr_mesh(dim=2, b=16, periodic=False, nbrick=(3, 2), nref=nref, lmin=1, lmax=4, seed=nref)
+    p = water_air_params(t, b=16, bc=(2, 2, 3, 3, 1, 1), thinc=thinc)
+    p.gamma, p.pinf = GASES["ideal"]
+    U = smooth_state(mesh, t, p)
+    o = Oracle(t, p)
+    ref, hist = o.run(U.copy(), 5)
+    impl = GodunovImplemGB300(p, t)
+    d_U = torch.from_numpy(U).cuda()
+    d_U2 = torch.zeros_like(d_U)
+    dts = torch.zeros((5, 1), dtype=torch.float64, device="cuda")
+    impl.run(d_U, d_U2, 5, mode="fp64", dt_hist=dts)
+    torch.cuda.synchronize()
+    assert impl.status() == 0
+    assert np.array_equal(dts.cpu().numpy().ravel(), np.asarray(hist).ravel())
+    assert np.array_equal(d_U.cpu().numpy(), ref)
