@@ -937,10 +937,21 @@ step3d_kernel(StepArgs a)
               c3[dir == 0 ? 1 : 0] = t1;
               c3[dir == 2 ? 1 : 2] = t2;
               const int fidx = c3[0] + ext0 * (c3[1] + ext1 * c3[2]);
-              double *  dst = a.reflux_buf + ((size_t)rs * B * B + tid) * 9;
+              if constexpr (MIXED)
+              {
+                // floats, component by component (coalesced; see reflux3d_kernel)
+                float * dst = reinterpret_cast<float *>(a.reflux_buf) + (size_t)rs * 9 * B * B + tid;
 #pragma unroll
-              for (int k = 0; k < 9; ++k)
-                dst[k] = (double)sFd[k * NFF + fidx];
+                for (int k = 0; k < 9; ++k)
+                  dst[k * B * B] = sFd[k * NFF + fidx];
+              }
+              else
+              {
+                double * dst = a.reflux_buf + ((size_t)rs * B * B + tid) * 9;
+#pragma unroll
+                for (int k = 0; k < 9; ++k)
+                  dst[k] = sFd[k * NFF + fidx];
+              }
             }
           }
           // own face fluxes of deferred cells, this direction (left then right)
@@ -953,12 +964,25 @@ step3d_kernel(StepArgs a)
                 continue;
               const int d2 = f >> 1;
               const int t1 = cc[d2 == 0 ? 1 : 0], t2 = cc[d2 == 2 ? 1 : 2];
-              double *  dst = a.defer_buf + (((size_t)dsl[f] * B * B + t1 + B * t2) * 6 + 2 * dir) * 9;
-#pragma unroll
-              for (int k = 0; k < 9; ++k)
+              if constexpr (MIXED)
               {
-                dst[k] = (double)sFd[k * NFF + il];
-                dst[9 + k] = (double)sFd[k * NFF + ir];
+                float * dst = reinterpret_cast<float *>(a.defer_buf) + ((size_t)dsl[f] * 54 + 18 * dir) * B * B + t1 + B * t2;
+#pragma unroll
+                for (int k = 0; k < 9; ++k)
+                {
+                  dst[k * B * B] = sFd[k * NFF + il];
+                  dst[(9 + k) * B * B] = sFd[k * NFF + ir];
+                }
+              }
+              else
+              {
+                double * dst = a.defer_buf + (((size_t)dsl[f] * B * B + t1 + B * t2) * 6 + 2 * dir) * 9;
+#pragma unroll
+                for (int k = 0; k < 9; ++k)
+                {
+                  dst[k] = sFd[k * NFF + il];
+                  dst[9 + k] = sFd[k * NFF + ir];
+                }
               }
             }
           }
@@ -1093,7 +1117,11 @@ step3d_kernel(StepArgs a)
 
 // reflux: coarse cells next to finer faces, one thread per (record, cell of
 // the face).  Replays update_U direction by direction with the fine face sums
-// (2x2 fine faces, / 8) of get_flux_from_fine_neighbor.
+// (2x2 fine faces, / 8) of get_flux_from_fine_neighbor.  The FP32-bulk form's
+// records hold floats, one component after another (64 cells each), so that the
+// threads of a warp write and read runs (9 doubles per face and cell, each
+// cell's together, cost 18.6 us per triple-point step of 2.0M cells in this
+// pass, and 18 conversions per deferred cell in the step).
 template <bool MIXED>
 __global__ void
 reflux3d_kernel(StepArgs a)
@@ -1146,8 +1174,7 @@ reflux3d_kernel(StepArgs a)
   if constexpr (MIXED)
   {
     // FP32-bulk form: per direction the two sides' fluxes as float pairs (a
-    // fine side is the float-float sum of its 2x2 fine faces, / 8; the
-    // records hold floats as doubles), their differences as exact float
+    // fine side is the float-float sum of its 2x2 fine faces, / 8), their differences as exact float
     // pairs, and the step kernel's update of the increments (apply_mixed_3d)
     const int eosk = a.p.mg_any ? 2 : ((a.p.gpx[0] != 0.0 || a.p.gpx[1] != 0.0) ? 1 : 0);
     float     fst0, fst1;
@@ -1186,13 +1213,14 @@ reflux3d_kernel(StepArgs a)
             raise_status(a.status, STATUS_MESH);
             return;
           }
-          const double * fb = a.reflux_buf + ((size_t)rs * B * B + fl[e1] + B * fl[e2]) * 9;
+          // (fl[e1] is even: two neighbouring fine faces per 8-byte load)
+          const float * fb = reinterpret_cast<const float *>(a.reflux_buf) + (size_t)rs * 9 * B * B + fl[e1] + B * fl[e2];
 #pragma unroll
           for (int k = 0; k < 9; ++k)
           {
-            const float v0 = d2f_fast(fb[k]), v1 = d2f_fast(fb[9 + k]);
-            const float v2 = d2f_fast(fb[B * 9 + k]), v3 = d2f_fast(fb[(B + 1) * 9 + k]);
-            float       s, t1, t2, t3;
+            const float2 p0 = *reinterpret_cast<const float2 *>(fb + k * B * B), p1 = *reinterpret_cast<const float2 *>(fb + k * B * B + B);
+            const float  v0 = p0.x, v1 = p0.y, v2 = p1.x, v3 = p1.y;
+            float        s, t1, t2, t3;
             two_sum(v0, v1, s, t1);
             two_sum(s, v2, s, t2);
             two_sum(s, v3, s, t3);
@@ -1202,11 +1230,11 @@ reflux3d_kernel(StepArgs a)
         }
         else
         {
-          const double * fr = own + fface * 9;
+          const float * fr = reinterpret_cast<const float *>(a.defer_buf) + ((size_t)dsl[face] * 54 + 9 * fface) * B * B + pos;
 #pragma unroll
           for (int k = 0; k < 9; ++k)
           {
-            Fh[side][k] = d2f_fast(fr[k]);
+            Fh[side][k] = fr[k * B * B];
             Fl[side][k] = 0.0f;
           }
         }
