@@ -40,11 +40,6 @@ neg_zero(double x)
 {
   return __double_as_longlong(x) == (long long)0x8000000000000000ULL;
 }
-__device__ __forceinline__ bool
-neg_zero(float x)
-{
-  return __float_as_uint(x) == 0x80000000u;
-}
 
 // The halo cells of an 8^3 block that the step reads, as ghosted offsets
 // (-2 .. 9); the other 128 cells of the 12^3 ghosted cube (two coordinates
@@ -112,13 +107,6 @@ halo_coords_3d(int h, int * g)
     g[k] = ((corner >> k) & 1) ? 7 + e : -e;
   }
 }
-
-// HLLC flux of face f of direction DIR (normal velocity swapped into u and
-// back), scaled by dt/dx into the face buffer sFd ([9][NFF])
-template <bool MIXED, int DIR, int THINC, bool MG = false>
-__device__ __forceinline__ void face_flux3(const typename Step3DTraits<MIXED>::R * sQ, const typename Step3DTraits<MIXED>::R * sHS,
-                                           int f, typename Step3DTraits<MIXED>::R * sFd, typename Step3DTraits<MIXED>::R dtdx_r,
-                                           const PhysParams & P);
 
 // conservative state seen by ghost cell g of block n (3D); false on a bad
 // index.  ALPHA_ONLY: u[IA0] only (the same loads and sums for that variable)
@@ -268,8 +256,6 @@ slope_at(const R * Qk, int gi, int o, R st)
   return slope_scalar<R>(Qk[gi], Qk[gi + o], Qk[gi - o], st);
 }
 
-// reconstructed state of cell (ci,cj,ck) at its face in direction dir
-// (side +1: right face, side -1: left face); q[7] = r0 r1 p u v w a0
 // |n_dir| of the Youngs normal of the alpha field at ghosted index gi
 // ((1,2,1) x (1,2,1) weighted central differences, unit cell, n = -grad/|grad|),
 // evaluated where THINC needs it (interface cells only)
@@ -294,189 +280,206 @@ youngs_abs_3d(const R * A, int gi, int dir)
   return (nrm > R(0)) ? fabs(-gd / nrm) : R(0);
 }
 
-template <bool MIXED, int THINC = -1>
+// FP64: the state of cell (ci, cj, ck) at its face in direction dir (side +1:
+// right face, -1: left face), in the reference's order; q[7] = r0 r1 p u v w a0.
+// The Hancock source is stored without its factor 1/2.
 __device__ __forceinline__ void
-face_state3(const typename Step3DTraits<MIXED>::R * sQ,
-            const typename Step3DTraits<MIXED>::R * sHS,
-            int                                     ci,
-            int                                     cj,
-            int                                     ck,
-            int                                     dir,
-            int                                     side,
-            const PhysParams &                      P,
-            typename Step3DTraits<MIXED>::R *       q)
+face_state3(const double * sQ, const double * sHS, int ci, int cj, int ck, int dir, int side, const PhysParams & P, double * q)
 {
-  using T = Step3DTraits<MIXED>;
-  using R = typename T::R;
+  using T = Step3DTraits<false>;
   constexpr int G = T::G, GG = T::GG, GGG = T::GGG, S = T::S, SS = T::SS, SSS = T::SSS;
   const int     gi = (ci + 2) + G * (cj + 2) + GG * (ck + 2);
   const int     si = (ci + 1) + S * (cj + 1) + SS * (ck + 1);
   const int     strides[3] = { 1, G, GG };
   const int     o = strides[dir];
-  R             st, smallr, thinc_eps, thinc_beta;
-  if constexpr (MIXED)
-  {
-    st = P.f_slope_type;
-    smallr = P.f_smallr;
-    thinc_eps = P.f_thinc_eps;
-    thinc_beta = P.f_thinc_beta;
-  }
-  else
-  {
-    st = P.slope_type;
-    smallr = P.smallr;
-    thinc_eps = P.thinc_eps;
-    thinc_beta = P.thinc_beta;
-  }
-  const bool hancock = P.integrator == 0;
-  const R    off = R(0.5) * R(side);
-  if constexpr (MIXED)
-  {
-    // two components per packed slope evaluation
+  const double  st = P.slope_type;
+  const bool    hancock = P.integrator == 0;
+  const double  off = 0.5 * side;
 #pragma unroll
-    for (int k = 0; k < 6; k += 2)
+  for (int k = 0; k < 6; ++k)
+  {
+    const double * Qk = sQ + k * GGG;
+    const double   qc = Qk[gi];
+    const double   dq = slope_at<double>(Qk, gi, o, st);
+    double         t = qc + off * dq;
+    // the reference adds the zero-offset terms of the other directions,
+    // ((q + o_x dq_x) + o_y dq_y) + o_z dq_z; they can only change the sign
+    // of a zero, so they are evaluated only when a negative zero occurs
+    if (neg_zero(qc) || neg_zero(t))
     {
-      const R *    Q0 = sQ + k * GGG;
-      const R *    Q1 = Q0 + GGG;
-      const float2 qc = make_float2(Q0[gi], Q1[gi]);
-      const float2 dq = slope_pair(qc, make_float2(Q0[gi + o], Q1[gi + o]), make_float2(Q0[gi - o], Q1[gi - o]), st);
-      q[k] = qc.x + off * dq.x;
-      q[k + 1] = qc.y + off * dq.y;
-      if (hancock)
-      {
-        q[k] += sHS[k * SSS + si];
-        q[k + 1] += sHS[(k + 1) * SSS + si];
-      }
-    }
-  }
-  else
-  {
+      double dd[3];
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
-    {
-      const R * Qk = sQ + k * GGG;
-      const R   qc = Qk[gi];
-      const R   dq = slope_at<R>(Qk, gi, o, st);
-      R         t = qc + off * dq;
-      // the reference adds the zero-offset terms of the other directions,
-      // ((q + o_x dq_x) + o_y dq_y) + o_z dq_z; they can only change the sign
-      // of a zero, so they are evaluated only when a negative zero occurs
-      if (neg_zero(qc) || neg_zero(t))
-      {
-        R dd[3];
-#pragma unroll
-        for (int e = 0; e < 3; ++e)
-          dd[e] = slope_at<R>(Qk, gi, strides[e], st);
-        const R o0 = dir == 0 ? off : R(0), o1 = dir == 1 ? off : R(0), o2 = dir == 2 ? off : R(0);
-        t = qc + o0 * dd[0] + o1 * dd[1] + o2 * dd[2];
-      }
-      q[k] = t;
-      if (hancock)
-        q[k] += R(0.5) * sHS[k * SSS + si]; // (the FP64 form stores the source without its factor 1/2)
+      for (int e = 0; e < 3; ++e)
+        dd[e] = slope_at<double>(Qk, gi, strides[e], st);
+      const double o0 = dir == 0 ? off : 0.0, o1 = dir == 1 ? off : 0.0, o2 = dir == 2 ? off : 0.0;
+      t = qc + o0 * dd[0] + o1 * dd[1] + o2 * dd[2];
     }
+    q[k] = t;
+    if (hancock)
+      q[k] += 0.5 * sHS[k * SSS + si];
   }
-  const R a0 = sQ[6 * GGG + gi];
+  const double a0 = sQ[6 * GGG + gi];
   q[6] = a0;
-  if (THINC < 0 ? P.thinc != 0 : THINC == 1)
+  if (P.thinc != 0)
   {
-    const R *  A = sQ + 6 * GGG;
-    const R    aP = A[gi + o], aM = A[gi - o];
-    const R    mono = (aP - a0) * (a0 - aM);
-    const bool req = (a0 > thinc_eps) && (a0 < R(1) - thinc_eps) && mono > R(0);
-    if (req)
+    const double * A = sQ + 6 * GGG;
+    const double   aP = A[gi + o], aM = A[gi - o];
+    const double   mono = (aP - a0) * (a0 - aM);
+    if ((a0 > P.thinc_eps) && (a0 < 1.0 - P.thinc_eps) && mono > 0.0)
     {
-      const R nd = youngs_abs_3d<R, G, GG>(A, gi, dir);
-      const R beta = thinc_beta * nd + R(0.01);
-      const R Aa = (aP + aM) / R(2);
-      const R Bb = (aP - aM) / R(2);
-      R       C, D;
-      if constexpr (MIXED)
-      {
-        C = tanhf(R(0.5) * beta);
-        D = tanhf(R(0.5) * beta * (a0 - Aa) / Bb);
-      }
-      else
-      {
-        C = tanh_d(R(0.5) * beta);
-        D = tanh_d(R(0.5) * beta * (a0 - Aa) / Bb);
-      }
-      const R bs = R(side);
-      const R af = Aa + bs * Bb * (C + bs * D / C) / (R(1) + bs * D);
-      const R r0 = sQ[0 * GGG + gi], r1 = sQ[1 * GGG + gi];
-      R       q0 = r0 + r0 / a0 * (af - a0);
-      R       q1 = r1 + r1 / (R(1) - a0) * (a0 - af);
+      const double nd = youngs_abs_3d<double, G, GG>(A, gi, dir);
+      const double beta = P.thinc_beta * nd + 0.01;
+      const double Aa = (aP + aM) / 2.0;
+      const double Bb = (aP - aM) / 2.0;
+      const double C = tanh_d(0.5 * beta);
+      const double D = tanh_d(0.5 * beta * (a0 - Aa) / Bb);
+      const double bs = (double)side;
+      const double af = Aa + bs * Bb * (C + bs * D / C) / (1.0 + bs * D);
+      const double r0 = sQ[0 * GGG + gi], r1 = sQ[1 * GGG + gi];
+      q[0] = r0 + r0 / a0 * (af - a0);
+      q[1] = r1 + r1 / (1.0 - a0) * (a0 - af);
       if (hancock)
       {
-        q0 += (MIXED ? R(1) : R(0.5)) * sHS[0 * SSS + si];
-        q1 += (MIXED ? R(1) : R(0.5)) * sHS[1 * SSS + si];
+        q[0] += 0.5 * sHS[0 * SSS + si];
+        q[1] += 0.5 * sHS[1 * SSS + si];
       }
-      q[0] = q0;
-      q[1] = q1;
       q[6] = af;
     }
   }
   else
   {
-    q[0] = fmax(smallr, q[0]);
-    q[1] = fmax(smallr, q[1]);
+    q[0] = fmax(P.smallr, q[0]);
+    q[1] = fmax(P.smallr, q[1]);
   }
 }
 
-template <bool MIXED, int DIR, int THINC, bool MG>
+// FP64: HLLC flux of face f of direction DIR (normal velocity swapped into u
+// and back), scaled by dt/dx into the face buffer sFd ([9][NFF])
+template <int DIR>
 __device__ __forceinline__ void
-face_flux3(const typename Step3DTraits<MIXED>::R * sQ, const typename Step3DTraits<MIXED>::R * sHS, int f,
-           typename Step3DTraits<MIXED>::R * sFd, typename Step3DTraits<MIXED>::R dtdx_r, const PhysParams & P)
+face_flux3(const double * sQ, const double * sHS, int f, double * sFd, double dtdx, const PhysParams & P)
 {
-  using T = Step3DTraits<MIXED>;
-  using R = typename T::R;
+  using T = Step3DTraits<false>;
   using H = V<3>;
-  constexpr int B = T::B, NFF = T::NFF;
-  int           fi, fj, fk;
-  if (DIR == 0)
-  {
-    fi = f % (B + 1);
-    fj = (f / (B + 1)) % B;
-    fk = f / ((B + 1) * B);
-  }
-  else if (DIR == 1)
-  {
-    fi = f % B;
-    fj = (f / B) % (B + 1);
-    fk = f / (B * (B + 1));
-  }
-  else
-  {
-    fi = f % B;
-    fj = (f / B) % B;
-    fk = f / (B * B);
-  }
-  R qL[7], qR[7], fl[9];
-  face_state3<MIXED, THINC>(sQ, sHS, fi - (DIR == 0), fj - (DIR == 1), fk - (DIR == 2), DIR, +1, P, qL);
-  face_state3<MIXED, THINC>(sQ, sHS, fi, fj, fk, DIR, -1, P, qR);
+  constexpr int B = T::B, NFF = T::NFF, EX = B + (DIR == 0), EY = B + (DIR == 1);
+  const int     fi = f % EX, fj = (f / EX) % EY, fk = f / (EX * EY);
+  double        qL[7], qR[7], fl[9];
+  face_state3(sQ, sHS, fi - (DIR == 0), fj - (DIR == 1), fk - (DIR == 2), DIR, +1, P, qL);
+  face_state3(sQ, sHS, fi, fj, fk, DIR, -1, P, qR);
   if (DIR > 0)
   {
     constexpr int iw = DIR == 1 ? 4 : 5; // component swapped with u
-    R             t = qL[3];
+    double        t = qL[3];
     qL[3] = qL[iw];
     qL[iw] = t;
     t = qR[3];
     qR[3] = qR[iw];
     qR[iw] = t;
   }
-  if constexpr (MIXED)
-    hllc_fp32<3>(qL, qR, P.f_xi[0], P.f_xi[1], P.f_gpx[0], P.f_gpx[1], P.f_smallr, P.f_smallp, P.f_smallc, fl, MG ? &P : nullptr);
-  else
-    hllc_fp64<3>(qL, qR, P, fl);
+  hllc_fp64<3>(qL, qR, P, fl);
   if (DIR > 0)
   {
     constexpr int fw = DIR == 1 ? H::FV : H::FW;
-    const R       t = fl[H::FU];
+    const double  t = fl[H::FU];
     fl[H::FU] = fl[fw];
     fl[fw] = t;
   }
 #pragma unroll
   for (int k = 0; k < 9; ++k)
-    sFd[k * NFF + f] = fl[k] * dtdx_r;
+    sFd[k * NFF + f] = fl[k] * dtdx;
+}
+
+// The FP32-bulk face flux with the direction as a run-time value: the two
+// passes' four rounds of faces have one copy of the code each pass (three
+// directions' code inlined six times missed the instruction cache: 380 -> 359 us
+// per triple-point step of 2.0M cells)
+template <int THINC, bool MG>
+__device__ __forceinline__ void
+face_flux3_dir(const float * sQ, const float * sHS, int f, int dir, float * sFd, float dtdx, const PhysParams & P)
+{
+  using T = Step3DTraits<true>;
+  using H = V<3>;
+  constexpr int B = T::B, G = T::G, GG = T::GG, GGG = T::GGG, S = T::S, SS = T::SS, SSS = T::SSS, NFF = T::NFF;
+  const int     ex = B + (dir == 0), ey = B + (dir == 1);
+  const int     fz = dir == 2 ? f >> 6 : f / 72, rem = f - fz * (ex * ey);
+  const int     fy = dir == 0 ? rem / 9 : rem >> 3, fx = rem - fy * ex;
+  const int     o = dir == 0 ? 1 : (dir == 1 ? G : GG), so = dir == 0 ? 1 : (dir == 1 ? S : SS);
+  const int     gR = (fx + 2) + G * (fy + 2) + GG * (fz + 2), sR = (fx + 1) + S * (fy + 1) + SS * (fz + 1);
+  float         q[2][7], fl[9];
+#pragma unroll
+  for (int side = 0; side < 2; ++side)
+  {
+    const int   gi = side == 0 ? gR - o : gR, si = side == 0 ? sR - so : sR;
+    const float off = side == 0 ? 0.5f : -0.5f, st = P.f_slope_type;
+    const bool  hancock = P.integrator == 0;
+    float *     qs = q[side];
+    // two components per packed slope evaluation
+#pragma unroll
+    for (int k = 0; k < 6; k += 2)
+    {
+      const float * Q0 = sQ + k * GGG;
+      const float * Q1 = Q0 + GGG;
+      const float2  qc = make_float2(Q0[gi], Q1[gi]);
+      const float2  dq = slope_pair(qc, make_float2(Q0[gi + o], Q1[gi + o]), make_float2(Q0[gi - o], Q1[gi - o]), st);
+      qs[k] = qc.x + off * dq.x;
+      qs[k + 1] = qc.y + off * dq.y;
+      if (hancock)
+      {
+        qs[k] += sHS[k * SSS + si];
+        qs[k + 1] += sHS[(k + 1) * SSS + si];
+      }
+    }
+    const float a0 = sQ[6 * GGG + gi];
+    qs[6] = a0;
+    if constexpr (THINC == 1)
+    {
+      const float * A = sQ + 6 * GGG;
+      const float   aP = A[gi + o], aM = A[gi - o];
+      const float   mono = (aP - a0) * (a0 - aM);
+      if ((a0 > P.f_thinc_eps) && (a0 < 1.0f - P.f_thinc_eps) && mono > 0.0f)
+      {
+        const float nd = youngs_abs_3d<float, G, GG>(A, gi, dir);
+        const float beta = P.f_thinc_beta * nd + 0.01f;
+        const float Aa = (aP + aM) / 2.0f;
+        const float Bb = (aP - aM) / 2.0f;
+        const float C = tanhf(0.5f * beta);
+        const float D = tanhf(0.5f * beta * (a0 - Aa) / Bb);
+        const float bs = side == 0 ? 1.0f : -1.0f;
+        const float af = Aa + bs * Bb * (C + bs * D / C) / (1.0f + bs * D);
+        const float r0 = sQ[0 * GGG + gi], r1 = sQ[1 * GGG + gi];
+        float       q0 = r0 + r0 / a0 * (af - a0);
+        float       q1 = r1 + r1 / (1.0f - a0) * (a0 - af);
+        if (hancock)
+        {
+          q0 += sHS[0 * SSS + si];
+          q1 += sHS[1 * SSS + si];
+        }
+        qs[0] = q0;
+        qs[1] = q1;
+        qs[6] = af;
+      }
+    }
+    else
+    {
+      qs[0] = fmaxf(P.f_smallr, qs[0]);
+      qs[1] = fmaxf(P.f_smallr, qs[1]);
+    }
+    // normal velocity first
+    const float u = qs[3], un = dir == 0 ? qs[3] : (dir == 1 ? qs[4] : qs[5]);
+    qs[4] = dir == 1 ? u : qs[4];
+    qs[5] = dir == 2 ? u : qs[5];
+    qs[3] = un;
+  }
+  hllc_fp32<3>(q[0], q[1], P.f_xi[0], P.f_xi[1], P.f_gpx[0], P.f_gpx[1], P.f_smallr, P.f_smallp, P.f_smallc, fl, MG ? &P : nullptr);
+  {
+    const float u = fl[H::FU], un = dir == 0 ? fl[H::FU] : (dir == 1 ? fl[H::FV] : fl[H::FW]);
+    fl[H::FV] = dir == 1 ? u : fl[H::FV];
+    fl[H::FW] = dir == 2 ? u : fl[H::FW];
+    fl[H::FU] = un;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k)
+    sFd[k * NFF + f] = fl[k] * dtdx;
 }
 
 // FP64: Hancock half-step source (ComputeFluxesAndStoreFunctor.cpp:273-306,
@@ -641,7 +644,7 @@ apply_mixed_3d(double * u2, const float (&hh)[3][2], const float (&ll)[3][2], co
 // time, the FP64 form)
 template <bool MIXED, int THINC = -1, int STIFF = -1>
 __global__ void __launch_bounds__(512, MIXED ? 2 : 1)
-step3d_kernel(StepArgs a)
+step3d_kernel(const __grid_constant__ StepArgs a)
 {
   using T = Step3DTraits<MIXED>;
   using R = typename T::R;
@@ -689,7 +692,6 @@ step3d_kernel(StepArgs a)
       for (int v = 0; v < H::NV; ++v)
         uin[v] = base[v * NC];
     }
-    store_prim3<MIXED>(sQ, (ci + 2) + G * (cj + 2) + GG * (ck + 2), uin, P, eosk);
     // FP32-bulk form: the owned cell's volume-fraction source-term factors
     // and its volume fractions as floats, taken now so that the nine doubles
     // of the cell do not stay live through the gather, slope and face phases;
@@ -705,15 +707,23 @@ step3d_kernel(StepArgs a)
       a1f = af1 * fst1;
     }
     const int nhalo = HALO3_FULL + ((THINC < 0 ? P.thinc != 0 : THINC == 1) ? HALO3_ALPHA : 0);
-    for (int h = tid; h < nhalo; h += NT)
+    // (the own cell is the loop's first item: one copy of the conversion)
+    for (int h = tid - NT; h < nhalo; h += NT)
     {
-      int g[3];
-      halo_coords_3d(h, g);
+      int g[3] = { ci, cj, ck };
+      if (h >= 0)
+        halo_coords_3d(h, g);
       const int gidx = (g[0] + 2) + G * (g[1] + 2) + GG * (g[2] + 2);
       double    u[H::NV];
       if (h < HALO3_FULL)
       {
-        if (!gather_ghost_3d(a, n, c0, g, u))
+        if (h < 0)
+        {
+#pragma unroll
+          for (int v = 0; v < H::NV; ++v)
+            u[v] = uin[v];
+        }
+        else if (!gather_ghost_3d(a, n, c0, g, u))
         {
           raise_status(a.status, STATUS_MESH);
           const double * own = a.U + (size_t)n * H::NV * NC + tid;
@@ -877,22 +887,16 @@ step3d_kernel(StepArgs a)
         constexpr int YA = NT - XR;       // Y faces of pass 0 (448)
         constexpr int YB = NFF - YA;      // Y faces of pass 1 (128)
         R *           sF1 = sF + T::NF * NFF;
-        if (pass == 0)
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r)
         {
-          face_flux3<MIXED, 0, THINC, STIFF == 2>(sQ, sHS, tid, sF, dtdx_r, P);
-          if (tid < XR)
-            face_flux3<MIXED, 0, THINC, STIFF == 2>(sQ, sHS, tid + NT, sF, dtdx_r, P);
-          else
-            face_flux3<MIXED, 1, THINC, STIFF == 2>(sQ, sHS, tid - XR, sF1, dtdx_r, P);
-        }
-        else
-        {
-          if (tid < YB)
-            face_flux3<MIXED, 1, THINC, STIFF == 2>(sQ, sHS, tid + YA, sF1, dtdx_r, P);
-          else
-            face_flux3<MIXED, 2, THINC, STIFF == 2>(sQ, sHS, tid - YB, sF, dtdx_r, P);
-          if (tid < NFF - (NT - YB))
-            face_flux3<MIXED, 2, THINC, STIFF == 2>(sQ, sHS, tid + NT - YB, sF, dtdx_r, P);
+          // pass 0: X faces, the last 64 with the first 448 Y faces; pass 1:
+          // the other Y faces with the first 384 Z faces, then the rest
+          const bool first = pass == 0 ? (r == 0 || tid < XR) : (r == 0 && tid < YB);
+          const int  dir = pass == 0 ? (first ? 0 : 1) : (first ? 1 : 2);
+          const int  f = pass == 0 ? (first ? tid + r * NT : tid - XR) : (first ? tid + YA : tid + r * NT - YB);
+          if (f < NFF)
+            face_flux3_dir<THINC, STIFF == 2>(sQ, sHS, f, dir, dir == 1 ? sF1 : sF, dtdx_r, P);
         }
       }
       else
@@ -900,11 +904,11 @@ step3d_kernel(StepArgs a)
         for (int f = tid; f < NFF; f += NT)
         {
           if (pass == 0)
-            face_flux3<MIXED, 0, THINC, STIFF == 2>(sQ, sHS, f, sF, dtdx_r, P);
+            face_flux3<0>(sQ, sHS, f, sF, dtdx_r, P);
           else if (pass == 1)
-            face_flux3<MIXED, 1, THINC, STIFF == 2>(sQ, sHS, f, sF, dtdx_r, P);
+            face_flux3<1>(sQ, sHS, f, sF, dtdx_r, P);
           else
-            face_flux3<MIXED, 2, THINC, STIFF == 2>(sQ, sHS, f, sF, dtdx_r, P);
+            face_flux3<2>(sQ, sHS, f, sF, dtdx_r, P);
         }
       }
       __syncthreads();

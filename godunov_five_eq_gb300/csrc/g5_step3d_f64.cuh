@@ -146,11 +146,11 @@ __device__ __noinline__ void
 face_flux_cold3(const double * sQ, const double * sHS, double * sF, int f, int dir, double dtdx, const PhysParams * P)
 {
   if (dir == 0)
-    face_flux3<false, 0, -1>(sQ, sHS, f, sF, dtdx, *P);
+    face_flux3<0>(sQ, sHS, f, sF, dtdx, *P);
   else if (dir == 1)
-    face_flux3<false, 1, -1>(sQ, sHS, f, sF, dtdx, *P);
+    face_flux3<1>(sQ, sHS, f, sF, dtdx, *P);
   else
-    face_flux3<false, 2, -1>(sQ, sHS, f, sF, dtdx, *P);
+    face_flux3<2>(sQ, sHS, f, sF, dtdx, *P);
 }
 
 // the THINC entry of the cell (x, y, z) of direction dir: 10 cells along it,
@@ -214,7 +214,7 @@ thinc_eval3(const double * sQ, double * sAF, int dir, int i, const PhysParams & 
   return bad;
 }
 
-// HLLC flux of face f of direction dir, scaled by dt/dx (face_flux3<false>)
+// HLLC flux of face f of direction dir, scaled by dt/dx (face_flux3)
 template <bool MG>
 __device__ __forceinline__ bool
 face_flux_fast3(const double * sQ, const double * sHS, const double * sS, const double * sAF, double * sF, int f, int dir, double dtdx, const PhysParams & P)
@@ -228,7 +228,7 @@ face_flux_fast3(const double * sQ, const double * sHS, const double * sS, const 
   const int     o = ghost_stride3(dir);
   double        qL[7], qR[7], fl[9];
   bool          bad = false;
-  // both sides' linear states (face_state3<false>, the normal velocity first):
+  // both sides' linear states (face_state3, the normal velocity first):
   // of a component's four values across the face, the middle difference serves
   // both slopes
   const int     sL = sR - ring_stride3(dir), st = P.st64;
