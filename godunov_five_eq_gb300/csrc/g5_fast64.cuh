@@ -441,6 +441,14 @@ thinc_none64()
   return __longlong_as_double(-1LL);
 }
 
+// the S of a ring cell one of whose values left the fast form's range: its
+// faces take the reference arithmetic (a NaN, so itself out of range)
+__device__ __forceinline__ double
+bad_cell64()
+{
+  return __longlong_as_double(-2LL);
+}
+
 // whether the cell takes the THINC profile along a direction (its neighbours'
 // volume fractions aM, aP): a product of differences of volume fractions
 // cannot underflow, so its sign is the differences'

@@ -10,8 +10,9 @@
 // half of the resident CTAs takes that round in halves, one per CTA: 512x32
 // shock tube (64 blocks on 152 SMs) 45 -> 31 us per step, 486k-cell AMR
 // shock-bubble (6.25 rounds) 388 -> 383 us.
-// A value outside the fast form's range sends the rest of the tile to the
-// reference arithmetic (the `cold` functions).
+// A value outside the fast form's range sends the cells and faces that read
+// it, and the update of the tile, to the reference arithmetic (the `cold`
+// functions).
 #pragma once
 
 #include "g5_fast64.cuh"
@@ -76,7 +77,7 @@ thinc_cell(int i, int ty, int & dir, int & ci, int & cj)
 // the pair's face values, from its entry
 template <int B>
 __device__ __forceinline__ bool
-thinc_eval2(const double * sQ, double * sAF, int i, int ty, const PhysParams & P)
+thinc_eval2(const double * sQ, double * sRec, double * sAF, int i, int ty, const PhysParams & P)
 {
   using T = Step2DTraits<B, false>;
   constexpr int  G = T::G, GG = G * G;
@@ -90,6 +91,8 @@ thinc_eval2(const double * sQ, double * sAF, int i, int ty, const PhysParams & P
   const double nd = youngs_ratio64(dir == 0 ? gx : gy, gx * gx + gy * gy, bad);
   const int    o = dir == 0 ? 1 : G;
   thinc_pair64(A[0], A[-o], A[o], nd, P, sAF[i], sAF[Step2D64<B>::NTH + i], bad);
+  if (bad) // its faces take the reference arithmetic
+    sRec[15 * T::S * T::S + (ci + 1) + T::S * (cj + 1)] = bad_cell64();
   return bad;
 }
 
@@ -142,12 +145,15 @@ face_state_fast64(const double * sQ, const double * sRec, const double * sAF, in
 
 template <int B, bool MG>
 __device__ __forceinline__ bool
-face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, double * sF, int ty, int dir, int ff, double dtdx, const PhysParams & P)
+face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, double * sF, int ty, int dir, int ff, bool check, double dtdx,
+                 const PhysParams & P)
 {
   using H = V<2>;
-  constexpr int NFF = B * (B + 1);
+  constexpr int NFF = B * (B + 1), S = B + 2, SS = S * S;
   int           li, lj, ri, rj;
   face_cells<B>(dir, ff, li, lj, ri, rj);
+  if (check && (bits64(sRec[15 * SS + (li + 1) + S * (lj + 1)]) == bits64(bad_cell64()) || bits64(sRec[15 * SS + (ri + 1) + S * (rj + 1)]) == bits64(bad_cell64())))
+    return true;
   double       qL[6], qR[6], fl[8];
   bool         bad = false;
   const double Sl = face_state_fast64<B>(sQ, sRec, sAF, li, lj, ty, dir, 1, P, qL, bad);
@@ -156,10 +162,7 @@ face_flux_fast64(const double * sQ, const double * sRec, const double * sAF, dou
   const Side64 R = hllc_side64<2, MG>(qR, Sr, P, bad);
   hllc_fast64<2>(qL, qR, L, R, dtdx, fl, bad);
   if (bad)
-  {
-    face_flux_cold64<B>(sQ, sRec, sF, dir, ff, dtdx, &P);
     return true;
-  }
 #pragma unroll
   for (int k = 0; k < 8; ++k)
     sF[(k == H::FU ? H::FU + dir : k == H::FV ? H::FV - dir : k) * NFF + ff] = fl[k];
@@ -237,8 +240,6 @@ hancock_fast64(const double * sQ, double * sRec, int gi, int r, double dtdx, con
     sRec[13 * SS + r] = sv[0];
     sRec[14 * SS + r] = sv[1];
   }
-  if (bad)
-    hancock_cold64<B>(sQ, sRec, gi, r, dtdx, &P);
   return bad;
 }
 
@@ -330,6 +331,13 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
   __shared__ int     sSlot[10]; // the block's reflux slots (faces 0-3), its defer slots, its outside-twin range
   __shared__ int     sNext;     // the CTA's next item
   __shared__ int     sThinc;    // entries of the THINC list
+  // faces that take the reference arithmetic, and the ghosted cells with a
+  // primitive out of range (one bit each)
+  using FaceId = typename std::conditional<B == 8, unsigned char, short>::type;
+  constexpr int       NW = (GG + 31) / 32;
+  __shared__ int      sCold;
+  __shared__ FaceId   sFace[2 * NFF];
+  __shared__ unsigned sBad[NW];
   const int          tid = threadIdx.x;
   const PhysParams & P = a.p;
   auto               item_block = [&](int i) {
@@ -337,7 +345,10 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
     return a.work ? a.work[w] : w;
   };
   if (tid == 0)
-    sThinc = 0;
+    sThinc = sCold = 0;
+  if (tid < NW)
+    sBad[tid] = 0u;
+  __syncthreads();
 
   for (int iw = blockIdx.x; iw < n_items;)
   {
@@ -409,6 +420,11 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
         for (int v = 0; v < H::NV; ++v)
           s.v[v] = u[v];
         prim_ref64<2>(s, &P, sQ + gidx, GG);
+        bool out = false;
+        for (int k = 0; k < 6; ++k)
+          out = out || x64_raw_bad(sQ[k * GG + gidx]);
+        if (out)
+          atomicOr(&sBad[gidx >> 5], 1u << (gidx & 31));
       }
       else
       {
@@ -456,10 +472,24 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
         }
       }
       const int r = (ri + 1) + S * (rj + 1), gi = (ri + 2) + G * (rj + 2);
-      if (cold0)
+      // In a tile with a value out of range each cell decides by the values
+      // that it reads, each face by its two cells, and the faces left over
+      // are evaluated from a list, with full warps.  A flow that started at
+      // rest holds velocities that fall off to 1e-323 ahead of the waves:
+      // 14 % of the shock-bubble's blocks, a few columns of cells in each
+      // (431k cells after 5, 20 and 300 steps: 430, 490, 487 -> 364, 395, 391
+      // us against the reference arithmetic for the whole tile; 331 us
+      // without such values; 383 -> 385 us for 486k cells that have none).
+      auto out = [&](int g) { return (sBad[g >> 5] >> (g & 31)) & 1u; };
+      bool bad = cold0 && (x64_raw_bad(dtdx) || (out(gi) | out(gi - 1) | out(gi + 1) | out(gi - G) | out(gi + G)) != 0u);
+      if (!bad)
+        bad = hancock_fast64<B, MG>(sQ, sRec, gi, r, dtdx, P);
+      if (bad)
+      {
+        cold = true;
         hancock_cold64<B>(sQ, sRec, gi, r, dtdx, &P);
-      else
-        cold |= hancock_fast64<B, MG>(sQ, sRec, gi, r, dtdx, P);
+        sRec[15 * SS + r] = bad_cell64();
+      }
     }
     // the interface cells of the THINC reconstruction
     if (P.thinc != 0)
@@ -477,10 +507,10 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
       }
     }
     cold = __syncthreads_or(cold) != 0;
-    if (P.thinc != 0 && sThinc > 0 && !cold)
+    if (P.thinc != 0 && sThinc > 0)
     {
       for (int i = tid; i < sThinc; i += NT)
-        cold |= thinc_eval2<B>(sQ, sAF, sList[i], ty, P);
+        cold |= thinc_eval2<B>(sQ, sRec, sAF, sList[i], ty, P);
       cold = __syncthreads_or(cold) != 0;
     }
 
@@ -491,10 +521,11 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
     {
       const int dir = f < nfx ? 0 : 1, ff = f - dir * nfx;
       double *  sF = dir == 0 ? sFx : sFy;
-      if (cold1)
-        face_flux_cold64<B>(sQ, sRec, sF, dir, ff, dtdx, &P);
-      else
-        cold |= face_flux_fast64<B, MG>(sQ, sRec, sAF, sF, ty, dir, ff, dtdx, P);
+      if (face_flux_fast64<B, MG>(sQ, sRec, sAF, sF, ty, dir, ff, cold1, dtdx, P))
+      {
+        cold = true;
+        sFace[atomicAdd(&sCold, 1)] = (FaceId)f;
+      }
     }
     // the own cell's state again (an L2 hit, in flight while the CTA waits at
     // the barrier; held from the gather it cost 16 registers)
@@ -506,6 +537,19 @@ step2d_fast64_kernel(const __grid_constant__ StepArgs a, int n_full, int n_items
         uown[v] = __ldcg(own + v * NC);
     }
     cold = __syncthreads_or(cold) != 0;
+    if (cold)
+    {
+      for (int i = tid; i < sCold; i += NT)
+      {
+        const int f = sFace[i], dir = f < nfx ? 0 : 1;
+        face_flux_cold64<B>(sQ, sRec, dir == 0 ? sFx : sFy, dir, f - dir * nfx, dtdx, &P);
+      }
+      __syncthreads();
+      if (tid == 0)
+        sCold = 0;
+      if (tid < NW)
+        sBad[tid] = 0u;
+    }
     if (tid == 0)
       sThinc = 0; // (read before the barrier above, used again after the next)
 
