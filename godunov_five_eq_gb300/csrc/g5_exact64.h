@@ -17,6 +17,9 @@
 // error is a few units of the 63rd bit (bounds at each function), so the
 // rounding to 53 bits is certain unless the ten bits below are within that
 // error of the midpoint; only then the sign of the exact remainder decides.
+// A seed is kept in [1/2, 1), where its mantissa bits are all of it: next to
+// either end (a mantissa just below 2 or 4, or at 1) the approximation may step
+// over.
 // A quotient or root of doubles is never exactly a midpoint.
 //
 // Range.  Operands are zero or normal (never subnormal, infinite or NaN); a
@@ -104,8 +107,9 @@ x64_mant(uint32_t hi, uint32_t lo)
   return ((uint64_t)((hi & 0x000FFFFFu) | 0x00100000u) << 42) | ((uint64_t)lo << 10);
 }
 
-// bits of a float approximation of 1/f and 1/sqrt(f) (f given by its bits,
-// positive and normal), within 2 units of the last place
+// bits of a float approximation of 1/f (f in [1, 2]) within 2^-23, of
+// 1/sqrt(f) (f in [1, 4]) within 2^-22.9 of its value, which is what PTX
+// promises for the two instructions; f by its bits
 G5_HD uint32_t
 x64_seed_rcp(uint32_t fb)
 {
@@ -138,6 +142,23 @@ x64_seed_rsqrt(uint32_t fb)
 #endif
 }
 
+// a mantissa (of 20 and 32 bits) rounded to 24 bits, as the bits of a float in
+// [1, 2], of one in [2, 4] with `odd`
+G5_HD uint32_t
+x64_float_mant(uint32_t hi, uint32_t lo, uint32_t odd)
+{
+  return 0x3F800000u + (odd << 23) + (((hi & 0x000FFFFFu) << 3) | (lo >> 29)) + ((lo >> 28) & 1u);
+}
+
+// a seed as an integer multiple of 2^-24, in [2^23, 2^24)
+G5_HD uint32_t
+x64_seed_mant(uint32_t sb)
+{
+  sb = sb > 0x3F7FFFFFu ? 0x3F7FFFFFu : sb;
+  sb = sb < 0x3F000000u ? 0x3F000000u : sb;
+  return (sb & 0x007FFFFFu) | 0x00800000u;
+}
+
 G5_HD uint64_t
 x64_mulhi3(uint64_t a, uint64_t b)
 {
@@ -162,24 +183,21 @@ struct Recip64
   uint32_t hi, lo; // the divisor
 };
 
-// y0 = m 2^-24 from the float seed: |e| < 2^-22.3 (2 units of 2^-24 from the
-// seed, 2^-24 from rounding the mantissa to 24 bits).  y0 (1 + e + e^2) is
-// e^3 < 2^-66 away; D is exact, the truncations of T weigh 2^-12 units of y,
-// the two shifts of z at most one unit.
+// y0 = m 2^-24 from the float seed (of x64_float_mant's bits): |e| < 2^-21.6
+// (2^-23 from the seed and 2^-24 from rounding the mantissa to 24 bits, times
+// the mantissa).  y0 (1 + e + e^2) is e^3 < 2^-64.8 away, half a unit of y; D
+// is exact, the truncations of T weigh 2^-12 units of y, the two shifts of z
+// at most one unit.
 G5_HD Recip64
-recip64(double b, bool & bad)
+recip64_seeded(double b, uint32_t seed, bool & bad)
 {
   Recip64 r;
   r.hi = x64_hi(b);
   r.lo = x64_lo(b);
   bad = bad || (r.hi & 0x7FF00000u) == 0u; // a zero divisor
   const uint32_t mh = (r.hi & 0x000FFFFFu) | 0x00100000u;
-  // the mantissa rounded to 24 bits, as a float in [1, 2]
-  const uint32_t fb = 0x3F800000u + (((r.hi & 0x000FFFFFu) << 3) | (r.lo >> 29)) + ((r.lo >> 28) & 1u);
-  uint32_t       sb = x64_seed_rcp(fb);
-  sb = sb > 0x3F7FFFFFu ? 0x3F7FFFFFu : sb; // below 1
-  const uint32_t m = (sb & 0x007FFFFFu) | 0x00800000u;
-  // D = 2^76 e, exact modulo 2^64, |D| < 2^54
+  const uint32_t m = x64_seed_mant(seed);
+  // D = 2^76 e, exact modulo 2^64, |D| < 2^54.4
   const int64_t D = (int64_t)(0u - ((uint64_t)m * r.lo + ((uint64_t)(m * mh) << 32)));
   // T = 2^76 (e + e^2)
   const int32_t Dh = (int32_t)(D >> 24);
@@ -188,6 +206,12 @@ recip64(double b, bool & bad)
   const int64_t z = (int64_t)(int32_t)m * (int32_t)(T >> 32) + (int64_t)(((uint64_t)m * (uint32_t)T) >> 32);
   r.y = ((uint64_t)m << 40) + (uint64_t)(z >> 4);
   return r;
+}
+
+G5_HD Recip64
+recip64(double b, bool & bad)
+{
+  return recip64_seeded(b, x64_seed_rcp(x64_float_mant(x64_hi(b), x64_lo(b), 0u)), bad);
 }
 
 // a / b.  q holds the quotient's top 63 bits to -8 .. +2 units (a y to -4
@@ -220,23 +244,29 @@ div64(double a, double b, bool & bad)
   return quot64(a, recip64(b, bad), bad);
 }
 
+// whether the root of a high word takes the doubled mantissa
+G5_HD uint32_t
+x64_odd(uint32_t hi)
+{
+  return ((hi >> 20) & 1u) ^ 1u;
+}
+
 // sqrt(x), x >= 0.  With x = m 4^k, m in [1, 4): N = 2^62 m; y0 = c 2^-24
-// from the float seed, e = 1 - m y0^2, |e| < 2^-21.3; y0 (1 + e/2 + 3 e^2/8)
-// is 5 e^3 / 16 < 2^-65 away; D drops less than one unit of 2^-78.  The root's
-// 63 bits N y come to -5 .. +2 units.
+// from the float seed, e = 1 - m y0^2, |e| < 2^-21.5 (twice the seed's 2^-22.9,
+// 2^-24 from rounding the mantissa to 24 bits); y0 (1 + e/2 + 3 e^2/8) is 5 e^3
+// / 16 < 2^-66 away; D drops less than one unit of 2^-78 (a seed 2 units of
+// 2^-24 off would take D >> 26 past 31 bits).  The root's 63 bits N y come to
+// -5 .. +2 units.
 G5_HD double
-sqrt64(double x, bool & bad)
+sqrt64_seeded(double x, uint32_t seed)
 {
   const uint32_t hx = x64_hi(x), lx = x64_lo(x);
   const bool     zero = hx == 0u;
   const uint32_t mh = (hx & 0x000FFFFFu) | 0x00100000u;
-  const uint32_t odd = ((hx >> 20) & 1u) ^ 1u;
+  const uint32_t odd = x64_odd(hx);
   const uint64_t m53 = ((uint64_t)mh << 32) | lx;
   const uint64_t N = m53 << (10u + odd);
-  const uint32_t fb = 0x3F800000u + (odd << 23) + (((hx & 0x000FFFFFu) << 3) | (lx >> 29)) + ((lx >> 28) & 1u);
-  uint32_t       sb = x64_seed_rsqrt(fb);
-  sb = sb > 0x3F7FFFFFu ? 0x3F7FFFFFu : sb;
-  const uint32_t c = (sb & 0x007FFFFFu) | 0x00800000u;
+  const uint32_t c = x64_seed_mant(seed);
   // D = 2^78 e, modulo 2^64, |D| < 2^57
   const uint64_t W = (uint64_t)c * c;
   const uint32_t wh = (uint32_t)(W >> 32), wl = (uint32_t)W, nh = (uint32_t)(N >> 32), nl = (uint32_t)N;
@@ -254,6 +284,13 @@ sqrt64(double x, bool & bad)
   }
   const uint32_t t = ((((hx >> 20) + 1021u - odd) >> 1) << 20);
   return x64_make(zero ? hx : (uint32_t)(M >> 32) + t, zero ? lx : (uint32_t)M);
+}
+
+G5_HD double
+sqrt64(double x, bool & bad)
+{
+  const uint32_t hx = x64_hi(x);
+  return sqrt64_seeded(x, x64_seed_rsqrt(x64_float_mant(hx, x64_lo(x), x64_odd(hx))));
 }
 
 // a b, correctly rounded (ties to even): the 126-bit product of the 63-bit
