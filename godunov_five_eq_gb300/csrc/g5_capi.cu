@@ -48,8 +48,11 @@ struct G5Context
   unsigned int * d_status = nullptr;
   // g5_remap's tables on the device: stream-ordered allocations of a pool of
   // the context's own that keeps its memory (the device's default pool gives
-  // it back at every synchronisation), released by g5_destroy
+  // it back at every synchronisation) up to REMAP_KEEP bytes, the driver's
+  // first reservation and the tables of 1M 3D blocks; g5_mem_bytes counts it,
+  // g5_destroy releases it
   cudaMemPool_t  remap_pool = nullptr;
+  static constexpr uint64_t REMAP_KEEP = 32u << 20;
   int64_t        bytes = 0;
   struct PoolEntry
   {
@@ -581,7 +584,7 @@ g5_destroy(G5Context * ctx)
   if (hp.s_out)
     cudaStreamDestroy(hp.s_out);
   if (ctx->remap_pool)
-    cudaMemPoolDestroy(ctx->remap_pool); // (outstanding frees complete first)
+    cudaMemPoolDestroy(ctx->remap_pool); // (returns at once; the memory goes when the last pending free has run)
   delete ctx;
   return G5_OK;
 }
@@ -837,7 +840,15 @@ g5_set_mesh(G5Context * c, const G5Mesh * m)
 extern "C" int64_t
 g5_mem_bytes(const G5Context * ctx)
 {
-  return ctx ? ctx->bytes : (int64_t)G5_ERR_ARG;
+  if (!ctx)
+    return (int64_t)G5_ERR_ARG;
+  uint64_t pool = 0;
+  if (ctx->remap_pool && cudaMemPoolGetAttribute(ctx->remap_pool, cudaMemPoolAttrReservedMemCurrent, &pool) != cudaSuccess)
+  {
+    cudaGetLastError();
+    pool = 0;
+  }
+  return ctx->bytes + (int64_t)pool;
 }
 
 extern "C" int
@@ -1263,7 +1274,7 @@ remap_alloc(G5Context * c, void ** p, size_t bytes, cudaStream_t st)
       c->remap_pool = nullptr;
       return e;
     }
-    uint64_t keep = UINT64_MAX;
+    uint64_t keep = G5Context::REMAP_KEEP;
     cudaMemPoolSetAttribute(c->remap_pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
   return cudaMallocFromPoolAsync(p, bytes, c->remap_pool, st);
