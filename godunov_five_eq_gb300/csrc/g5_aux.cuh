@@ -701,87 +701,89 @@ defer_info_kernel(DevMesh m, const int32_t * codes, int n, int32_t * info)
     row[k] = 0;
 }
 
-// ComputeDerivedQuantities::run (utils/ComputeDerivedQuantities.h:96-180):
-// one derived quantity of a cell's conservative state, FP64 in the
-// reference's operation order.  quantity: 0 RHO_MIX, 1 THERMAL_PRESSURE,
+// the derived quantities a field list asks for (bits of FieldList::need)
+constexpr int NEED_PRESSURE = 1 << 1, NEED_SOUND = 1 << 2, NEED_EKIN = 1 << 3, NEED_MACH = 1 << 4, NEED_VELOCITY = (1 << 5) | (1 << 6) | (1 << 7);
+
+// ComputeDerivedQuantities::run (utils/ComputeDerivedQuantities.h:96-180): the
+// derived quantities of a cell's conservative state that `need` asks for, FP64
+// in the reference's operation order.  d[q]: 0 RHO_MIX, 1 THERMAL_PRESSURE,
 // 2 SPEED_OF_SOUND, 3 SPECIFIC_EKIN, 4 LOCAL_MACH_NUMBER, 5 VX, 6 VY, 7 VZ
 // (the DERIVED_QUANTITY enum order).
 template <int DIM>
-__device__ __forceinline__ double
-derived_value(const double * u, int quantity, const PhysParams & P)
+__device__ __forceinline__ void
+derived_ref64(const double * u, int need, const PhysParams & P, double * d)
 {
   using H = V<DIM>;
-  double r = 0.0;
-  if (quantity == 0)
-    r = u[H::ID];
-  else if (quantity == 1 || quantity == 3)
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    d[k] = 0.0;
+  d[0] = u[H::ID];
+  if (need & (NEED_PRESSURE | NEED_EKIN))
   {
     // compute_mixture_ekin (models/utils.h:124-151): density from ID
-    const double d = fmax(u[H::ID], P.smallr);
-    const double ux = u[H::IU] / d, uy = u[H::IV] / d;
+    const double rho = fmax(u[H::ID], P.smallr);
+    const double ux = u[H::IU] / rho, uy = u[H::IV] / rho;
     double       ekin;
     if constexpr (DIM == 2)
       ekin = 0.5 * (ux * ux + uy * uy);
     else
     {
-      const double uz = u[H::IW] / d;
+      const double uz = u[H::IW] / rho;
       ekin = 0.5 * (ux * ux + uy * uy + uz * uz);
     }
-    if (quantity == 3)
-      r = ekin;
-    else
+    d[3] = ekin;
+    if (need & NEED_PRESSURE)
     {
       // compute_mixture_pressure (models/utils.h:160-185): density from the partial densities
       const double dm = fmax(u[H::IAD0] + u[H::IAD1], P.smallr);
       const double eint = u[H::IE] / dm - ekin;
       const double a0 = u[H::IA0];
       if (!P.mg_any)
-        r = (dm * eint - eosPI(P, a0, 1 - a0)) / eosS(P, a0, 1 - a0);
+        d[1] = (dm * eint - eosPI(P, a0, 1 - a0)) / eosS(P, a0, 1 - a0);
       else
       {
         double S, PI, C1, C0;
         mg_mixture(P, a0, 1 - a0, u[H::IAD0], u[H::IAD1], S, PI, C1, C0);
-        r = (dm * eint - PI) / S;
+        d[1] = (dm * eint - PI) / S;
       }
     }
   }
-  else
+  if (need & (NEED_SOUND | NEED_MACH | NEED_VELOCITY))
   {
-    double       q[7];
-    const double cs = prim_fp64<DIM>(u, q, P);
-    if (quantity == 2)
-      r = cs;
-    else if (quantity == 4)
+    double q[7];
+    d[2] = prim_fp64<DIM>(u, q, P);
+    d[5] = q[H::QU];
+    d[6] = q[H::QV];
+    double un = q[H::QU] * q[H::QU] + q[H::QV] * q[H::QV];
+    if constexpr (DIM == 3)
     {
-      double un = q[H::QU] * q[H::QU] + q[H::QV] * q[H::QV];
-      if constexpr (DIM == 3)
-        un += q[H::QW] * q[H::QW];
-      un = sqrt(un);
-      r = un / cs;
+      d[7] = q[H::QW];
+      un += q[H::QW] * q[H::QW];
     }
-    else if (quantity == 5)
-      r = q[H::QU];
-    else if (quantity == 6)
-      r = q[H::QV];
-    else if constexpr (DIM == 3)
-      r = q[H::QW];
+    if (need & NEED_MACH)
+      d[4] = sqrt(un) / d[2];
   }
+}
+
+struct Derived64
+{
+  double v[8];
+};
+
+// one call per cell: with a call per quantity, each converting the cell again,
+// eight quantities of 486k cells that all take it were 479 us, of constants
+// outside the fast form's range 559 us; 184 and 186 us this way
+template <int DIM>
+__device__ __noinline__ Derived64
+derived_cold64(State64<DIM> s, int need, const PhysParams * P)
+{
+  Derived64 r;
+  derived_ref64<DIM>(s.v, need, *P, r.v);
   return r;
 }
 
-template <int DIM>
-__device__ __noinline__ double
-derived_cold64(State64<DIM> s, int quantity, const PhysParams * P)
-{
-  return derived_value<DIM>(s.v, quantity, *P);
-}
-
-// the derived quantities a field list asks for (bits of FieldList::need)
-constexpr int NEED_PRESSURE = 1 << 1, NEED_SOUND = 1 << 2, NEED_EKIN = 1 << 3, NEED_MACH = 1 << 4, NEED_VELOCITY = (1 << 5) | (1 << 6) | (1 << 7);
-
-// every quantity of `need` at once (derived_value one at a time converts the
-// cell for each of them): d[q] of DERIVED_QUANTITY q.  False when a value
-// leaves the range of g5_fast64.cuh.
+// the same from the fast operations; false when a value leaves the range of
+// g5_fast64.cuh
 template <int DIM, bool MG>
 __device__ __forceinline__ bool
 derived_fast64(const double * u, int need, const PhysParams & P, double * d)
@@ -845,8 +847,9 @@ derived_fast64(const double * u, int need, const PhysParams & P, double * d)
 // num_octs), in one pass over U: field k of cell g (counted from oct_begin) to
 // out[k * stride + g] (FieldList codes: a variable of U, or FIELD_DERIVED + a
 // derived quantity).  KIND 0, 1 (stiffened gases, Mie-Grueneisen laws): the
-// derived quantities computed together; 2: one by one in the reference's arithmetic.  12 fields (4
-// derived) of 486k cells: 262 us with the reference arithmetic per field.
+// derived quantities from the fast operations; 2: in the reference's
+// arithmetic.  12 fields (4 derived) of 486k cells: 262 us with the reference
+// arithmetic per field, 37 us from the fast operations, 164 us in KIND 2.
 template <int DIM, int B, int KIND>
 __global__ void __launch_bounds__(256)
 fields_kernel(const double * __restrict__ U, double * __restrict__ out, const __grid_constant__ FieldList fl, long long stride, long long oct_begin,
@@ -863,13 +866,25 @@ fields_kernel(const double * __restrict__ U, double * __restrict__ out, const __
 #pragma unroll
     for (int v = 0; v < H::NV; ++v)
       u[v] = U[(oct * H::NV + v) * NC + cell];
-    bool fast = KIND != 2;
-    if constexpr (KIND != 2)
-    {
-      if (fl.need != 0)
-        fast = derived_fast64<DIM, KIND == 1>(u, fl.need, P, d);
-    }
     d[0] = u[H::ID];
+    if (fl.need != 0)
+    {
+      bool fast = false;
+      if constexpr (KIND != 2)
+        fast = derived_fast64<DIM, KIND == 1>(u, fl.need, P, d);
+      if (!fast)
+      {
+        State64<DIM> s;
+#pragma unroll
+        for (int v = 0; v < H::NV; ++v)
+          s.v[v] = u[v];
+        const Derived64 r = derived_cold64<DIM>(s, fl.need, &P);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          d[q] = r.v[q];
+      }
+      d[0] = u[H::ID];
+    }
     for (int k = 0; k < fl.n; ++k)
     {
       const int c = fl.code[k];
@@ -879,20 +894,9 @@ fields_kernel(const double * __restrict__ U, double * __restrict__ out, const __
         r = c == v ? u[v] : r;
       if (c >= FIELD_DERIVED)
       {
-        if (fast)
-        {
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            r = c == FIELD_DERIVED + q ? d[q] : r;
-        }
-        else
-        {
-          State64<DIM> s;
-#pragma unroll
-          for (int v = 0; v < H::NV; ++v)
-            s.v[v] = u[v];
-          r = derived_cold64<DIM>(s, c - FIELD_DERIVED, &P);
-        }
+        for (int q = 0; q < 8; ++q)
+          r = c == FIELD_DERIVED + q ? d[q] : r;
       }
       out[k * stride + g] = r;
     }
