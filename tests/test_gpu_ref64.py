@@ -51,3 +51,79 @@ def test_fields_and_cfl_rate(dim, b, gas, floor):
         assert np.array_equal(impl.derived_quantity(d_U, q).cpu().numpy()[:n, 0], ref[:n], equal_nan=True), q
     assert np.array_equal(every[8], U[:n, 1]) and np.array_equal(every[9], U[:n, 0])
     assert np.array_equal(impl.compute_inv_dt(d_U).cpu().numpy(), o.inv_dt(U))
+
+
+CASES = [
+    # dim, block, law, options
+    (2, 16, None, {}),
+    (2, 16, None, dict(thinc=1, source_term=1)),
+    (2, 16, None, dict(integrator=1, slope_type=2.0)),
+    (2, 8, None, dict(slope_type=0.0)),
+    (2, 8, None, dict(thinc=1, slope_type=2.0)),
+    (2, 8, "jwl", dict(thinc=1)),
+    (2, 16, "shockwave", dict(source_term=1)),
+    (3, 8, None, {}),
+    (3, 8, None, dict(thinc=1, source_term=1, slope_type=2.0)),
+    (3, 8, None, dict(integrator=1)),
+    (3, 8, "jwl", dict(thinc=1)),
+]
+
+
+@pytest.mark.parametrize("floor", sorted(FLOORS))
+@pytest.mark.parametrize("dim,b,gas,kw", CASES, ids=["-".join([str(c[0]), str(c[1]), str(c[2])] + sorted(c[3])) for c in CASES])
+def test_step(dim, b, gas, kw, floor):
+    t, p, U = build(dim, b, floor, gas, **kw)
+    o = Oracle(t, p)
+    o.fill_outside(U)
+    dt = 0.5 * o.dt(U)
+    ref = o.step(U, dt)
+    impl = GodunovImplemGB300(p, t)
+    d_U, d_U2 = device(U)
+    inv = torch.zeros(t.n_inst, dtype=torch.float64, device="cuda")
+    impl.do_time_step(d_U, d_U2, dt, mode="fp64", inv_dt_out=inv)
+    n = t.n_owned
+    assert np.array_equal(d_U2.cpu().numpy()[:n], ref[:n], equal_nan=True)
+    full = np.zeros_like(U)
+    full[:n] = ref[:n]
+    assert np.array_equal(inv.cpu().numpy(), o.inv_dt(full))
+
+
+@pytest.mark.parametrize("dim,b", [(2, 16), (2, 8), (3, 8)])
+@pytest.mark.parametrize("integrator", [0, 2])
+@pytest.mark.parametrize("thinc", [0, 1])
+def test_solver_loop(dim, b, integrator, thinc):
+    """Walls, coarse/fine records and the boundary fill inside the step, five
+    steps of the device-driven loop; RK2's combination with its CFL rate."""
+    mesh, t = amr_mesh(dim=dim, b=b, periodic=False, nref=4, lmin=1, lmax=3, seed=9)
+    p = water_air_params(t, dim=dim, b=b, bc=(2, 2, 3, 3, 2, 3), integrator=integrator, thinc=thinc, smallc=0.0)
+    U = smooth_state(mesh, t, p, seed=3)
+    ref, hist = Oracle(t, p).run(U.copy(), 5)
+    impl = GodunovImplemGB300(p, t)
+    d_U, d_U2 = device(U)
+    dts = torch.zeros((5, 1), dtype=torch.float64, device="cuda")
+    impl.run(d_U, d_U2, 5, mode="fp64", dt_hist=dts)
+    assert impl.status() == 0
+    assert np.array_equal(dts.cpu().numpy().ravel(), np.asarray(hist).ravel())
+    assert np.array_equal(d_U.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("dim,b", [(2, 16), (2, 8), (3, 8)])
+def test_host_step_and_shapes(dim, b):
+    """Chunks with work lists, and every launch shape, give the plain step's bits."""
+    t, p, U = build(dim, b, "smallc0")
+    o = Oracle(t, p)
+    o.fill_outside(U)
+    dt = o.dt(U)
+    ref = o.step(U, dt)[: t.n_owned]
+    impl = GodunovImplemGB300(p, t)
+    hU, hU2 = torch.from_numpy(U.copy()).pin_memory(), torch.zeros(U.shape, dtype=torch.float64).pin_memory()
+    impl.do_time_step_host(hU, hU2, dt, mode="fp64")
+    torch.cuda.synchronize()
+    assert np.array_equal(hU2.numpy()[: t.n_owned], ref)
+    d_U, d_U2 = device(U)
+    for ctas in (1, 2, 0):
+        for claim in (0, 1):
+            impl.set_shape("fp64", ctas_per_sm=ctas, claim=claim, walk_cf_first=claim)
+            d_U2.zero_()
+            impl.do_time_step(d_U, d_U2, dt, mode="fp64")
+            assert np.array_equal(d_U2.cpu().numpy()[: t.n_owned], ref)
