@@ -773,8 +773,8 @@ step2d_kernel(const __grid_constant__ StepArgs a)
       // (the own cell's loads are in flight while the halo gather runs; its
       // primitives are stored last)
       const int ci = tid % B, cj = tid / B;
-      // (the FP64 form has more threads than cells; the ones without a cell
-      // take the first halo cells)
+      // (the FP32-bulk form of 8x8 blocks has two threads per cell; the ones
+      // without a cell take the first halo cells)
       const bool owner = NT == NC || tid < NC;
       double     uin[H::NV];
       if (owner)

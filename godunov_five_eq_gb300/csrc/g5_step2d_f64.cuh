@@ -12,7 +12,8 @@
 // shock-bubble (6.25 rounds) 388 -> 383 us.
 // A value outside the fast form's range sends the cells and faces that read
 // it, and the update of the tile, to the reference arithmetic (the `cold`
-// functions).
+// functions).  Blocks that hold such values throughout take longer than in
+// step2d_kernel (all momenta below 1e-136, 486k cells: 1,397 us against 1,174).
 #pragma once
 
 #include "g5_fast64.cuh"
@@ -26,7 +27,7 @@ struct Step2D64
 {
   using T = Step2DTraits<B, false>;
   // more threads than cells, so that the 320 (96) slope cells take one round
-  // and the 544 (144) faces two, at 96 registers (16x16: 420 us per
+  // and the 544 (144) faces two, at 96 (80) registers (16x16: 420 us per
   // shock-bubble step of 486k cells against 444 us with 256 threads at 128
   // registers, 438 us with 384 at 80; 8x8: 147 us against 161 with 64 threads)
   static constexpr int NT = B == 16 ? 320 : 96;

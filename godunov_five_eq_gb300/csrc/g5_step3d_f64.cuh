@@ -4,7 +4,8 @@
 // form is the reference arithmetic; the results are the same doubles.
 //
 // One CTA of 576 threads per 8^3 block: the 576 faces of a direction take one
-// round (512 threads took two, the second with 64 faces), at 112 registers.
+// round (512 threads took two, the second with 64 faces), at 96 registers (what
+// 18 warps leave each; 388 bytes of spill stores, with the general laws 658).
 // The three directions run through one copy of the face code (a run-time
 // direction): three would not fit the instruction cache.  A value outside the
 // fast form's range sends the rest of the block to the reference arithmetic
